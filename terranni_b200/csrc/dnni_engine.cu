@@ -69,7 +69,7 @@ ScratchSizes scratch_sizes(const HostBatch& hb) {
     z.rownear = sizeof(int) * std::max<int64_t>(hb.blk_base.back(), 1);
     z.near = sizeof(int64_t) * std::max<int64_t>(hb.blk_base.back(), 1);
     z.pix = sizeof(int2) * std::max<int64_t>(hb.n_pix, 1);
-    z.far = sizeof(FarSlot) * std::max<int64_t>(hb.n_far, 1);
+    z.far = kFarSlotBytes * std::max<int64_t>(hb.n_far, 1);
     z.D = sizeof(unsigned long long) * std::max<int64_t>(hb.n_cells, 1);
     z.Dc = sizeof(int) * std::max<int64_t>(hb.n_cells, 1);
     z.sc = sizeof(Scalars) * n;
@@ -97,7 +97,7 @@ dnni_status ensure_scratch(dnni_ctx* c, Scratch& s, const ScratchSizes& z, DevAr
     a.rownear = (int*)s.rownear.p;
     a.near = (int64_t*)s.near.p;
     a.pix = (int2*)s.pix.p;
-    a.far = (FarSlot*)s.far.p;
+    a.far = (int4*)s.far.p;
     a.D = (unsigned long long*)s.D.p;
     a.Dc = (int*)s.Dc.p;
     a.sc = (Scalars*)s.sc.p;
@@ -140,6 +140,17 @@ void set_dense_smem_attr() {
     }
 }
 
+// The span path: as many CTAs as the SMs hold at once take the work items
+// that k_decide listed (layers: stacked rasters of nrt_layer raster tiles and
+// lstride records each, 0 = one).
+void launch_spans(const HostBatch& hb, const BatchTables& bt, const DevArrays& a, const int2* pix, const FarLayout& far,
+                  int nrt_layer, int64_t lstride, int sms, cudaStream_t st) {
+    const size_t smem = sizeof(unsigned long long) * hb.win_words;
+    const int per_sm = std::max(1, std::min(6, (int)((220u << 10) / (smem + 1024))));
+    k_scatter_window<<<sms * per_sm, dim3(32, 8), smem, st>>>(bt, pix, a.sc, a.D, a.Dc, hb.win_words, far, a.ctr,
+                                                             nrt_layer, lstride);
+}
+
 // Launch sequence, part 1: per-tile scalars and (with bbox) the point
 // bounding boxes, which a single work package needs before its bins are
 // planned; batches pass bbox = false and have k_bin_count take the boxes.
@@ -177,19 +188,19 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
     }
     if (ev) cudaEventRecord(ev[0], st);
     const int nrt = hb.rt_base.back();
-    k_near_dense<<<nrt, dim3(32, 8), kDenseSmem, st>>>(bt, a.sorted, a.start, a.pix, d_site, a.far, a.sc, a.ctr,
+    const FarLayout far = far_layout(a.far, hb.n_far, nrt);
+    k_near_dense<<<nrt, dim3(32, 8), kDenseSmem, st>>>(bt, a.sorted, a.start, a.pix, d_site, far, a.sc, a.ctr,
                                                        hb.far_blocks, hb.dense_band);
     if (ev) cudaEventRecord(ev[4], st);
     if (nchunk > 0)
-        k_near_far<<<sms * 6, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, a.far, a.pix, d_site,
-                                            a.sc, a.ctr);
+        k_near_far<<<sms * 6, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site,
+                                            a.sc, a.ctr, hb.far_blocks);
     if (sites_only) return;
-    k_decide<<<(int)hb.tiles.size(), 32, 0, st>>>(bt, a.sc);
+    k_decide<<<(int)hb.tiles.size(), 256, 0, st>>>(bt, a.sc, far, a.ctr, hb.win_words);
     if (ev) cudaEventRecord(ev[1], st);
     cudaMemsetAsync(a.D, 0, sizeof(unsigned long long) * hb.n_cells, st);
     cudaMemsetAsync(a.Dc, 0, sizeof(int) * hb.n_cells, st);
-    k_scatter_window<<<nrt, dim3(32, 8), sizeof(unsigned long long) * hb.win_words, st>>>(bt, a.pix, a.sc, a.D,
-                                                                                         a.Dc, hb.win_words);
+    launch_spans(hb, bt, a, a.pix, far, 0, 0, sms, st);
     if (ev) cudaEventRecord(ev[2], st);
     launch_rows_final(bt, hb.band_base.back(), hb.rs, a.pix, a.sc, a.D, a.Dc, d_h, st);
 }
@@ -1166,7 +1177,7 @@ bool carve_noalloc(unsigned char* base, const ScratchSizes& z, DevArrays& a) {
     a.sc = (Scalars*)take(z.sc);
     a.ctr = (BatchCounters*)take(z.ctr);
     a.pix = (int2*)take(z.pix);
-    a.far = (FarSlot*)take(z.far);
+    a.far = (int4*)take(z.far);
     a.D = (unsigned long long*)take(z.D);
     a.Dc = (int*)take(z.Dc);
     a.sorted = (int4*)take(z.sorted);

@@ -36,7 +36,7 @@ struct DevArrays {
     int* rownear = nullptr;
     int64_t* near = nullptr;
     int2* pix = nullptr;
-    dnni::FarSlot* far = nullptr;
+    int4* far = nullptr;             // worklist buffer, 16 B per slot (far_layout)
     unsigned long long* D = nullptr;
     int* Dc = nullptr;
     dnni::Scalars* sc = nullptr;

@@ -59,10 +59,12 @@ struct BatchTables {
 };
 
 struct BatchCounters {
-    int nfar;                    // far worklist slots used
+    int nfar;                    // far groups listed
     int err;                     // kErrRange when a point was out of range
     int far_next;                // next far group to hand out
-    int pad;
+    int nspan;                   // span work items listed
+    int span_next;               // next span work item to hand out
+    int pad[3];
 };
 
 template <typename B>
@@ -87,7 +89,7 @@ __global__ void k_init_scalars(BatchTables bt, Scalars* sc, BatchCounters* ctr) 
         s->bbox[2] = INT_MAX; s->bbox[3] = INT_MIN;
         s->bbox[4] = INT_MAX; s->bbox[5] = INT_MIN;
         s->err = 0; s->packed = 0; s->kbits = 0; s->zbase = 0;
-        if (t == 0) { ctr->nfar = 0; ctr->err = 0; ctr->far_next = 0; }
+        if (t == 0) { ctr->nfar = 0; ctr->err = 0; ctr->far_next = 0; ctr->nspan = 0; ctr->span_next = 0; }
     }
     if (l < kStatSlots) {
         s->max_r2[l] = -1; s->big_pixels[l] = 0; s->spans[l] = 0; s->nodata[l] = 0;
@@ -451,11 +453,45 @@ struct StatAcc {
     }
 };
 
-// Far worklist slot: tile, raster pixel index within the tile (-1 = empty
-// slot), sorted-array position of the best site so far (-1 = none).
-struct FarSlot {
-    int tile, pix, idx, pad;
+// One group of the far worklist: 32 neighbouring pixels of one tile (an 8 x 4
+// block or a 32 x 1 row, far_lane), from raster pixel (i0, j0).  idx: per
+// lane the sorted-array position of the best site so far (-1 = none,
+// kFarIdle = settled or outside the raster).
+struct FarGroup {
+    int tile, rt, i0, j0;        // rt: raster tile (launch index) the group lies in
+    int idx[32];
 };
+constexpr int kFarIdle = -2;
+
+// Pixel of a group's lane relative to the group's first one.
+__device__ __forceinline__ void far_lane(int far_blocks, int lane, int& di, int& dj) {
+    di = far_blocks ? lane & 7 : lane;
+    dj = far_blocks ? lane >> 3 : 0;
+}
+
+// The worklist buffer (kFarSlotBytes per pixel of the padded rasters) holds
+// the far groups, then one int per raster tile (the largest R2 of its
+// pixels) and the span work items (at most kSpanItemsPerTile per raster tile).
+constexpr int kFarSlotBytes = 16;
+constexpr int kSpanItemsPerTile = 64;
+struct FarLayout {
+    FarGroup* groups;
+    int* rtmax;
+    int2* items;
+};
+__host__ __device__ inline FarLayout far_layout(void* base, int64_t slots, int64_t nrt) {
+    unsigned char* b = (unsigned char*)base;
+    FarLayout L;
+    L.groups = (FarGroup*)b;
+    b += (sizeof(FarGroup) * (slots / 32) + 255) & ~(size_t)255;
+    L.rtmax = (int*)b;
+    b += (sizeof(int) * nrt + 255) & ~(size_t)255;
+    L.items = (int2*)b;
+    return L;
+}
+// groups 4.5 B per slot, rtmax 4 B and items 512 B per 2048 slots, two roundings
+static_assert(sizeof(FarGroup) == 144 && 2048 / 32 * sizeof(FarGroup) + 2 * 260 + 8 * kSpanItemsPerTile <=
+                  2048 * kFarSlotBytes, "the worklist buffer holds its three parts");
 
 // R2 of a pixel record that the ring search left unsettled (the far pass
 // overwrites it); real records hold R2 >= -1.
@@ -472,7 +508,7 @@ constexpr int kFarBlocksDefault = 1;   // far groups of 8 x 4 pixels
 // "no site".
 __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int4* __restrict__ pts_all,
                                                        const int* __restrict__ start_all, int2* __restrict__ pix,
-                                                       uint32_t* __restrict__ site, FarSlot* __restrict__ far,
+                                                       uint32_t* __restrict__ site, FarLayout far,
                                                        Scalars* __restrict__ sc, BatchCounters* __restrict__ ctr,
                                                        int far_blocks, int band0) {
     extern __shared__ int4 smem[];
@@ -481,6 +517,7 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
     int* s_gstart = s_lstart + kWinMaxBins + 1;
     __shared__ int s_rowbase[kWinMaxRows];
     __shared__ int s_total;
+    __shared__ int s_max[8];
     const int tid = threadIdx.y * 32 + threadIdx.x;
     const int t = find_tile(bt.rt_base, bt.ntiles, blockIdx.x);
     const TileParams& T = bt.tiles[t];
@@ -623,14 +660,17 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
         if (far_pixel) pix[T.pix_off + (int64_t)j * T.rw + i] = make_int2(b.idx, kPixFar);
     } else {
         // worklist: a warp with any unsettled pixel appends its whole row of
-        // 32 slots as one group (settled or absent pixels as empty slots), so
+        // 32 pixels as one group (settled or absent pixels idle), so
         // that a far warp later takes 32 neighbouring pixels of one tile
         const unsigned mfar = __ballot_sync(0xffffffffu, far_pixel);
         if (mfar) {
             int base = 0;
-            if (lane == 0) base = atomicAdd(&ctr->nfar, 32);
+            if (lane == 0) {
+                base = atomicAdd(&ctr->nfar, 1);
+                *reinterpret_cast<int4*>(&far.groups[base]) = make_int4(t, (int)blockIdx.x, i0, j);
+            }
             base = __shfl_sync(0xffffffffu, base, 0);
-            far[base + lane] = far_pixel ? FarSlot{t, j * T.rw + i, b.idx, 0} : FarSlot{t, -1, -1, 0};
+            far.groups[base].idx[lane] = far_pixel ? b.idx : kFarIdle;
         }
     }
     acc.add(T, R2, b.nev);
@@ -638,15 +678,25 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
     __syncthreads();     // the next band restages the window
     }
     acc.flush(sc + t, blockIdx.x + threadIdx.y, false);
+    // the largest R2 of the pixels settled here, for the span work items (the
+    // far pass raises it for the others)
+    {
+        const int m = __reduce_max_sync(0xffffffffu, acc.mx);
+        if (lane == 0) s_max[warp] = m;
+        __syncthreads();
+        if (tid < 32) {
+            const int v = __reduce_max_sync(0xffffffffu, s_max[tid & 7]);
+            if (tid == 0) far.rtmax[blockIdx.x] = v;
+        }
+    }
     if (far_blocks) {
         // worklist in 8 x 4 pixel blocks: a block with any unsettled pixel
         // appends its 32 pixels as one group (lane = 8 * row + column), so
         // that a far warp takes a compact patch whose discs overlap most;
-        // the records written above are visible after the barrier
-        __syncthreads();
+        // the records written above are visible after the barrier above
         for (int blk = warp; blk < (kTileX / 8) * (kTileY / 4); blk += 8) {
-            const int ii = i0 + (blk % (kTileX / 8)) * 8 + (lane & 7);
-            const int jj = j0 + (blk / (kTileX / 8)) * 4 + (lane >> 3);
+            const int bi = i0 + (blk % (kTileX / 8)) * 8, bj = j0 + (blk / (kTileX / 8)) * 4;
+            const int ii = bi + (lane & 7), jj = bj + (lane >> 3);
             bool fp = false;
             int idx = -1;
             if (ii < T.rw && jj < T.rh) {
@@ -656,9 +706,12 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
             }
             if (__ballot_sync(0xffffffffu, fp)) {
                 int base = 0;
-                if (lane == 0) base = atomicAdd(&ctr->nfar, 32);
+                if (lane == 0) {
+                    base = atomicAdd(&ctr->nfar, 1);
+                    *reinterpret_cast<int4*>(&far.groups[base]) = make_int4(t, (int)blockIdx.x, bi, bj);
+                }
                 base = __shfl_sync(0xffffffffu, base, 0);
-                far[base + lane] = fp ? FarSlot{t, jj * T.rw + ii, idx, 0} : FarSlot{t, -1, -1, 0};
+                far.groups[base].idx[lane] = fp ? idx : kFarIdle;
             }
         }
     }
@@ -888,9 +941,9 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
                                                      const uint64_t* __restrict__ bmask_all,
                                                      const uint64_t* __restrict__ smask_all,
                                                      const int64_t* __restrict__ near_all,
-                                                     const FarSlot* __restrict__ far, int2* __restrict__ pix,
+                                                     FarLayout far, int2* __restrict__ pix,
                                                      uint32_t* __restrict__ site, Scalars* __restrict__ sc,
-                                                     BatchCounters* __restrict__ ctr) {
+                                                     BatchCounters* __restrict__ ctr, int far_blocks) {
     const int count = ctr->nfar;
     const int lane = threadIdx.x & 31;
     // groups differ in cost by orders of magnitude (a lake's centre against
@@ -898,27 +951,30 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
     // a fixed stride
     for (;;) {
         int base = 0;
-        if (lane == 0) base = atomicAdd(&ctr->far_next, 32);
+        if (lane == 0) base = atomicAdd(&ctr->far_next, 1);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= count) break;
-        const FarSlot item = far[base + lane];
-        const int t = __shfl_sync(0xffffffffu, item.tile, 0);
+        const int4 head = *reinterpret_cast<const int4*>(&far.groups[base]);
+        const int own = far.groups[base].idx[lane];
+        const int t = head.x;
         const TileParams& T = bt.tiles[t];
         const BinGrid g = T.bg;
         const int4* pts = pts_all + T.srt_off;
         const int* start = start_all + T.bin_off;
         const uint64_t* bmask = bmask_all + T.blk_off;
         const uint64_t* smask = smask_all + T.sup_off;
-        const bool act = item.pix >= 0;
+        const bool act = own != kFarIdle;
         int i = 0, j = 0, px = 0, py = 0;
         Best b{LLONG_MAX, 0xFFFFFFFFu, INT_MAX, -1, 0};
         if (act) {
-            i = item.pix % T.rw;
-            j = item.pix / T.rw;
+            int di, dj;
+            far_lane(far_blocks, lane, di, dj);
+            i = head.z + di;
+            j = head.w + dj;
             px = (T.rx0 + i) * T.cs;
             py = (T.ry0 + j) * T.cs;
-            if (item.idx >= 0) {
-                consider(b, __ldg(&pts[item.idx]), item.idx, px, py);
+            if (own >= 0) {
+                consider(b, __ldg(&pts[own]), own, px, py);
                 b.nev += 1;
             }
             int bx = udiv32((long long)px - g.gx0, g.bs), by = udiv32((long long)py - g.gy0, g.bs);
@@ -946,6 +1002,8 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
         StatAcc acc;
         acc.add(T, R2, b.nev);
         acc.flush(sc + t, blockIdx.x * 3 + (threadIdx.x >> 5), true);
+        const int m = __reduce_max_sync(0xffffffffu, R2);
+        if (lane == 0 && m > T.rs * T.rs) atomicMax(&far.rtmax[head.y], m);
     }
 }
 
@@ -953,21 +1011,111 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
 // scatter-accumulate and finalize
 // ---------------------------------------------------------------------------
 
-// Per tile: the accumulator form of the span path (see decide_packing).
-__global__ void k_decide(BatchTables bt, Scalars* sc) {
+constexpr int kSpanWindowWords = 4096;      // default: 32 KB per CTA (two int32 arrays)
+constexpr int kSpanWindowMaxWords = 26624;  // 208 KB, the most one CTA may take
+constexpr int kSpanChunksPerItem = 2;       // window chunks of one span work item, at least
+
+// The grid cells that the discs of one 32 x kTileY raster tile may touch, from
+// its largest R2: columns [c0, c1] and rows [r0, r1] of the grid (empty when
+// c0 > c1 or r0 > r1), taken `rows` rows at a time by `win_words` cells of
+// shared memory (direct: one item, no window), `per` rows to a work item.
+struct SpanWindow {
+    int c0, c1, r0, r1, W, rows, per;
+    bool inside;                 // no span meets the grid's left or right edge
+};
+
+__device__ __forceinline__ SpanWindow span_window(const TileParams& T, int lt, int r2, int win_words, bool direct) {
+    SpanWindow w;
+    const int ntx = (T.rw + kTileX - 1) / kTileX;
+    const int i0 = (lt % ntx) * kTileX, j0 = (lt / ntx) * kTileY;
+    const int r = isqrt_i32(r2);
+    const int xlo = T.rx0 + i0 - r, xhi = T.rx0 + min(i0 + kTileX, T.rw) + r;
+    const int ylo = T.ry0 + j0 - r, yhi = T.ry0 + min(j0 + kTileY, T.rh) - 1 + r;
+    w.inside = xlo >= 0 && xhi < T.ncols;
+    w.c0 = max(xlo, 0);
+    w.c1 = min(xhi, T.ncols - 1);
+    w.r0 = max(ylo, 0);
+    w.r1 = min(yhi, T.nrows - 1);
+    w.W = w.c1 - w.c0 + 1;
+    const int n = w.r1 - w.r0 + 1;
+    w.rows = w.W > 0 ? (win_words & ~3) / w.W : 0;
+    if (direct || w.rows < 1) {
+        w.rows = 0;
+        w.per = max(n, 1);
+    } else {
+        w.rows = min(w.rows, n);
+        const int chunks = max((n + w.rows - 1) / w.rows, 1);
+        w.per = w.rows * max((chunks + kSpanItemsPerTile - 1) / kSpanItemsPerTile, kSpanChunksPerItem);
+    }
+    return w;
+}
+
+// The window sums z relative to zbase and the counts in two int32 arrays
+// (native shared-memory atomics); a window cell receives at most one marker
+// per pixel of the tile, so |sum| <= kTileX * kTileY * zabs must stay below
+// 2^31.  Otherwise, and without the packed word, every marker goes straight
+// to the grid.
+__device__ __forceinline__ bool span_direct(const Scalars& s, int zmin, int zmax) {
+    const long long zabs = max((long long)zmax - s.zbase, s.zbase - (long long)zmin);
+    return !s.packed || zabs >= (1LL << 31) / (kTileX * kTileY);
+}
+
+// Lists the span work items of a tile's raster tiles (and layers of them):
+// one item per group of window chunks, so that the discs of one raster tile,
+// which differ in work by orders of magnitude (a lake's centre against its
+// shore), spread over the SMs.
+__device__ __forceinline__ void list_span_items(const BatchTables& bt, int t, int layers, bool direct, int win_words,
+                                                const FarLayout& far, BatchCounters* ctr) {
+    const TileParams& T = bt.tiles[t];
+    const int b0 = bt.rt_base[t], nrt = bt.rt_base[t + 1] - b0, rs2 = T.rs * T.rs;
+    const int lane = threadIdx.x & 31;
+    for (int k0 = 0; k0 < nrt * layers; k0 += blockDim.x) {
+        const int k = k0 + threadIdx.x;
+        int n = 0;
+        SpanWindow w;
+        if (k < nrt * layers) {
+            const int r2 = far.rtmax[b0 + k];
+            if (r2 > rs2) {
+                w = span_window(T, k % nrt, r2, win_words, direct);
+                if (w.c0 <= w.c1 && w.r0 <= w.r1) n = (w.r1 - w.r0 + w.per) / w.per;
+            }
+        }
+        int x = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        int base = 0;
+        if (lane == 31 && x) base = atomicAdd(&ctr->nspan, x);
+        base = __shfl_sync(0xffffffffu, base, 31) + x - n;
+        for (int e = 0; e < n; ++e) far.items[base + e] = make_int2(b0 + k, w.r0 + e * w.per);
+    }
+}
+
+// Per tile: the accumulator form of the span path (see decide_packing) and
+// its work items.
+__global__ void __launch_bounds__(256) k_decide(BatchTables bt, Scalars* sc, FarLayout far, BatchCounters* ctr,
+                                                int win_words) {
+    __shared__ int direct;
     const int t = blockIdx.x, l = threadIdx.x;
     const TileParams& T = bt.tiles[t];
     Scalars* s = sc + t;
-    int mx = s->max_r2[l];
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (l == 0) {
-        int packed, K;
-        long long zbase;
-        decide_packing(mx, (long long)T.rw * T.rh, s->bbox[4], s->bbox[5], packed, K, zbase);
-        s->packed = packed;
-        s->kbits = K;
-        s->zbase = zbase;
+    if (l < 32) {
+        int mx = s->max_r2[l];
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (l == 0) {
+            int packed, K;
+            long long zbase;
+            decide_packing(mx, (long long)T.rw * T.rh, s->bbox[4], s->bbox[5], packed, K, zbase);
+            s->packed = packed;
+            s->kbits = K;
+            s->zbase = zbase;
+            direct = span_direct(*s, s->bbox[4], s->bbox[5]);
+        }
     }
+    __syncthreads();
+    list_span_items(bt, t, 1, direct != 0, win_words, far, ctr);
 }
 
 __device__ __forceinline__ void emit_span(int row, int a, int b, int ncols, int nrows, bool packed,
@@ -991,99 +1139,109 @@ __device__ __forceinline__ void emit_span(int row, int a, int b, int ncols, int 
     }
 }
 
+// The rows of one disc inside a chunk, walked from a per-lane start and
+// wrapping at the last one: half_width() is floor(sqrt(R2 - dy^2)) of the
+// current row, row its offset in the window.
+//
+// R2 < 2^20: t = R2 - dy^2 + 1/2 is exact in a float, and for k^2 <= t - 1/2 <
+// (k+1)^2, k < 1024, its root lies at least 1/(4k+4) > 2.4e-4 from both k and
+// k+1, twice the error of the hardware estimate (relative 2^-23, so 1.3e-4);
+// the estimate rounded down is therefore the half-width itself.  The floor
+// is taken by adding 2^23 with rounding towards minus infinity, which leaves
+// the integer in the low mantissa bits: no conversion instructions.  Larger
+// discs take the estimate and one exact integer step each way.
+struct SpanRows {
+    float R2h, dyf, dy_last, back;
+    int row, row_back, stride, R2;
+    bool small;
+    __device__ __forceinline__ SpanRows(int R2_, int dy, int dy_last_, int nrow, int row_, int stride_)
+        : R2h((float)R2_ + 0.5f), dyf((float)dy), dy_last((float)dy_last_), back((float)(nrow - 1)), row(row_),
+          row_back((nrow - 1) * stride_), stride(stride_), R2(R2_), small(R2_ < (1 << 20)) {}
+    __device__ __forceinline__ int half_width() const {
+        if (small) return __float_as_int(__fadd_rd(sqrt_est(fmaf(-dyf, dyf, R2h)), 8388608.0f)) - 0x4B000000;
+        const int dy = (int)dyf;
+        const unsigned t2 = (unsigned)R2 - (unsigned)(dy * dy);
+        unsigned w = (unsigned)sqrt_est((float)t2);
+        w -= (w * w > t2) ? 1u : 0u;
+        w += ((w + 1) * (w + 1) <= t2) ? 1u : 0u;
+        return (int)w;
+    }
+    __device__ __forceinline__ void next() {
+        const bool wrap = dyf == dy_last;
+        dyf = wrap ? dyf - back : dyf + 1.0f;
+        row = wrap ? row - row_back : row + stride;
+    }
+};
+
 // Span path: every pixel with R2 > rs^2 adds its disc as row spans (+v at
 // the first cell, -v after the last, into the per-row difference words).
-// One CTA (32 x 8 threads) per 32 x kTileY raster tile.  The tile's discs
-// cover a window of grid cells a little larger than the tile by the largest
-// radius; the window is processed in chunks of whole rows that fit
-// `win_words` 8-byte cells of shared memory.  For each chunk every disc of
-// the tile adds its row spans' markers (z - zbase and 1 at the first cell,
-// their negatives after the last) to two int32 arrays with native
-// shared-memory atomics,
-// and each touched cell is then added to the grid's difference array as one
-// packed word, (sum << K) + count, with one coalesced global atomic.  The
-// markers of a tile's discs fall on far fewer distinct cells than there are
-// markers (neighbouring pixels' discs share rows and end near each other),
-// so the grid sees a fraction of the global atomics of the direct path, and
-// those it sees are contiguous.  The sum is the same: the words add modulo
-// 2^64 in any order and the packed form is linear.  Tiles with the unpacked
-// accumulators (separate int64 Z and int32 C), with a z range the int32
-// window sums could overflow, or with windows wider than one chunk row,
-// take the direct path.
-constexpr int kSpanWindowWords = 4096;      // default: 32 KB per CTA (two int32 arrays)
-constexpr int kSpanWindowMaxWords = 26624;  // 208 KB, the most one CTA may take
-
-// Minimum (or maximum) of v over a 32 x 8 CTA; red: 8 ints of shared memory.
-template <bool kMax>
-__device__ __forceinline__ int block_reduce_int(int v, int* red) {
-    v = kMax ? __reduce_max_sync(0xffffffffu, v) : __reduce_min_sync(0xffffffffu, v);
-    if (threadIdx.x == 0) red[threadIdx.y] = v;
-    __syncthreads();
-    int r = red[0];
-#pragma unroll
-    for (int k = 1; k < 8; ++k) r = kMax ? max(r, red[k]) : min(r, red[k]);
-    __syncthreads();
-    return r;
-}
-
-__global__ void __launch_bounds__(256) k_scatter_window(BatchTables bt, const int2* __restrict__ pix,
+// Persistent CTAs (32 x 8 threads) take the work items of list_span_items:
+// the rows of one group of chunks of one 32 x kTileY raster tile's window,
+// whose chunks of whole rows fit `win_words` 8-byte cells of shared memory.
+// For each chunk every disc of the tile adds its row spans' markers (z -
+// zbase and 1 at the first cell, their negatives after the last) to two int32
+// arrays with native shared-memory atomics, and each touched cell is then
+// added to the grid's difference array as one packed word, (sum << K) +
+// count, with one coalesced global atomic.  The markers of a tile's discs
+// fall on far fewer distinct cells than there are markers (neighbouring
+// pixels' discs share rows and end near each other), so the grid sees a
+// fraction of the global atomics of the direct path, and those it sees are
+// contiguous.  The sum is the same: the words add modulo 2^64 in any order
+// and the packed form is linear.  Tiles with the unpacked accumulators
+// (separate int64 Z and int32 C), with a z range the int32 window sums could
+// overflow, or with windows wider than one chunk row, take the direct path.
+__global__ void __launch_bounds__(256) k_scatter_window(BatchTables bt, const int2* __restrict__ pix_all,
                                                         const Scalars* __restrict__ sc,
                                                         unsigned long long* __restrict__ D_all,
-                                                        int* __restrict__ Dc_all, int win_words) {
+                                                        int* __restrict__ Dc_all, int win_words, FarLayout far,
+                                                        BatchCounters* __restrict__ ctr, int nrt_layer,
+                                                        int64_t lstride) {
     extern __shared__ int swin[];              // 2 x win_words: z - zbase sums, then counts
-    __shared__ int red[8];
-    const int t = find_tile(bt.rt_base, bt.ntiles, blockIdx.x);
+    __shared__ int s_item;
+    const int count = ctr->nspan;
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    const int ww4 = win_words & ~3;           // whole int4s
+    int* sz = swin;                           // z - zbase sums
+    int* scn = swin + ww4;                    // counts
+    if (count > 0)                            // each chunk leaves the window zeroed
+        for (int e = tid; e < ww4 >> 1; e += 256) reinterpret_cast<int4*>(swin)[e] = make_int4(0, 0, 0, 0);
+    for (;;) {
+    __syncthreads();                           // the previous item's reads of s_item are done
+    if (tid == 0) s_item = atomicAdd(&ctr->span_next, 1);
+    __syncthreads();
+    if (s_item >= count) break;
+    const int2 item = far.items[s_item];
+    const int layer = nrt_layer ? item.x / nrt_layer : 0;
+    const int rt = item.x - layer * nrt_layer;
+    const int t = find_tile(bt.rt_base, bt.ntiles, rt);
     const TileParams T = bt.tiles[t];          // by value: the loops below keep what they use in registers
-    const int lt = blockIdx.x - __ldg(&bt.rt_base[t]);
+    const int2* pix = pix_all + T.pix_off + layer * lstride;
+    const int lt = rt - __ldg(&bt.rt_base[t]);
     const int ntx = (T.rw + kTileX - 1) / kTileX;
     const int i = (lt % ntx) * kTileX + threadIdx.x;
     const int jt = (lt / ntx) * kTileY + threadIdx.y;
     const int rs2 = T.rs * T.rs;
     const int px = T.rx0 + i;
+    const Scalars& s = sc[t];
+    const bool direct = span_direct(s, s.bbox[4], s.bbox[5]);
+    const SpanWindow win = span_window(T, lt, far.rtmax[item.x], win_words, direct);
     int R2v[kDenseSub], zv[kDenseSub], rv[kDenseSub];
-    int xlo = INT_MAX, xhi = INT_MIN, ylo = INT_MAX, yhi = INT_MIN;
 #pragma unroll
     for (int sub = 0; sub < kDenseSub; ++sub) {
         const int j = jt + 8 * sub;
         int R2 = -1, z = 0;
         if (i < T.rw && j < T.rh) {
-            const int2 r = pix[T.pix_off + (int64_t)j * T.rw + i];
+            const int2 r = pix[(int64_t)j * T.rw + i];
             z = r.x;
             R2 = r.y;
         }
-        const int r = R2 > rs2 ? isqrt_i32(R2) : -1;
         R2v[sub] = R2;
         zv[sub] = z;
-        rv[sub] = r;
-        if (r >= 0) {
-            const int py = T.ry0 + j;
-            xlo = min(xlo, px - r);
-            xhi = max(xhi, px + r + 1);
-            ylo = min(ylo, py - r);
-            yhi = max(yhi, py + r);
-        }
+        rv[sub] = R2 > rs2 ? isqrt_i32(R2) : -1;
     }
-    xlo = block_reduce_int<false>(xlo, red);
-    if (xlo == INT_MAX) return;                 // no disc in this tile takes the span path
-    xhi = block_reduce_int<true>(xhi, red);
-    ylo = block_reduce_int<false>(ylo, red);
-    yhi = block_reduce_int<true>(yhi, red);
-    const int c0 = max(xlo, 0), c1 = min(xhi, T.ncols - 1);
-    const int r0 = max(ylo, 0), r1 = min(yhi, T.nrows - 1);
-    if (c0 > c1 || r0 > r1) return;             // every disc lies outside the grid
-    const Scalars& s = sc[t];
-    const bool packed = s.packed != 0;
     unsigned long long* D = D_all + T.cell_off;
     int* Dc = Dc_all + T.cell_off;
-    const int W = c1 - c0 + 1;
-    const int CH = (win_words & ~3) / W;
-    // the window sums z relative to zbase and the counts in two int32 arrays
-    // (native shared-memory atomics); a window cell receives at most one
-    // marker per pixel of the tile, so |sum| <= kTileX * kTileY * zabs must
-    // stay below 2^31
-    const long long zabs = max((long long)s.bbox[5] - s.zbase, s.zbase - (long long)s.bbox[4]);
-    const bool fits32 = zabs < (1LL << 31) / (kTileX * kTileY);
-    if (!packed || CH < 1 || !fits32) {
+    if (win.rows < 1) {
         // direct path: every span's markers straight to the grid
 #pragma unroll 1
         for (int sub = 0; sub < kDenseSub; ++sub) {
@@ -1096,26 +1254,21 @@ __global__ void __launch_bounds__(256) k_scatter_window(BatchTables bt, const in
             for (int dy = 0; dy <= r; ++dy) {
                 const long long t2 = (long long)R2 - (long long)dy * dy;
                 while ((long long)w * w > t2) --w;
-                emit_span(py + dy, px - w, px + w, T.ncols, T.nrows, packed, v, z, D, Dc);
-                if (dy) emit_span(py - dy, px - w, px + w, T.ncols, T.nrows, packed, v, z, D, Dc);
+                emit_span(py + dy, px - w, px + w, T.ncols, T.nrows, s.packed != 0, v, z, D, Dc);
+                if (dy) emit_span(py - dy, px - w, px + w, T.ncols, T.nrows, s.packed != 0, v, z, D, Dc);
             }
         }
-        return;
+        continue;
     }
-    const int tid = threadIdx.y * 32 + threadIdx.x;
+    const int W = win.W, CH = win.rows, c0 = win.c0;
+    const int r0 = item.y, r1 = min(item.y + win.per - 1, win.r1);
+    const bool inside = win.inside;
     const int ncols = T.ncols;
-    const int ww4 = win_words & ~3;           // whole int4s: the chunk is zeroed 16 bytes at a time
-    int* sz = swin;                           // z - zbase sums
-    int* scn = swin + ww4;                    // counts
+    const int zbase = (int)s.zbase;           // |z - zbase| fits (span_direct)
+    const int kbits = s.kbits;
 #pragma unroll 1
     for (int y0 = r0; y0 <= r1; y0 += CH) {
         const int y1 = min(y0 + CH - 1, r1);
-        const int nw = (y1 - y0 + 1) * W;
-        for (int e = tid; e < (nw + 3) >> 2; e += 256) {
-            reinterpret_cast<int4*>(sz)[e] = make_int4(0, 0, 0, 0);
-            reinterpret_cast<int4*>(scn)[e] = make_int4(0, 0, 0, 0);
-        }
-        __syncthreads();
 #pragma unroll 1
         for (int sub = 0; sub < kDenseSub; ++sub) {
             const int r = rv[sub];
@@ -1123,46 +1276,57 @@ __global__ void __launch_bounds__(256) k_scatter_window(BatchTables bt, const in
             const int py = T.ry0 + jt + 8 * sub;
             const int ya = max(py - r, y0), yb = min(py + r, y1);
             if (ya > yb) continue;
-            const unsigned R2 = (unsigned)R2v[sub];
-            const int zr = (int)((long long)zv[sub] - s.zbase);
+            const int zr = zv[sub] - zbase;
             // the lanes of a warp are 32 neighbouring pixels of one row, whose
             // markers on a common row often fall on one cell (same-address
             // atomics serialise); each lane starts its rows at its own offset
-            // so that the warp's markers spread over the chunk's rows.  The
-            // half-width floor(sqrt(t2)) comes from the hardware square-root
-            // estimate, within one of it for t2 < 2^31, and one exact step
-            // each way.
+            // so that the warp's markers spread over the chunk's rows
             const int nrow = yb - ya + 1;
-            int y = ya + (int)(threadIdx.x % (unsigned)nrow);
-            for (int k = 0; k < nrow; ++k, y = (y == yb) ? ya : y + 1) {
-                const int dy = y - py;
-                const unsigned t2 = R2 - (unsigned)(dy * dy);
-                unsigned w = (unsigned)sqrt_est((float)t2);
-                w -= (w * w > t2) ? 1u : 0u;
-                w += ((w + 1) * (w + 1) <= t2) ? 1u : 0u;
-                const int a = max(px - (int)w, 0), b = px + (int)w + 1;
-                if (a >= ncols || b <= 0) continue;       // this row's span misses the grid
-                const int row = (y - y0) * W - c0;     // a and b lie in [c0, c1]
-                atomicAdd(&sz[row + a], zr);
-                atomicAdd(&scn[row + a], 1);
-                if (b < ncols) {
-                    atomicAdd(&sz[row + b], -zr);
-                    atomicAdd(&scn[row + b], -1);
+            const int y = ya + (int)(threadIdx.x % (unsigned)nrow);
+            SpanRows rows(R2v[sub], y - py, yb - py, nrow, (y - y0) * W - c0, W);
+            if (inside) {
+#pragma unroll 2
+                for (int k = 0; k < nrow; ++k) {
+                    const int w = rows.half_width();
+                    const int a = rows.row + px - w, b = rows.row + px + 1 + w;
+                    atomicAdd(&sz[a], zr);
+                    atomicAdd(&scn[a], 1);
+                    atomicAdd(&sz[b], -zr);
+                    atomicAdd(&scn[b], -1);
+                    rows.next();
+                }
+            } else {
+                for (int k = 0; k < nrow; ++k) {
+                    const int w = rows.half_width();
+                    const int a = max(px - w, 0), b = px + w + 1;
+                    if (a < ncols && b > 0) {                // else this row's span misses the grid
+                        atomicAdd(&sz[rows.row + a], zr);    // a and b lie in [c0, c1]
+                        atomicAdd(&scn[rows.row + a], 1);
+                        if (b < ncols) {
+                            atomicAdd(&sz[rows.row + b], -zr);
+                            atomicAdd(&scn[rows.row + b], -1);
+                        }
+                    }
+                    rows.next();
                 }
             }
         }
         __syncthreads();
-        // one packed word per touched cell: (sum zrel << K) + count, modulo 2^64
+        // one packed word per touched cell: (sum zrel << K) + count, modulo
+        // 2^64; the cells read are zeroed for the next chunk
         for (int rr = threadIdx.y; rr <= y1 - y0; rr += 8) {
             unsigned long long* dst = D + (int64_t)(y0 + rr) * ncols + c0;
             for (int c = threadIdx.x; c < W; c += 32) {
                 const int zs = sz[rr * W + c], cn = scn[rr * W + c];
-                if (zs | cn)
-                    atomicAdd(&dst[c], ((unsigned long long)(long long)zs << s.kbits) +
-                                           (unsigned long long)(long long)cn);
+                if (zs | cn) {
+                    atomicAdd(&dst[c], ((unsigned long long)(long long)zs << kbits) + (unsigned long long)(long long)cn);
+                    sz[rr * W + c] = 0;
+                    scn[rr * W + c] = 0;
+                }
             }
         }
         __syncthreads();
+    }
     }
 }
 

@@ -258,7 +258,7 @@ dnni_status srv_launch(dnni_server* s, SrvSlot& sl, std::vector<SrvItem>& items,
     a.sc = (Scalars*)take(z.sc);
     a.ctr = (BatchCounters*)take(z.ctr);
     a.pix = (int2*)take(z.pix);
-    a.far = (FarSlot*)take(z.far);
+    a.far = (int4*)take(z.far);
     a.D = (unsigned long long*)take(z.D);
     a.Dc = (int*)take(z.Dc);
     a.sorted = (int4*)take(z.sorted);

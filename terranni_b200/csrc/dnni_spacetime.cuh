@@ -165,13 +165,14 @@ __global__ void __launch_bounds__(256) k_st_scatter(const int32_t* __restrict__ 
 // The site maps hold input indices (the batch's gids); xyz is the input.
 __global__ void __launch_bounds__(256) k_st_lift(TileParams T, StParams P, const uint32_t* __restrict__ site,
                                                  const int32_t* __restrict__ xyz, int2* __restrict__ pix,
-                                                 Scalars* __restrict__ sc) {
+                                                 Scalars* __restrict__ sc, int* __restrict__ rtmax, int nrt) {
     const int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    int R2 = -1;
+    int R2 = -1, rt = 0;
     if (w < (2LL * P.rt + 1) * P.npix) {
         const int s = (int)(w / P.npix);
         const int64_t p = w - (int64_t)s * P.npix;
         const int i = (int)(p % T.rw), j = (int)(p / T.rw);
+        rt = s * nrt + (j / kTileY) * ((T.rw + kTileX - 1) / kTileX) + i / kTileX;
         const long long px = (long long)(T.rx0 + i) * T.cs, py = (long long)(T.ry0 + j) * T.cs;
         unsigned long long bd = ~0ull;
         uint32_t bg = 0xFFFFFFFFu;
@@ -207,21 +208,37 @@ __global__ void __launch_bounds__(256) k_st_lift(TileParams T, StParams P, const
     const int m = __reduce_max_sync(0xffffffffu, R2);
     if ((threadIdx.x & 31) == 0 && m >= 0)
         atomicMax(&sc->max_r2[(blockIdx.x * 8 + (threadIdx.x >> 5)) & (kStatSlots - 1)], m);
+    // the largest R2 of each raster tile of each slice, for the span work items
+    if (m > T.rs * T.rs) {
+        const unsigned grp = __match_any_sync(0xffffffffu, rt);
+        const int g = __reduce_max_sync(grp, R2);
+        if ((threadIdx.x & 31) == (unsigned)(__ffs(grp) - 1) && g > T.rs * T.rs) atomicMax(&rtmax[rt], g);
+    }
 }
 
 // Accumulator form for `layers` stacked slices (decide_packing with the
 // per-cell count bound multiplied by the slice count).
-__global__ void k_st_decide(Scalars* sc, int zmin, int zmax, long long npix, int layers) {
-    int mx = sc->max_r2[threadIdx.x];
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (threadIdx.x == 0) {
-        int packed, K;
-        long long zbase;
-        decide_packing(mx, npix, zmin, zmax, packed, K, zbase, layers);
-        sc->packed = packed;
-        sc->kbits = K;
-        sc->zbase = zbase;
+// Also records the points' z range and lists the span work items.
+__global__ void __launch_bounds__(1024) k_st_decide(BatchTables bt, Scalars* sc, int zmin, int zmax, long long npix,
+                                                    int layers, FarLayout far, BatchCounters* ctr, int win_words) {
+    __shared__ int direct;
+    if (threadIdx.x < 32) {
+        int mx = sc->max_r2[threadIdx.x];
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (threadIdx.x == 0) {
+            int packed, K;
+            long long zbase;
+            decide_packing(mx, npix, zmin, zmax, packed, K, zbase, layers);
+            sc->packed = packed;
+            sc->kbits = K;
+            sc->zbase = zbase;
+            sc->bbox[4] = zmin;
+            sc->bbox[5] = zmax;
+            direct = span_direct(*sc, zmin, zmax);
+        }
     }
+    __syncthreads();
+    list_span_items(bt, 0, layers, direct != 0, win_words, far, ctr);
 }
 
 // Stencil and divide over `layers` stacked pixel rasters (layer stride lstride): each
@@ -416,16 +433,21 @@ static dnni_status spacetime_run(dnni_ctx* c, const dnni_workpackage* wp, const 
     k_init_scalars<<<1, 32, 0, st>>>(bt, a.sc, a.ctr);
     int2* pix = (int2*)c->st.pix.p;
     const int64_t lifts = (int64_t)S * npix;
-    k_st_lift<<<(unsigned)((lifts + 255) / 256), 256, 0, st>>>(T, P, (const uint32_t*)c->st.site.p, dxyz, pix,
-                                                               a.sc);
-    k_st_decide<<<1, 32, 0, st>>>(a.sc, m > 0 ? zmin : 1, m > 0 ? zmax : 0, npix, S);
+    // the worklist buffer serves the span work items of every slice (no far
+    // groups here, and at most 33 slices: 33 * (4 + 512) B of the 32 KB per
+    // raster tile)
+    const int nrt = hb.rt_base.back();
+    const FarLayout far = far_layout(a.far, 0, (int64_t)S * nrt);
+    static_assert((2 * kStMaxRadius + 1) * (4 + 8 * kSpanItemsPerTile) + 512 <= kTileX * kTileY * kFarSlotBytes,
+                  "the slices' span work items fit the worklist buffer");
+    CK(cudaMemsetAsync(far.rtmax, 0xFF, sizeof(int) * (size_t)S * nrt, st));
+    k_st_lift<<<(unsigned)((lifts + 255) / 256), 256, 0, st>>>(T, P, (const uint32_t*)c->st.site.p, dxyz, pix, a.sc,
+                                                               far.rtmax, nrt);
+    k_st_decide<<<1, 1024, 0, st>>>(bt, a.sc, m > 0 ? zmin : 1, m > 0 ? zmax : 0, npix, S, far, a.ctr, hb.win_words);
     if (timing) CK(cudaEventRecord(c->ev[2], st));
     CK(cudaMemsetAsync(a.D, 0, sizeof(unsigned long long) * (size_t)cells, st));
     CK(cudaMemsetAsync(a.Dc, 0, sizeof(int) * (size_t)cells, st));
-    const int nrt = hb.rt_base.back();
-    for (int s = 0; s < S; ++s)
-        k_scatter_window<<<nrt, dim3(32, 8), sizeof(unsigned long long) * hb.win_words, st>>>(
-            bt, pix + (int64_t)s * npix, a.sc, a.D, a.Dc, hb.win_words);
+    launch_spans(hb, bt, a, pix, far, nrt, npix, c->sm_count, st);
     if (timing) CK(cudaEventRecord(c->ev[3], st));
     k_rowscan<<<hb.grow_base.back(), kScanThreads, 0, st>>>(bt, a.D, a.Dc, a.sc);
     launch_st_final(bt, hb.ct_base.back(), hb.rs, pix, S, npix, a.sc, a.D, a.Dc, dh, st);
