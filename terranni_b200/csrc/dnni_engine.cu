@@ -133,7 +133,8 @@ void set_dense_smem_attr() {
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lock(mu);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(k_near_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem);
+        cudaFuncSetAttribute(k_near_dense<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem);
+        cudaFuncSetAttribute(k_near_dense<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem);
         cudaFuncSetAttribute(k_scatter_window, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(sizeof(unsigned long long) * kSpanWindowMaxWords));
         done[dev] = true;
@@ -157,7 +158,7 @@ void launch_spans(const HostBatch& hb, const BatchTables& bt, const DevArrays& a
 void launch_prologue(const HostBatch& hb, const BatchTables& bt, const DevArrays& a, const int32_t* d_xyz,
                      cudaStream_t st, bool bbox = true) {
     const int n = (int)hb.tiles.size();
-    k_init_scalars<<<n, 32, 0, st>>>(bt, a.sc, a.ctr);
+    k_init_scalars<<<n, 256, 0, st>>>(bt, a.sc, a.ctr, far_layout(a.far, hb.n_far, hb.rt_base.back()).rtmax);
     const int nchunk = hb.chunk_base.back();
     if (bbox && nchunk > 0) k_bbox<<<nchunk, 256, 0, st>>>(bt, d_xyz, a.sc, a.ctr);
 }
@@ -189,8 +190,13 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
     if (ev) cudaEventRecord(ev[0], st);
     const int nrt = hb.rt_base.back();
     const FarLayout far = far_layout(a.far, hb.n_far, nrt);
-    k_near_dense<<<nrt, dim3(32, 8), kDenseSmem, st>>>(bt, a.sorted, a.start, a.pix, d_site, far, a.sc, a.ctr,
-                                                       hb.far_blocks, hb.dense_band);
+    // a raster tile goes to several CTAs while the tiles alone leave the SMs
+    // (four CTAs each) without two rounds of work
+    int split = 1;
+    while (split < kTileY / 8 && (int64_t)nrt * split < 8 * (int64_t)sms) split *= 2;
+    const auto dense = d_gid ? k_near_dense<true> : k_near_dense<false>;
+    dense<<<nrt * split, 256, kDenseSmem, st>>>(bt, a.sorted, a.start, a.pix, d_site, far, a.sc, a.ctr, hb.far_blocks,
+                                                hb.dense_band, split);
     if (ev) cudaEventRecord(ev[4], st);
     if (nchunk > 0)
         k_near_far<<<sms * 6, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site,

@@ -81,9 +81,11 @@ __device__ __forceinline__ int find_tile(const B* __restrict__ base, int ntiles,
 // point passes
 // ---------------------------------------------------------------------------
 
-__global__ void k_init_scalars(BatchTables bt, Scalars* sc, BatchCounters* ctr) {
+__global__ void __launch_bounds__(256) k_init_scalars(BatchTables bt, Scalars* sc, BatchCounters* ctr, int* rtmax) {
     const int t = blockIdx.x, l = threadIdx.x;
     Scalars* s = sc + t;
+    if (rtmax)
+        for (int k = bt.rt_base[t] + l; k < bt.rt_base[t + 1]; k += blockDim.x) rtmax[k] = -1;
     if (l == 0) {
         s->bbox[0] = INT_MAX; s->bbox[1] = INT_MIN;
         s->bbox[2] = INT_MAX; s->bbox[3] = INT_MIN;
@@ -411,15 +413,12 @@ __global__ void k_block_near(BatchTables bt, const int* __restrict__ rownear, in
 // nearest site per raster pixel
 // ---------------------------------------------------------------------------
 
-// Records a settled pixel: its record and (optionally) its site; returns
-// its R2.
-__device__ __forceinline__ int settle_pixel(const TileParams& T, int i, int j, const Best& b, int2* __restrict__ pix,
-                                            uint32_t* __restrict__ site) {
-    const int R2 = r2_of(b.d2, (long long)T.cs * T.cs, T.r2cap);
+// Records a settled pixel: its record and (optionally) its site.
+__device__ __forceinline__ void settle_pixel(const TileParams& T, int i, int j, const Best& b, int R2,
+                                             int2* __restrict__ pix, uint32_t* __restrict__ site) {
     const int64_t o = (int64_t)j * T.rw + i;
     pix[T.pix_off + o] = make_int2(b.z, R2);
     if (site && T.site_off >= 0) site[T.site_off + o] = b.gid;
-    return R2;
 }
 
 // Statistics of settled pixels, accumulated per thread and flushed once per
@@ -498,44 +497,49 @@ static_assert(sizeof(FarGroup) == 144 && 2048 / 32 * sizeof(FarGroup) + 2 * 260 
 constexpr int kPixFar = -2;
 constexpr int kFarBlocksDefault = 1;   // far groups of 8 x 4 pixels
 
-// Dense pass.  One CTA per 32 x kTileY raster tile of a work package
-// (blockDim 32 x 8; warp w takes pixel rows w, w + 8, ... of the tile): the
-// tile's bin window (bin rings
-// of every pixel) is staged in shared memory and the rings are searched
-// there; windows too large for shared memory use the global arrays.  A warp
-// with pixels the rings do not settle appends its whole row as one group of
-// 32 slots to the far worklist.  With no points every pixel is settled as
-// "no site".
+// Dense pass.  One CTA (256 threads) per 32 x kTileY raster tile of a work
+// package, or per 1/split of its rows; each warp takes 8 x 4 blocks of
+// pixels.  The block's bin window (bin rings of every pixel) is staged in
+// shared memory and the rings are searched there; windows too large for
+// shared memory use the global arrays.  Pixels the rings do not settle go to
+// the far worklist, 32 to a group: the warp's 8 x 4 block, or a 32 x 1 row.
+// With no points every pixel is settled as "no site".
+template <bool kDup>
 __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int4* __restrict__ pts_all,
                                                        const int* __restrict__ start_all, int2* __restrict__ pix,
                                                        uint32_t* __restrict__ site, FarLayout far,
                                                        Scalars* __restrict__ sc, BatchCounters* __restrict__ ctr,
-                                                       int far_blocks, int band0) {
+                                                       int far_blocks, int band0, int split) {
     extern __shared__ int4 smem[];
     int4* s_pts = smem;
-    int* s_lstart = (int*)(smem + kWinMaxPts);
+    int* s_lstart = (int*)(smem + kWinMaxPts + 1);
     int* s_gstart = s_lstart + kWinMaxBins + 1;
     __shared__ int s_rowbase[kWinMaxRows];
-    __shared__ int s_total;
     __shared__ int s_max[8];
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    const int t = find_tile(bt.rt_base, bt.ntiles, blockIdx.x);
-    const TileParams& T = bt.tiles[t];
+    const int tid = threadIdx.x;
+    const int rt = blockIdx.x / split;
+    const int t = find_tile(bt.rt_base, bt.ntiles, rt);
+    const TileParams T = bt.tiles[t];   // by value: what the loops use stays in registers
     const BinGrid g = T.bg;
+    const float inv_bs = 1.0f / (float)g.bs, inv_cs2 = 1.0f / ((float)T.cs * (float)T.cs);
     const int4* pts = pts_all + T.srt_off;
     const int* start = start_all + T.bin_off;
-    const int lt = blockIdx.x - __ldg(&bt.rt_base[t]);
+    const int lt = rt - __ldg(&bt.rt_base[t]);
     const int ntx = (T.rw + kTileX - 1) / kTileX;
-    const int i0 = (lt % ntx) * kTileX, j0 = (lt / ntx) * kTileY;
-    const int i = i0 + threadIdx.x;
+    const int rows = kTileY / split;
+    const int i0 = (lt % ntx) * kTileX, j0 = (lt / ntx) * kTileY + (blockIdx.x - rt * split) * rows;
+    if (j0 >= T.rh) return;
     const int warp = tid >> 5, lane = tid & 31;
+    // a warp's 8 x 4 pixels inside each 32 x 8 strip
+    const int bi = i0 + (warp & 3) * 8, i = bi + (lane & 7);
+    const int sj = (warp >> 2) * 4;
     // the tile's rows go in bands, each with its own staged window: band0
     // rows (8, 16, 32 or 64: the shape of the pixel block that shares one
     // window, a tuning choice) when that window fits shared memory, else
     // halves, down to 8 rows
     StatAcc acc;
-    int band = band0;
-    for (int jb = 0; jb < kTileY && j0 + jb < T.rh; jb += band) {
+    int band = min(min(band0, rows), T.band);
+    for (int jb = 0; jb < rows && j0 + jb < T.rh; jb += band) {
     int wx0 = 0, wy0 = 0, wnx = 0, wny = 0;
     bool staged = false;
     while (T.npts > 0) {
@@ -577,47 +581,51 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
                 if (lane == 0) s_rowbase[r] = rowsum;
             }
             __syncthreads();
-            if (warp == 0) {
-                int run = 0;
+            int total = 0;
+            for (int r0 = 0; r0 < wny; r0 += 32)
+                total += __reduce_add_sync(0xffffffffu, r0 + lane < wny ? s_rowbase[r0 + lane] : 0);
+            if (total > kWinMaxPts && band > 8) {     // too many points: a shorter band
+                band >>= 1;
+                __syncthreads();
+                continue;
+            }
+            staged = total <= kWinMaxPts;
+            if (staged) {
+                // every warp scans the row sums and places its own rows: adds
+                // the row's base to the bins' starts and copies the points
+                // (asynchronous 16-byte copies, all in flight before one
+                // wait); the bins of one window row inside one block are
+                // consecutive in both layouts, lanes striding over the points
+                const int cb0 = wx0 >> 3, cb1 = (wx0 + wnx - 1) >> 3;
+                int base = 0;
                 for (int r0 = 0; r0 < wny; r0 += 32) {
-                    const int r = r0 + lane;
-                    const int v = r < wny ? s_rowbase[r] : 0;
+                    const int v = r0 + lane < wny ? s_rowbase[r0 + lane] : 0;
                     int x = v;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
                         const int y = __shfl_up_sync(0xffffffffu, x, o);
                         if (lane >= o) x += y;
                     }
-                    if (r < wny) s_rowbase[r] = run + x - v;
-                    run += __shfl_sync(0xffffffffu, x, 31);
+                    for (int r = r0 + warp; r < min(r0 + 32, wny); r += 8) {
+                        const int rb = base + __shfl_sync(0xffffffffu, x - v, r - r0);
+                        const int re = base + __shfl_sync(0xffffffffu, x, r - r0);
+                        int* ls = s_lstart + r * wnx;
+                        for (int c = lane; c < wnx; c += 32) ls[c] += rb;
+                        __syncwarp();
+                        for (int cb = cb0; cb <= cb1; ++cb) {
+                            const int xa = max(cb * 8 - wx0, 0), xb = cb * 8 + 8 - wx0;
+                            const int l0 = ls[xa], l1 = xb < wnx ? ls[xb] : re;
+                            const int4* src = pts + (s_gstart[r * wnx + xa] - l0);
+                            for (int q = l0 + lane; q < l1; q += 32) {
+                                __pipeline_memcpy_async(&s_pts[q], &src[q], sizeof(int4));
+                                // a copy of the last point follows it (scan_local32)
+                                if (q == total - 1) __pipeline_memcpy_async(&s_pts[total], &src[q], sizeof(int4));
+                            }
+                        }
+                    }
+                    base += __shfl_sync(0xffffffffu, x, 31);
                 }
-                if (lane == 0) { s_lstart[nwb] = run; s_total = run; }
-            }
-            __syncthreads();
-            for (int r = warp; r < wny; r += 8)
-                for (int c = lane; c < wnx; c += 32) s_lstart[r * wnx + c] += s_rowbase[r];
-            __syncthreads();
-            if (s_total > kWinMaxPts && band > 8) {   // too many points: a shorter band
-                band >>= 1;
-                __syncthreads();
-                continue;
-            }
-            staged = s_total <= kWinMaxPts;
-            if (staged) {
-                // copy the window's points run by run (asynchronous 16-byte
-                // copies, all in flight before one wait): the bins of one
-                // window row inside one block are consecutive in both layouts;
-                // one warp per run, lanes striding over its points
-                const int cb0 = wx0 >> 3, cb1 = (wx0 + wnx - 1) >> 3;
-                const int nseg = cb1 - cb0 + 1, nrun = nseg * wny;
-                for (int run = warp; run < nrun; run += 8) {
-                    const int r = run / nseg, sg = run - r * nseg;
-                    const int xa = (cb0 + sg) * 8 > wx0 ? (cb0 + sg) * 8 : wx0;
-                    const int xb = (cb0 + sg) * 8 + 7 < wx0 + wnx - 1 ? (cb0 + sg) * 8 + 7 : wx0 + wnx - 1;
-                    const int lk0 = r * wnx + (xa - wx0), lk1 = r * wnx + (xb - wx0);
-                    const int l0 = s_lstart[lk0], cntp = s_lstart[lk1 + 1] - l0, g0 = s_gstart[lk0];
-                    for (int q = lane; q < cntp; q += 32) __pipeline_memcpy_async(&s_pts[l0 + q], &pts[g0 + q], sizeof(int4));
-                }
+                if (tid == 0) s_lstart[nwb] = total;
                 __pipeline_commit();
                 __pipeline_wait_prior(0);
             }
@@ -625,9 +633,10 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
         }
         break;
     }
+    const bool fits32 = staged && window_fits32(g, BinWindow{wx0, wy0, wnx, wny, s_lstart, s_gstart, s_pts});
 #pragma unroll 1
-    for (int sub = 0; sub < band / 8; ++sub) {
-    const int j = j0 + jb + threadIdx.y + 8 * sub;
+    for (int sub = 0; sub < band / 8 && j0 + jb + 8 * sub < T.rh; ++sub) {
+    const int bj = j0 + jb + 8 * sub + sj, j = bj + (lane >> 3);
     const bool valid = i < T.rw && j < T.rh;
     int R2 = -1;
     bool far_pixel = false;
@@ -638,13 +647,15 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
             bool done;
             if (staged) {
                 const BinWindow w{wx0, wy0, wnx, wny, s_lstart, s_gstart, s_pts};
-                done = window_fits32(g, w) ? search_window_fast32(g, w, px, py, b) : search_window_fast(g, w, px, py, b);
+                done = fits32 ? search_window32<kDup>(g, w, inv_bs, px, py, b) : search_window_fast(g, w, px, py, b);
                 if (!done) b.idx = window_global_index(w, b.idx);
             } else {
                 done = search_bins(g, pts, start, px, py, b);
             }
             if (done) {
-                R2 = settle_pixel(T, i, j, b, pix, site);
+                R2 = fits32 && T.cs < (1 << 15) ? r2_of32((unsigned)b.d2, T.cs, inv_cs2, T.r2cap)
+                                                : r2_of(b.d2, (long long)T.cs * T.cs, T.r2cap);
+                settle_pixel(T, i, j, b, R2, pix, site);
             } else {
                 far_pixel = true;
             }
@@ -655,29 +666,26 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
         }
     }
     if (far_blocks) {
-        // marked for the block pass below: the record holds the best site
-        // found so far (-1: none) and kPixFar
-        if (far_pixel) pix[T.pix_off + (int64_t)j * T.rw + i] = make_int2(b.idx, kPixFar);
-    } else {
-        // worklist: a warp with any unsettled pixel appends its whole row of
-        // 32 pixels as one group (settled or absent pixels idle), so
-        // that a far warp later takes 32 neighbouring pixels of one tile
-        const unsigned mfar = __ballot_sync(0xffffffffu, far_pixel);
-        if (mfar) {
+        // a block with any unsettled pixel is one group of the worklist
+        if (__any_sync(0xffffffffu, far_pixel)) {
             int base = 0;
             if (lane == 0) {
                 base = atomicAdd(&ctr->nfar, 1);
-                *reinterpret_cast<int4*>(&far.groups[base]) = make_int4(t, (int)blockIdx.x, i0, j);
+                *reinterpret_cast<int4*>(&far.groups[base]) = make_int4(t, rt, bi, bj);
             }
             base = __shfl_sync(0xffffffffu, base, 0);
             far.groups[base].idx[lane] = far_pixel ? b.idx : kFarIdle;
         }
+    } else if (far_pixel) {
+        // marked for the row pass below: the record holds the best site found
+        // so far (-1: none) and kPixFar
+        pix[T.pix_off + (int64_t)j * T.rw + i] = make_int2(b.idx, kPixFar);
     }
     acc.add(T, R2, b.nev);
     }
     __syncthreads();     // the next band restages the window
     }
-    acc.flush(sc + t, blockIdx.x + threadIdx.y, false);
+    acc.flush(sc + t, blockIdx.x + warp, false);
     // the largest R2 of the pixels settled here, for the span work items (the
     // far pass raises it for the others)
     {
@@ -686,29 +694,26 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
         __syncthreads();
         if (tid < 32) {
             const int v = __reduce_max_sync(0xffffffffu, s_max[tid & 7]);
-            if (tid == 0) far.rtmax[blockIdx.x] = v;
+            if (tid == 0 && v >= 0) atomicMax(&far.rtmax[rt], v);
         }
     }
-    if (far_blocks) {
-        // worklist in 8 x 4 pixel blocks: a block with any unsettled pixel
-        // appends its 32 pixels as one group (lane = 8 * row + column), so
-        // that a far warp takes a compact patch whose discs overlap most;
-        // the records written above are visible after the barrier above
-        for (int blk = warp; blk < (kTileX / 8) * (kTileY / 4); blk += 8) {
-            const int bi = i0 + (blk % (kTileX / 8)) * 8, bj = j0 + (blk / (kTileX / 8)) * 4;
-            const int ii = bi + (lane & 7), jj = bj + (lane >> 3);
+    if (!far_blocks) {
+        // worklist in pixel rows: a row with any unsettled pixel is one group
+        // (the records written above are visible after the barrier)
+        for (int r = warp; r < rows; r += 8) {
+            const int ii = i0 + lane, jj = j0 + r;
             bool fp = false;
             int idx = -1;
             if (ii < T.rw && jj < T.rh) {
-                const int2 r = pix[T.pix_off + (int64_t)jj * T.rw + ii];
-                fp = r.y == kPixFar;
-                idx = r.x;
+                const int2 rec = pix[T.pix_off + (int64_t)jj * T.rw + ii];
+                fp = rec.y == kPixFar;
+                idx = rec.x;
             }
-            if (__ballot_sync(0xffffffffu, fp)) {
+            if (__any_sync(0xffffffffu, fp)) {
                 int base = 0;
                 if (lane == 0) {
                     base = atomicAdd(&ctr->nfar, 1);
-                    *reinterpret_cast<int4*>(&far.groups[base]) = make_int4(t, (int)blockIdx.x, bi, bj);
+                    *reinterpret_cast<int4*>(&far.groups[base]) = make_int4(t, rt, i0, jj);
                 }
                 base = __shfl_sync(0xffffffffu, base, 0);
                 far.groups[base].idx[lane] = fp ? idx : kFarIdle;
@@ -998,7 +1003,10 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
         }
         search_disc_warp(g, pts, start, bmask, smask, act, px, py, b);
         int R2 = -1;
-        if (act) R2 = settle_pixel(T, i, j, b, pix, site);
+        if (act) {
+            R2 = r2_of(b.d2, (long long)T.cs * T.cs, T.r2cap);
+            settle_pixel(T, i, j, b, R2, pix, site);
+        }
         StatAcc acc;
         acc.add(T, R2, b.nev);
         acc.flush(sc + t, blockIdx.x * 3 + (threadIdx.x >> 5), true);

@@ -101,6 +101,16 @@ inline void plan_bins(const int32_t bbox[6], int64_t n, double bin_target, TileP
     t.bg.n2x = (int32_t)(nbx / kBinsPerSuperEdge);
     t.bg.n2y = (int32_t)(nby / kBinsPerSuperEdge);
     t.bg.nbins = nbx * nby;
+    // the ring search's bands: halved while the window of an average place
+    // (evenly spread points) would pass the shared-memory arrays' sizes; a
+    // denser place halves its band further in the kernel
+    const double ppu = (double)n / ((double)W * (double)Hh), wx = (double)kTileX * cs + 5.0 * bs;
+    t.band = kTileY;
+    while (t.band > 8) {
+        const double wy = (double)t.band * cs + 5.0 * bs;
+        if (wx * wy * ppu <= 0.92 * kWinMaxPts && (wx / bs) * (wy / bs) <= kWinMaxBins) break;
+        t.band >>= 1;
+    }
 }
 
 }  // namespace dnni

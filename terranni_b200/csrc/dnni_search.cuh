@@ -70,6 +70,8 @@ struct TileParams {
     int32_t rx0, ry0, rw, rh;    // raster origin (cell index) and size
     int32_t r2cap;               // no pixel/cell pair is farther apart (cell units^2)
     int32_t rs;                  // small-disc radius of the stencil path
+    int32_t band;                // ring search: most pixel rows whose window is expected to fit
+    int32_t pad;
     int32_t has_gid;
     int64_t npts;
     double z_scale, z_offset;
@@ -151,6 +153,21 @@ DNNI_HD int r2_of(long long d2, long long cs2, int cap) {
     while (q > 0 && q * cs2 > d2) --q;
     while ((q + 1) * cs2 <= d2) ++q;
     return (int)(q < cap ? q : cap);
+}
+
+// The same for d2 < 2^31 and cs < 2^15, inv = 1 / cs^2: below 2^22 the float
+// estimate of the quotient is within one of it and corrected with an exact
+// remainder (a 32-bit divide costs several times more).
+DNNI_HD int r2_of32(unsigned d2, int cs, float inv, int cap) {
+    const unsigned cs2 = (unsigned)(cs * cs);
+    int q = (int)((float)d2 * inv);
+    if (q < (1 << 22)) {
+        const int r = (int)(d2 - (unsigned)q * cs2);
+        q += r < 0 ? -1 : (r >= (int)cs2 ? 1 : 0);
+    } else {
+        q = (int)(d2 / cs2);
+    }
+    return q < cap ? q : cap;
 }
 
 DNNI_HD int64_t bin_id(const BinGrid& g, int bx, int by) {
@@ -390,31 +407,45 @@ DNNI_HD bool search_window_fast(const BinGrid& g, const BinWindow& w, int px, in
 
 // The same search with 32-bit distances, for windows that span less than
 // 2^15 LAS units in each direction (squared distances then fit in 31 bits).
-// The (d^2, gid) part of the (d^2, gid, z) order is one 64-bit key.
+// The (d^2, gid) part of the (d^2, gid, z) order is one 64-bit key; z only
+// decides between equal keys (callers' duplicate gids, kDup).
 struct Best32 {
     unsigned long long key;   // d2 << 32 | gid; ~0 = none
-    int z;
     int idx;
     int nev;                  // candidate distance evaluations
 };
 
-DNNI_HD void consider32(Best32& b, const int4 p, int q, int px, int py) {
+template <bool kDup>
+DNNI_HD void consider32(Best32& b, const int4* lpts, int q, int px, int py) {
+    const int4 p = lpts[q];
     const int dx = p.x - px, dy = p.y - py;
     const unsigned d2 = (unsigned)(dx * dx) + (unsigned)(dy * dy);
     const unsigned long long key = ((unsigned long long)d2 << 32) | (unsigned)p.w;
-    if (key < b.key || (key == b.key && p.z < b.z)) {
+    if (kDup && __builtin_expect(key == b.key, 0) && b.idx >= 0 && p.z < lpts[b.idx].z) b.idx = q;
+    if (key < b.key) {
         b.key = key;
-        b.z = p.z;
         b.idx = q;
     }
 }
 
-DNNI_HD long long best32_d2(const Best32& b) { return b.key == ~0ull ? LLONG_MAX : (long long)(b.key >> 32); }
+DNNI_HD unsigned best32_d2(const Best32& b) { return (unsigned)(b.key >> 32); }   // none: 2^32 - 1
 
+// The points of window-local positions [s, e).  On the device two at a time:
+// the odd one out is then followed by the next bin's first point, or at the
+// window's end by a copy of the last point; both are real sites, so
+// evaluating one more changes no result.
+template <bool kDup>
 DNNI_HD void scan_local32(Best32& b, const int4* lpts, int s, int e, int px, int py) {
     b.nev += e - s;
-#pragma unroll 2
-    for (int q = s; q < e; ++q) consider32(b, lpts[q], q, px, py);
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+    for (int q = s; q < e; q += 2) {
+        consider32<kDup>(b, lpts, q, px, py);
+        consider32<kDup>(b, lpts, q + 1, px, py);
+    }
+#else
+    for (int q = s; q < e; ++q) consider32<kDup>(b, lpts, q, px, py);
+#endif
 }
 
 DNNI_HD bool window_fits32(const BinGrid& g, const BinWindow& w) {
@@ -423,66 +454,79 @@ DNNI_HD bool window_fits32(const BinGrid& g, const BinWindow& w) {
            ax + (long long)(g.nbx + 1) * g.bs < (1LL << 31) && ay + (long long)(g.nby + 1) * g.bs < (1LL << 31);
 }
 
-// ring_done for the 32-bit window path: every coordinate involved lies
-// within the window (less than 2^15 LAS units from the pixel), so the margins
-// and their squares fit in 32 bits; a missing best (none found) never stops.
-DNNI_HD bool ring_done32(long long best, int px, int py, const BinGrid& g, int x0, int x1, int y0, int y1) {
-    if (best == LLONG_MAX) return false;
-    int m = INT_MAX;
-    bool open = false;
-    const int gx0 = g.gx0, gy0 = g.gy0, bs = g.bs;
-    if (x0 > 0) { const int v = px - (gx0 + x0 * bs) + 1; m = v < m ? v : m; open = true; }
-    if (x1 < g.nbx - 1) { const int v = gx0 + (x1 + 1) * bs - px; m = v < m ? v : m; open = true; }
-    if (y0 > 0) { const int v = py - (gy0 + y0 * bs) + 1; m = v < m ? v : m; open = true; }
-    if (y1 < g.nby - 1) { const int v = gy0 + (y1 + 1) * bs - py; m = v < m ? v : m; open = true; }
-    if (!open) return true;
-    return best < (long long)m * m;
+// floor(x / u) for 0 <= x < 2^22 from a float product with 1/u (within one of
+// the quotient there), corrected with exact integer products.
+DNNI_HD int floor_div_est(int x, int u, float inv_u) {
+    int q = (int)((float)x * inv_u);
+    q -= q * u > x ? 1 : 0;
+    q += (q + 1) * u <= x ? 1 : 0;
+    return q;
+}
+
+// Bin rings 0..kRingsBins around the pixel on a window that fits 32 bits;
+// inv_bs = 1 / g.bs.  The pixel's own row of three bins first, then the rows
+// above and below and the second ring's rows and columns, each only while the
+// gap to it does not exceed the best distance so far: a point beyond a gap
+// lies at least that far away, so what is left out holds no nearer (nor, the
+// comparison being inclusive, an equally near) site.  True when every bin
+// not visited lies beyond the best distance.
+template <bool kDup>
+DNNI_HD bool search_window32(const BinGrid& g, const BinWindow& w, float inv_bs, int px, int py, Best& out) {
+    const int bs = g.bs;
+    const int ux = px - (g.gx0 + w.wx0 * bs), uy = py - (g.gy0 + w.wy0 * bs);   // 0 <= u < 2^15
+    const int lx = floor_div_est(ux, bs, inv_bs), ly = floor_div_est(uy, bs, inv_bs);
+    const int fx = ux - lx * bs, fy = uy - ly * bs;
+    const int x0 = lx > 0 ? lx - 1 : 0, x1 = lx + 2 < w.wnx ? lx + 2 : w.wnx;   // bins [x0, x1)
+    const int* row = w.lstart + ly * w.wnx;
+    Best32 b{~0ull, -1, 0};
+    scan_local32<kDup>(b, w.lpts, row[x0], row[x1], px, py);
+    // (of the rows above and below, the corner bins under the same rule)
+    const unsigned cl = (unsigned)((fx + 1) * (fx + 1)), cr = (unsigned)((bs - fx) * (bs - fx));
+    const unsigned cb = (unsigned)((fy + 1) * (fy + 1)), ct = (unsigned)((bs - fy) * (bs - fy));
+    if (ly > 0 && cb <= best32_d2(b))
+        scan_local32<kDup>(b, w.lpts, row[(cl + cb <= best32_d2(b) ? x0 : lx) - w.wnx],
+                           row[(cr + cb <= best32_d2(b) ? x1 : lx + 1) - w.wnx], px, py);
+    if (ly + 1 < w.wny && ct <= best32_d2(b))
+        scan_local32<kDup>(b, w.lpts, row[(cl + ct <= best32_d2(b) ? x0 : lx) + w.wnx],
+                           row[(cr + ct <= best32_d2(b) ? x1 : lx + 1) + w.wnx], px, py);
+    // the gaps to the second ring; a side at the grid's border is closed:
+    // nothing lies beyond it (65535^2 exceeds every distance here)
+    const int bx = w.wx0 + lx, by = w.wy0 + ly;
+    const unsigned gl = bx > 1 ? fx + bs + 1 : 65535, gr = bx < g.nbx - 2 ? 2 * bs - fx : 65535;
+    const unsigned gb = by > 1 ? fy + bs + 1 : 65535, gt = by < g.nby - 2 ? 2 * bs - fy : 65535;
+    const unsigned mx = gl < gr ? gl : gr, my = gb < gt ? gb : gt, m = mx < my ? mx : my;
+    bool done = best32_d2(b) < m * m;
+    if (!done) {
+        // second ring: inside the grid an open side's bins lie in the window
+        const int xa = lx > 1 ? lx - 2 : 0, xb = lx + 3 < w.wnx ? lx + 3 : w.wnx;
+        if (gb != 65535 && gb * gb <= best32_d2(b))
+            scan_local32<kDup>(b, w.lpts, row[xa - 2 * w.wnx], row[xb - 2 * w.wnx], px, py);
+        if (gt != 65535 && gt * gt <= best32_d2(b))
+            scan_local32<kDup>(b, w.lpts, row[xa + 2 * w.wnx], row[xb + 2 * w.wnx], px, py);
+        const int ya = ly > 0 ? -1 : 0, yb = ly + 1 < w.wny ? 1 : 0;
+        if (gl != 65535 && gl * gl <= best32_d2(b))
+            for (int r = ya; r <= yb; ++r)
+                scan_local32<kDup>(b, w.lpts, row[lx - 2 + r * w.wnx], row[lx - 1 + r * w.wnx], px, py);
+        if (gr != 65535 && gr * gr <= best32_d2(b))
+            for (int r = ya; r <= yb; ++r)
+                scan_local32<kDup>(b, w.lpts, row[lx + 2 + r * w.wnx], row[lx + 3 + r * w.wnx], px, py);
+        const unsigned hl = bx > 2 ? fx + 2 * bs + 1 : 65535, hr = bx < g.nbx - 3 ? 3 * bs - fx : 65535;
+        const unsigned hb = by > 2 ? fy + 2 * bs + 1 : 65535, ht = by < g.nby - 3 ? 3 * bs - fy : 65535;
+        const unsigned nx = hl < hr ? hl : hr, ny = hb < ht ? hb : ht, n = nx < ny ? nx : ny;
+        done = best32_d2(b) < n * n;
+    }
+    out.idx = b.idx;
+    out.nev += b.nev;
+    if (b.idx >= 0) {
+        out.d2 = (long long)best32_d2(b);
+        out.gid = (uint32_t)b.key;
+        out.z = w.lpts[b.idx].z;
+    }
+    return done;
 }
 
 DNNI_HD bool search_window_fast32(const BinGrid& g, const BinWindow& w, int px, int py, Best& out) {
-    const long long gx0 = g.gx0, gy0 = g.gy0, bs = g.bs;
-    int bx = udiv32((long long)px - gx0, bs);
-    int by = udiv32((long long)py - gy0, bs);
-    bx = bx < g.nbx - 1 ? bx : g.nbx - 1;
-    by = by < g.nby - 1 ? by : g.nby - 1;
-    const int lx = bx - w.wx0, ly = by - w.wy0;
-    Best32 b{~0ull, INT_MAX, -1, 0};
-    bool done;
-    {
-        const int x0 = lx - 1 > 0 ? lx - 1 : 0, x1 = lx + 1 < w.wnx - 1 ? lx + 1 : w.wnx - 1;
-        const int y0 = ly - 1 > 0 ? ly - 1 : 0, y1 = ly + 1 < w.wny - 1 ? ly + 1 : w.wny - 1;
-        for (int r = y0; r <= y1; ++r)
-            scan_local32(b, w.lpts, w.lstart[r * w.wnx + x0], w.lstart[r * w.wnx + x1 + 1], px, py);
-    }
-    done = ring_done32(best32_d2(b), px, py, g, bx - 1, bx + 1, by - 1, by + 1);
-    if (!done) {
-        const int x0 = lx - 2 > 0 ? lx - 2 : 0, x1 = lx + 2 < w.wnx - 1 ? lx + 2 : w.wnx - 1;
-        const long long X0 = gx0 + (long long)(w.wx0 + x0) * bs, X1 = gx0 + (long long)(w.wx0 + x1 + 1) * bs - 1;
-        for (int d = -2; d <= 2; d += 4) {
-            const int r = ly + d;
-            if (r < 0 || r >= w.wny) continue;
-            const long long Y0 = gy0 + (long long)(w.wy0 + r) * bs;
-            if (box_lb(px, py, X0, X1, Y0, Y0 + bs - 1) > best32_d2(b)) continue;
-            scan_local32(b, w.lpts, w.lstart[r * w.wnx + x0], w.lstart[r * w.wnx + x1 + 1], px, py);
-        }
-        const int ya = ly - 1 > 0 ? ly - 1 : 0, yb = ly + 1 < w.wny - 1 ? ly + 1 : w.wny - 1;
-        const long long Y0 = gy0 + (long long)(w.wy0 + ya) * bs, Y1 = gy0 + (long long)(w.wy0 + yb + 1) * bs - 1;
-        for (int d = -2; d <= 2; d += 4) {
-            const int c = lx + d;
-            if (c < 0 || c >= w.wnx) continue;
-            const long long CX0 = gx0 + (long long)(w.wx0 + c) * bs;
-            if (box_lb(px, py, CX0, CX0 + bs - 1, Y0, Y1) > best32_d2(b)) continue;
-            for (int r = ya; r <= yb; ++r)
-                scan_local32(b, w.lpts, w.lstart[r * w.wnx + c], w.lstart[r * w.wnx + c + 1], px, py);
-        }
-        done = ring_done32(best32_d2(b), px, py, g, bx - 2, bx + 2, by - 2, by + 2);
-    }
-    out.d2 = best32_d2(b);
-    out.gid = b.key == ~0ull ? 0xFFFFFFFFu : (uint32_t)(b.key & 0xFFFFFFFFull);
-    out.z = b.z;
-    out.idx = b.idx;
-    out.nev += b.nev;
-    return done;
+    return search_window32<true>(g, w, 1.0f / (float)g.bs, px, py, out);
 }
 
 // Sorted-array position of window-local point q (-1 stays -1).
@@ -781,7 +825,7 @@ DNNI_HD void decode_span_word(unsigned long long w, int K, long long zbase, long
 constexpr int kWinMaxBins = 1536;
 constexpr int kWinMaxRows = 256;
 constexpr int kWinMaxPts = 2560;
-constexpr size_t kDenseSmem = sizeof(int4) * kWinMaxPts + sizeof(int) * (2 * kWinMaxBins + 1);
+constexpr size_t kDenseSmem = sizeof(int4) * (kWinMaxPts + 1) + sizeof(int) * (2 * kWinMaxBins + 1);
 
 
 }  // namespace dnni

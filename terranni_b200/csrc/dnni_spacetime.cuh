@@ -430,7 +430,6 @@ static dnni_status spacetime_run(dnni_ctx* c, const dnni_workpackage* wp, const 
     if ((rs = ensure_scratch(c, c->scr, scratch_sizes(hb), a))) return rs;
     BatchTables bt = device_tables(a.tables, 1);
     if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
-    k_init_scalars<<<1, 32, 0, st>>>(bt, a.sc, a.ctr);
     int2* pix = (int2*)c->st.pix.p;
     const int64_t lifts = (int64_t)S * npix;
     // the worklist buffer serves the span work items of every slice (no far
@@ -440,6 +439,7 @@ static dnni_status spacetime_run(dnni_ctx* c, const dnni_workpackage* wp, const 
     const FarLayout far = far_layout(a.far, 0, (int64_t)S * nrt);
     static_assert((2 * kStMaxRadius + 1) * (4 + 8 * kSpanItemsPerTile) + 512 <= kTileX * kTileY * kFarSlotBytes,
                   "the slices' span work items fit the worklist buffer");
+    k_init_scalars<<<1, 256, 0, st>>>(bt, a.sc, a.ctr, nullptr);
     CK(cudaMemsetAsync(far.rtmax, 0xFF, sizeof(int) * (size_t)S * nrt, st));
     k_st_lift<<<(unsigned)((lifts + 255) / 256), 256, 0, st>>>(T, P, (const uint32_t*)c->st.site.p, dxyz, pix, a.sc,
                                                                far.rtmax, nrt);
