@@ -198,9 +198,12 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
     dense<<<nrt * split, 256, kDenseSmem, st>>>(bt, a.sorted, a.start, a.pix, d_site, far, a.sc, a.ctr, hb.far_blocks,
                                                 hb.dense_band, split);
     if (ev) cudaEventRecord(ev[4], st);
-    if (nchunk > 0)
-        k_near_far<<<sms * 6, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site,
+    if (nchunk > 0) {
+        k_near_far<<<sms * kFarCtasPerSm, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site,
                                             a.sc, a.ctr, hb.far_blocks);
+        k_near_far_heavy<<<sms * kFarCtasPerSm, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site,
+                                                  a.sc, a.ctr, hb.far_blocks);
+    }
     if (sites_only) return;
     k_decide<<<(int)hb.tiles.size(), 256, 0, st>>>(bt, a.sc, far, a.ctr, hb.win_words);
     if (ev) cudaEventRecord(ev[1], st);

@@ -64,7 +64,9 @@ struct BatchCounters {
     int far_next;                // next far group to hand out
     int nspan;                   // span work items listed
     int span_next;               // next span work item to hand out
-    int pad[3];
+    int nheavy;                  // far groups left to the heavy pass
+    int heavy_next;              // next of them to hand out
+    int pad;
 };
 
 template <typename B>
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(256) k_init_scalars(BatchTables bt, Scalars* s
         s->bbox[2] = INT_MAX; s->bbox[3] = INT_MIN;
         s->bbox[4] = INT_MAX; s->bbox[5] = INT_MIN;
         s->err = 0; s->packed = 0; s->kbits = 0; s->zbase = 0;
-        if (t == 0) { ctr->nfar = 0; ctr->err = 0; ctr->far_next = 0; ctr->nspan = 0; ctr->span_next = 0; }
+        if (t == 0) { ctr->nfar = 0; ctr->err = 0; ctr->far_next = 0; ctr->nspan = 0; ctr->span_next = 0; ctr->nheavy = 0; ctr->heavy_next = 0; }
     }
     if (l < kStatSlots) {
         s->max_r2[l] = -1; s->big_pixels[l] = 0; s->spans[l] = 0; s->nodata[l] = 0;
@@ -722,225 +724,401 @@ __global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int
     }
 }
 
-__device__ __forceinline__ long long warp_min64(long long v) {
+// ---------------------------------------------------------------------------
+// far pass: the exact nearest site of the pixels that the bin rings leave
+// ---------------------------------------------------------------------------
+
+// Number types of the search: 32-bit where every distance it can meet fits
+// (see far_fits32), 64-bit otherwise.
+template <bool k32> struct FarNum;
+template <> struct FarNum<true> {
+    using I = int;
+    using D = unsigned;
+    static __device__ __forceinline__ D warp_min(D v) { return __reduce_min_sync(0xffffffffu, v); }
+    static __device__ __forceinline__ D warp_max(D v) { return __reduce_max_sync(0xffffffffu, v); }
+    // at least floor(sqrt(v)) + 1: below 2^31 the estimate is within 0.05
+    static __device__ __forceinline__ I reach(D v) { return (I)sqrt_est((float)v) + 2; }
+};
+template <> struct FarNum<false> {
+    using I = long long;
+    using D = unsigned long long;
+    static __device__ __forceinline__ D warp_min(D v) {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) { const long long w = __shfl_xor_sync(0xffffffffu, v, o); v = w < v ? w : v; }
-    return v;
-}
-__device__ __forceinline__ long long warp_max64(long long v) {
+        for (int o = 16; o; o >>= 1) { const D w = __shfl_xor_sync(0xffffffffu, v, o); v = w < v ? w : v; }
+        return v;
+    }
+    static __device__ __forceinline__ D warp_max(D v) {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) { const long long w = __shfl_xor_sync(0xffffffffu, v, o); v = w > v ? w : v; }
-    return v;
-}
+        for (int o = 16; o; o >>= 1) { const D w = __shfl_xor_sync(0xffffffffu, v, o); v = w > v ? w : v; }
+        return v;
+    }
+    static __device__ __forceinline__ I reach(D v) { return reach_of((long long)v); }
+};
 
-__device__ __forceinline__ uint64_t warp_or64(uint64_t v) {
-    const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)v), hi = __reduce_or_sync(0xffffffffu, (unsigned)(v >> 32));
-    return ((uint64_t)hi << 32) | lo;
-}
-
-// 8 x 8 cell mask of the cells [a0,a1] x [b0,b1] (x = bit & 7, y = bit >> 3);
-// 0 when the range is empty.
-__device__ __forceinline__ uint64_t box_mask8(int a0, int a1, int b0, int b1) {
-    a0 = a0 < 0 ? 0 : a0;
-    b0 = b0 < 0 ? 0 : b0;
-    a1 = a1 > 7 ? 7 : a1;
-    b1 = b1 > 7 ? 7 : b1;
-    if (a0 > a1 || b0 > b1) return 0;
-    const uint64_t row = (uint64_t)((0xFFu << a0) & (0xFFu >> (7 - a1)) & 0xFFu);
-    uint64_t m = 0;
-    for (int y = b0; y <= b1; ++y) m |= row << (8 * y);
-    return m;
-}
-
-// Cells (u wide, 8 per side, origin o) that the box [c - r, c + r] may touch,
-// widened by one cell on each side so float rounding can only add cells.
-__device__ __forceinline__ void cell_span8(long long c, long long r, long long o, float inv_u, int& lo, int& hi) {
-    const float a = (float)(c - r - o) * inv_u, b = (float)(c + r - o) * inv_u;
-    lo = a < -2.0f ? -2 : (a > 9.0f ? 9 : (int)floorf(a)) - 1;
-    hi = b < -2.0f ? -2 : (b > 9.0f ? 9 : (int)floorf(b)) + 1;
-}
-
-// Squared box bound in 32-bit arithmetic, for gaps below 46341 (larger
-// gaps are clamped there, which still exceeds any bound below 2^31).
-__device__ __forceinline__ unsigned box_lb32(int rx, int ry, int x0, int x1, int y0, int y1) {
-    int dx = rx < x0 ? x0 - rx : (rx > x1 ? rx - x1 : 0);
-    int dy = ry < y0 ? y0 - ry : (ry > y1 ? ry - y1 : 0);
-    dx = dx < 46340 ? dx : 46340;
-    dy = dy < 46340 ? dy : 46340;
-    return (unsigned)(dx * dx) + (unsigned)(dy * dy);
-}
-
-// 8 x 8 mask of the cells (u wide, origin (X0, Y0)) that the union of the
-// active lanes' discs may touch, row by row: in cell row r the lanes' disc
-// chords, widened by one unit, are merged into their hull across the warp.
-// A superset of the cells within some lane's bound, so the search stays
-// exact; the lanes of a group are neighbouring pixels of one row, whose
-// chords overlap, so the hull adds little.  Warp-uniform result.
-__device__ __forceinline__ uint64_t chord_mask8(bool act, long long px, long long py, long long d2, long long X0,
-                                                long long Y0, long long u, bool small) {
-    uint64_t m = 0;
-#pragma unroll 1
-    for (int r = 0; r < 8; ++r) {
-        int a = 8, e = -1;
-        if (act) {
-            const long long gy = axis_gap(py, Y0 + r * u, Y0 + (r + 1) * u - 1);
-            if (gy * gy <= d2) {
-                const long long v = d2 - gy * gy;
-                const long long w = (small ? (long long)sqrtf((float)v) : (long long)sqrt((double)v)) + 1;
-                const long long lo = px - w - X0, hi = px + w - X0;
-                if (hi >= 0 && lo < 8 * u) {
-                    a = lo <= 0 ? 0 : udiv32(lo, u);
-                    e = hi >= 8 * u ? 7 : udiv32(hi, u);
-                }
+// One lane's pixel and best site so far.
+template <bool k32>
+struct FarLane {
+    using D = typename FarNum<k32>::D;
+    int px, py;
+    D d2;
+    uint32_t gid;
+    int z, idx;
+    __device__ __forceinline__ void consider(const int4 p, int q) {
+        D d;
+        if (k32) {
+            const int dx = p.x - px, dy = p.y - py;
+            d = (unsigned)(dx * dx) + (unsigned)(dy * dy);
+        } else {
+            const long long dx = (long long)p.x - px, dy = (long long)p.y - py;
+            d = (unsigned long long)(dx * dx) + (unsigned long long)(dy * dy);
+        }
+        if (__builtin_expect(d <= d2, 0)) {
+            const uint32_t g = (uint32_t)p.w;
+            if (d < d2 || g < gid || (g == gid && p.z < z)) {
+                d2 = d;
+                gid = g;
+                z = p.z;
+                idx = q;
             }
         }
-        a = __reduce_min_sync(0xffffffffu, a);
-        e = __reduce_max_sync(0xffffffffu, e);
-        if (a <= e) m |= (uint64_t)((0xFFu >> (7 - e)) & (0xFFu << a) & 0xFFu) << (8 * r);
     }
-    return m;
-}
+};
 
-// chord_mask8 for a warp whose every active lane has a bound below 2^31 (a
-// real site found), in 32-bit arithmetic relative to the mask's origin: rx,
-// ry = pixel - origin (|rx|, |ry| < 2^30), u = cell width (8u <= 2^30).  The
-// row gap beyond 46340 units already exceeds any such bound.  The chord's
-// cell range is the same as chord_mask8's: floor(x / u) for 0 < x < 8u from
-// a float product with 1/u (within one of the quotient there), corrected
-// with exact integer products.
-__device__ __forceinline__ int floor_div8(int x, int u, float inv_u) {
-    int q = (int)((float)x * inv_u);
-    q -= q * u > x ? 1 : 0;
-    q += (q + 1) * u <= x ? 1 : 0;
-    return q;
-}
-
-__device__ __forceinline__ uint64_t chord_mask8_32(bool act, int rx, int ry, unsigned d2, int u, float inv_u) {
-    uint64_t m = 0;
-#pragma unroll 1
-    for (int r = 0; r < 8; ++r) {
-        int a = 8, e = -1;
-        if (act) {
-            const int y0 = r * u, y1 = y0 + u - 1;
-            const int gy = ry < y0 ? y0 - ry : (ry > y1 ? ry - y1 : 0);
-            if (gy <= 46340 && (unsigned)(gy * gy) <= d2) {
-                const int w = (int)sqrt_est((float)(d2 - (unsigned)(gy * gy))) + 1;
-                const int lo = rx - w, hi = rx + w;
-                if (hi >= 0 && lo < 8 * u) {
-                    a = lo <= 0 ? 0 : floor_div8(lo, u, inv_u);
-                    e = hi >= 8 * u ? 7 : floor_div8(hi, u, inv_u);
-                }
-            }
-        }
-        a = __reduce_min_sync(0xffffffffu, a);
-        e = __reduce_max_sync(0xffffffffu, e);
-        if (a <= e) m |= (uint64_t)((0xFFu >> (7 - e)) & (0xFFu << a) & 0xFFu) << (8 * r);
-    }
-    return m;
+// Gap between the intervals [a0, a1] and [b0, b1] (0 when they meet).
+template <typename I>
+__device__ __forceinline__ I interval_gap(I a0, I a1, I b0, I b1) {
+    const I l = b0 - a1, r = a0 - b1, m = l > r ? l : r;
+    return m > 0 ? m : 0;
 }
 
 // A candidate block with at most this many points is scanned whole, which
-// costs less than its bin mask.
+// costs less than its bin rows.
 constexpr int kFarWholeBlock = 24;
+// A warp leaves a group to the heavy pass once it has searched this many
+// blocks for it and more remain: fewer while the groups leave warps without
+// work (below four to a warp), and none at all below one group per CTA of the
+// heavy pass, which then takes every group.
+constexpr int kFarDefer = 32, kFarDeferFew = 8;
+constexpr int kFarCtasPerSm = 4;
+__device__ __forceinline__ bool far_all_heavy(int groups) { return groups <= (int)gridDim.x; }
+constexpr int kFarPixels = 32;   // a group spans at most this many cells in x and y
 
-// Warp-cooperative exact search for the 32 pixels of one worklist group
-// (neighbouring pixels of one tile row; inactive lanes have act = false).
-// The warp walks the superblocks of the union of the lanes' bound boxes
-// (rows outward from the group's centre); inside a superblock the candidate
-// blocks are the non-empty ones under the chord hull of the lanes' discs
-// (chord_mask8), inside a candidate block the candidate bins likewise, and
-// every point of a candidate bin is considered by every active lane (the
-// comparison is exact, so extra candidates cost time, never correctness).
-// All control flow is uniform across the warp.  Complete for each active
-// lane whose b holds a real site on entry, by the same argument as
-// search_disc.
-__device__ void search_disc_warp(const BinGrid& g, const int4* __restrict__ pts, const int* __restrict__ start,
-                                 const uint64_t* __restrict__ bmask, const uint64_t* __restrict__ smask, bool act,
-                                 int px, int py, Best& b) {
+// A warp's buffer of candidate points: lanes fetch one point each, all in
+// flight at once, and every lane then evaluates all of them.
+struct FarBuf {
+    int4 p[32];
+    int q[32];
+    __device__ __forceinline__ void put(int k, const int4 v, int pos) {
+        p[k] = v;
+        q[k] = pos;
+    }
+    template <typename L>
+    __device__ __forceinline__ void consider_all(L& b, int n) const {
+        __syncwarp();
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) b.consider(p[k], q[k]);
+        __syncwarp();
+    }
+};
+
+// 32-bit arithmetic serves a search whose bound is `reach` (per lane, the
+// largest): a point it evaluates lies in a block some lane's disc touches, so
+// within reach + 8 bins + the group's extent of every lane, and that must stay
+// within 46340 for the squared distance to fit 32 bits.
+__device__ __forceinline__ bool far_fits32(long long reach, int bs, int cs) {
+    return reach + 8LL * bs + (long long)kFarPixels * cs <= 46340;
+}
+
+// Warp-cooperative exact search for the 32 pixels of one worklist group; every
+// lane holds a real site on entry (idle lanes repeat another lane's pixel).
+// The group's superblocks within the largest bound are walked from the
+// group's own; a superblock's blocks, two to a lane, are tested against the
+// group's box at once and searched nearest first, so that the bounds tighten
+// early; in a block, the bins within the largest bound form one run per row
+// (tested the same way), and a run some lane's disc touches is one range of
+// points, evaluated by every lane.  Every test is a lower bound of the
+// distance against an upper bound of what is sought, so nothing that could
+// hold an equally near site is left out.  Uniform control flow in the warp.
+//
+// kCta: the eight warps of a CTA search one group; warp w takes the blocks of
+// one residue class, and the lanes' bounds meet in s_bound.  Otherwise the
+// search ends with false after `most` blocks if more remain.
+template <bool k32, bool kCta>
+__device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restrict__ pts, const int* __restrict__ start,
+                                           const uint64_t* __restrict__ bmask, const uint64_t* __restrict__ smask,
+                                           FarLane<k32>& b, unsigned& nev, FarBuf* buf,
+                                           volatile unsigned long long* s_bound, int most) {
+    using N = FarNum<k32>;
+    using I = typename N::I;
+    using D = typename N::D;
     const unsigned full = 0xffffffffu;
-    const long long gx0 = g.gx0, gy0 = g.gy0, bs = g.bs;
-    const long long u1 = bs * kBinsPerBlockEdge, u2 = bs * kBinsPerSuperEdge;
-    const float inv_u1 = 1.0f / (float)u1, inv_bs = 1.0f / (float)bs;
-    const long long reach = act ? reach_of(b.d2) : 0;
-    const long long xlo = warp_min64(act ? px - reach : LLONG_MAX), xhi = warp_max64(act ? px + reach : LLONG_MIN);
-    const long long ylo = warp_min64(act ? py - reach : LLONG_MAX), yhi = warp_max64(act ? py + reach : LLONG_MIN);
-    if (xlo > xhi) return;   // no active lane
-    int sx0, sx1, sy0, sy1;
-    cell_range((xlo + xhi) / 2, (xhi - xlo) / 2 + 1, gx0, u2, g.n2x, sx0, sx1);
-    cell_range((ylo + yhi) / 2, (yhi - ylo) / 2 + 1, gy0, u2, g.n2y, sy0, sy1);
-    if (sx0 > sx1 || sy0 > sy1) return;
-    const long long cyy = warp_min64(act ? py : LLONG_MAX);
-    int csy = udiv32((cyy < gy0 ? gy0 : cyy) - gy0, u2);
-    csy = csy < sy0 ? sy0 : (csy > sy1 ? sy1 : csy);
-    const int span = (csy - sy0) > (sy1 - csy) ? (csy - sy0) : (sy1 - csy);
-    for (int r = 0; r <= 2 * span; ++r) {
-        const int sy = csy + ((r & 1) ? -((r + 1) >> 1) : (r >> 1));
-        if (sy < sy0 || sy > sy1) continue;
-        const long long SY0 = gy0 + (long long)sy * u2;
-        for (int sx = sx0; sx <= sx1; ++sx) {
-            const int sidx = sy * g.n2x + sx;
-            const uint64_t sm = __ldg(&smask[sidx]);
-            if (!sm) continue;
-            const long long SX0 = gx0 + (long long)sx * u2;
-            const bool need_s = act && box_lb(px, py, SX0, SX0 + u2 - 1, SY0, SY0 + u2 - 1) <= b.d2;
-            if (!__any_sync(full, need_s)) continue;
-            // 32-bit arithmetic while every bound is below 2^31 and every
-            // active lane lies within 2^29 units of the superblock's origin
-            // (then within 2^30 of each of its blocks' origins)
-            const long long ox = px - SX0, oy = py - SY0;
-            const bool near = !act || (ox > -(1LL << 29) && ox < (1LL << 29) && oy > -(1LL << 29) && oy < (1LL << 29));
-            bool small = __all_sync(full, !act || (b.d2 < (1LL << 31) && near));
-            uint64_t cand = sm & (small ? chord_mask8_32(act, (int)(px - SX0), (int)(py - SY0), (unsigned)b.d2,
-                                                         (int)u1, inv_u1)
-                                        : chord_mask8(act, px, py, b.d2, SX0, SY0, u1, false));
-            while (cand) {
-                const int m = ffs64(cand);
-                cand &= cand - 1;
-                const long long BX0 = SX0 + (long long)(m & 7) * u1, BY0 = SY0 + (long long)(m >> 3) * u1;
-                const int64_t blk = ((int64_t)sidx << 6) + m;
-                const int bp0 = __ldg(&start[blk << 6]), bp1 = __ldg(&start[(blk + 1) << 6]);
-                if (bp1 - bp0 <= kFarWholeBlock) {
-                    // few points: the block's range whole (its bins are consecutive)
-                    if (act) b.nev += bp1 - bp0;
-                    for (int q = bp0; q < bp1; ++q) {
-                        const int4 p = __ldg(&pts[q]);
-                        if (act) consider(b, p, q, px, py);
-                    }
-                    continue;
-                }
-                const uint64_t bm = __ldg(&bmask[blk]);
-                small = __all_sync(full, !act || (b.d2 < (1LL << 31) && near));
-                uint64_t qc = bm & (small ? chord_mask8_32(act, (int)(px - BX0), (int)(py - BY0), (unsigned)b.d2,
-                                                           (int)bs, inv_bs)
-                                          : chord_mask8(act, px, py, b.d2, BX0, BY0, bs, false));
-                while (qc) {
-                    const int l = ffs64(qc);
-                    qc &= qc - 1;
-                    const int64_t id = (blk << 6) + l;
-                    const int s0 = __ldg(&start[id]), e0 = __ldg(&start[id + 1]);
-                    if (act) b.nev += e0 - s0;
-                    if (small) {
-                        for (int q = s0; q < e0; ++q) {
-                            const int4 p = __ldg(&pts[q]);
-                            if (act) consider_below31(b, p, q, px, py);
-                        }
-                    } else {
-                        for (int q = s0; q < e0; ++q) {
-                            const int4 p = __ldg(&pts[q]);
-                            if (act) consider(b, p, q, px, py);
-                        }
-                    }
-                }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const I gx0 = g.gx0, gy0 = g.gy0, bs = g.bs, u1 = bs * kBinsPerBlockEdge, u2 = bs * kBinsPerSuperEdge;
+    const I X0 = __reduce_min_sync(full, b.px), X1 = __reduce_max_sync(full, b.px);
+    const I Y0 = __reduce_min_sync(full, b.py), Y1 = __reduce_max_sync(full, b.py);
+    // lane's bound: nothing farther can matter to it
+    auto bound = [&]() -> D {
+        if (!kCta) return b.d2;
+        const unsigned long long s = s_bound[lane];
+        return s < (unsigned long long)b.d2 ? (D)s : b.d2;
+    };
+    D maxd = N::warp_max(bound());
+    const I reach = N::reach(maxd);
+    auto cell = [&](I v, I o, int n) {   // superblock column (row) of v, clamped to the grid
+        const long long c = (long long)v - o;
+        return c <= 0 ? 0 : (c >= (long long)n * u2 ? n - 1 : udiv32(c, u2));
+    };
+    const int sx0 = cell(X0 - reach, gx0, g.n2x), sx1 = cell(X1 + reach, gx0, g.n2x);
+    const int sy0 = cell(Y0 - reach, gy0, g.n2y), sy1 = cell(Y1 + reach, gy0, g.n2y);
+    const int cx = cell(X0, gx0, g.n2x), cy = cell(Y0, gy0, g.n2y);
+    const int nsx = sx1 - sx0 + 1, ns = nsx * (sy1 - sy0 + 1);
+    int searched = 0;
+    for (int k = -1, sx = cx, sy = cy; k < ns; ++k) {
+        // the group's own superblock first, then the others row by row
+        if (k >= 0) {
+            sx = k == 0 ? sx0 : (sx == sx1 ? sx0 : sx + 1);
+            sy = k == 0 ? sy0 : (sx == sx0 ? sy + 1 : sy);
+            if (sx == cx && sy == cy) continue;
+        }
+        const int sidx = sy * g.n2x + sx;
+        const uint64_t sm = __ldg(&smask[sidx]);
+        if (!sm) continue;
+        const I SX0 = gx0 + (I)sx * u2, SY0 = gy0 + (I)sy * u2;
+        {
+            const I dx = interval_gap(X0, X1, SX0, SX0 + u2 - 1), dy = interval_gap(Y0, Y1, SY0, SY0 + u2 - 1);
+            if (dx > N::reach(maxd) || dy > N::reach(maxd) || (D)(dx * dx) + (D)(dy * dy) > maxd) continue;
+        }
+        // this lane's two blocks: column lane & 7, rows lane >> 3 and + 4
+        D key0, key1;
+        const D none = ~(D)0;
+        {
+            const I bx = SX0 + (I)(lane & 7) * u1, by = SY0 + (I)(lane >> 3) * u1;
+            I dx = interval_gap(X0, X1, bx, bx + u1 - 1);
+            I dy = interval_gap(Y0, Y1, by, by + u1 - 1), ey = interval_gap(Y0, Y1, by + 4 * u1, by + 5 * u1 - 1);
+            if (k32) {       // 46340^2 exceeds every bound here
+                dx = dx < 46340 ? dx : 46340;
+                dy = dy < 46340 ? dy : 46340;
+                ey = ey < 46340 ? ey : 46340;
+            }
+            key0 = (sm >> lane) & 1 ? (D)(dx * dx) + (D)(dy * dy) : none;
+            key1 = (sm >> (lane + 32)) & 1 ? (D)(dx * dx) + (D)(ey * ey) : none;
+            if (kCta) {
+                // residue classes of the blocks: neighbouring blocks go to different warps
+                const int c = (lane & 7) + 3 * (lane >> 3) + sx + sy;
+                if ((c & 7) != warp) key0 = none;
+                if (((c + 12) & 7) != warp) key1 = none;
             }
         }
+        // their occupancy and point ranges, all in flight at once
+        uint64_t mask0 = 0, mask1 = 0;
+        int first0 = 0, last0 = 0, first1 = 0, last1 = 0;
+        {
+            const int64_t k0 = ((int64_t)sidx << 6) + lane;
+            if (key0 <= maxd) {
+                mask0 = __ldg(&bmask[k0]);
+                first0 = __ldg(&start[k0 << 6]);
+                last0 = __ldg(&start[(k0 + 1) << 6]);
+            }
+            if (key1 <= maxd) {
+                mask1 = __ldg(&bmask[k0 + 32]);
+                first1 = __ldg(&start[(k0 + 32) << 6]);
+                last1 = __ldg(&start[(k0 + 33) << 6]);
+            }
+        }
+        for (;;) {
+            const D key = key0 < key1 ? key0 : key1, least = N::warp_min(key);
+            if (least > maxd || least == none) break;
+            const int who = __ffs(__ballot_sync(full, key == least)) - 1;
+            const int second = __shfl_sync(full, (int)(key0 != least), who);
+            if (lane == who) {
+                if (second) key1 = none; else key0 = none;
+            }
+            const int m = who + 32 * second;
+            const I BX0 = SX0 + (I)(m & 7) * u1, BY0 = SY0 + (I)(m >> 3) * u1;
+            // a disc must touch it (its gap to every lane is at most the bound, and fits)
+            const D bd = bound();
+            {
+                I dx = interval_gap((I)b.px, (I)b.px, BX0, BX0 + u1 - 1), dy = interval_gap((I)b.py, (I)b.py, BY0, BY0 + u1 - 1);
+                if (k32) { dx = dx < 46340 ? dx : 46340; dy = dy < 46340 ? dy : 46340; }
+                if (!__any_sync(full, (D)(dx * dx) + (D)(dy * dy) <= bd)) continue;
+            }
+            if (!kCta && ++searched > most) return false;
+            const int* st = start + (((int64_t)sidx << 6) + m << 6);
+            const int bp0 = __shfl_sync(full, second ? first1 : first0, who);
+            const int bp1 = __shfl_sync(full, second ? last1 : last0, who);
+            if (bp1 - bp0 <= kFarWholeBlock) {
+                // few points: the block's range whole (its bins are consecutive)
+                if (lane < bp1 - bp0) buf->put(lane, __ldg(&pts[bp0 + lane]), bp0 + lane);
+                buf->consider_all(b, bp1 - bp0);
+                nev += bp1 - bp0;
+            } else {
+                const int t0 = __ldg(&st[lane]), t1 = __ldg(&st[lane + 32]);
+                const unsigned bm0 = __shfl_sync(full, second ? (unsigned)mask1 : (unsigned)mask0, who);
+                const unsigned bm1 = __shfl_sync(full, second ? (unsigned)(mask1 >> 32) : (unsigned)(mask0 >> 32), who);
+                uint64_t run;
+                {
+                    const I qx = BX0 + (I)(lane & 7) * bs, qy = BY0 + (I)(lane >> 3) * bs;
+                    I dx = interval_gap(X0, X1, qx, qx + bs - 1);
+                    I dy = interval_gap(Y0, Y1, qy, qy + bs - 1), ey = interval_gap(Y0, Y1, qy + 4 * bs, qy + 5 * bs - 1);
+                    if (k32) {
+                        dx = dx < 46340 ? dx : 46340;
+                        dy = dy < 46340 ? dy : 46340;
+                        ey = ey < 46340 ? ey : 46340;
+                    }
+                    const unsigned lo = __ballot_sync(full, (D)(dx * dx) + (D)(dy * dy) <= maxd);
+                    const unsigned hi = __ballot_sync(full, (D)(dx * dx) + (D)(ey * ey) <= maxd);
+                    run = (uint64_t)(bm0 & lo) | ((uint64_t)(bm1 & hi) << 32);
+                }
+                // the rows' runs, first to last bin, that some disc touches;
+                // lanes 4r .. 4r + 3 take row r's run of points
+                int ia = 0, ie = 0;
+                while (run) {
+                    const int r = ffs64(run) >> 3;
+                    const unsigned bits = (unsigned)(run >> (8 * r)) & 0xFFu;
+                    run &= ~(0xFFull << (8 * r));
+                    const int a = __ffs(bits) - 1, e = 31 - __clz(bits);
+                    const I qx = BX0 + (I)a * bs, qy = BY0 + (I)r * bs;
+                    I dx = interval_gap((I)b.px, (I)b.px, qx, qx + (I)(e - a + 1) * bs - 1);
+                    I dy = interval_gap((I)b.py, (I)b.py, qy, qy + bs - 1);
+                    if (k32) { dx = dx < 46340 ? dx : 46340; dy = dy < 46340 ? dy : 46340; }
+                    if (__any_sync(full, (D)(dx * dx) + (D)(dy * dy) <= bd) && (lane >> 2) == r) {
+                        ia = 8 * r + a;
+                        ie = 8 * r + e + 1;
+                    }
+                }
+                const int sa0 = __shfl_sync(full, t0, ia & 31), sa1 = __shfl_sync(full, t1, ia & 31);
+                const int se0 = __shfl_sync(full, t0, ie & 31), se1 = __shfl_sync(full, t1, ie & 31);
+                const int e0 = ie == 64 ? bp1 : (ie < 32 ? se0 : se1);
+                for (int q = (ia < 32 ? sa0 : sa1) + (lane & 3); ; q += 4) {
+                    const bool in = q < e0 && ie != 0;
+                    const unsigned got = __ballot_sync(full, in);
+                    if (!got) break;
+                    if (in) buf->put(__popc(got & ((1u << lane) - 1u)), __ldg(&pts[q]), q);
+                    buf->consider_all(b, __popc(got));
+                    nev += __popc(got);
+                }
+            }
+            if (kCta && (unsigned long long)b.d2 < s_bound[lane])
+                atomicMin((unsigned long long*)&s_bound[lane], (unsigned long long)b.d2);
+            maxd = N::warp_max(bound());
+        }
+    }
+    return true;
+}
+
+// A group of the far worklist in one warp's registers: its pixels (idle
+// lanes repeat the first active lane's) and the best sites so far.
+struct FarWork {
+    int t, rt, i, j;
+    bool act;
+    Best b;
+    int px, py;
+    unsigned nev;
+};
+
+// Loads group k and seeds every lane with a real site: its own best so far,
+// the best of the lane that is nearest to one, and points of the non-empty
+// bin closest to the group in the non-empty block nearest to it.
+__device__ __forceinline__ void far_load(FarWork& w, const BatchTables& bt, const FarLayout& far, int k, int far_blocks,
+                                         const int4* __restrict__ pts_all, const int* __restrict__ start_all,
+                                         const uint64_t* __restrict__ bmask_all, const int64_t* __restrict__ near_all) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int4 head = *reinterpret_cast<const int4*>(&far.groups[k]);
+    const int own = far.groups[k].idx[lane];
+    w.t = head.x;
+    w.rt = head.y;
+    const TileParams& T = bt.tiles[w.t];
+    const BinGrid g = T.bg;
+    const int4* pts = pts_all + T.srt_off;
+    const int* start = start_all + T.bin_off;
+    w.act = own != kFarIdle;
+    int di, dj;
+    far_lane(far_blocks, lane, di, dj);
+    w.i = head.z + di;
+    w.j = head.w + dj;
+    const int first = __ffs(__ballot_sync(full, w.act)) - 1;
+    w.px = (T.rx0 + w.i) * T.cs;
+    w.py = (T.ry0 + w.j) * T.cs;
+    const int fx = __shfl_sync(full, w.px, first), fy = __shfl_sync(full, w.py, first);
+    if (!w.act) {
+        w.px = fx;
+        w.py = fy;
+    }
+    w.b = Best{LLONG_MAX, 0xFFFFFFFFu, INT_MAX, -1, 0};
+    w.nev = 0;
+    if (own >= 0) {
+        consider(w.b, __ldg(&pts[own]), own, w.px, w.py);
+        w.nev += 1;
+    }
+    if (__any_sync(full, own >= 0)) {
+        // float order is enough to choose a seed
+        const unsigned f = own >= 0 ? __float_as_uint((float)w.b.d2) : 0xffffffffu;
+        const int src = __ffs(__ballot_sync(full, f == __reduce_min_sync(full, f))) - 1;
+        const int q = __shfl_sync(full, own, src);
+        consider(w.b, __ldg(&pts[q]), q, w.px, w.py);
+        w.nev += 1;
+    }
+    const int gx = min(udiv32((long long)fx - g.gx0, g.bs), g.nbx - 1), gy = min(udiv32((long long)fy - g.gy0, g.bs), g.nby - 1);
+    const int64_t nb = __ldg(&near_all[T.blk_off + (int64_t)(gy >> 3) * (g.nbx >> 3) + (gx >> 3)]);
+    if (nb >= 0) {
+        const int sidx = (int)(nb >> 6), m = (int)(nb & 63);
+        const uint64_t bm = __ldg(&bmask_all[T.blk_off + nb]);
+        // bins relative to the first pixel, in bins: the nearest non-empty one
+        const int ox = (sidx % g.n2x) * 64 + (m & 7) * 8 + (lane & 7) - gx;
+        const int oy = (sidx / g.n2x) * 64 + (m >> 3) * 8 + (lane >> 3) - gy;
+        const float a = (float)ox * (float)ox, c = (float)oy * (float)oy, e = (float)(oy + 4) * (float)(oy + 4);
+        const unsigned k0 = (bm >> lane) & 1 ? __float_as_uint(a + c) : 0xffffffffu;
+        const unsigned k1 = (bm >> (lane + 32)) & 1 ? __float_as_uint(a + e) : 0xffffffffu;
+        const unsigned least = __reduce_min_sync(full, min(k0, k1));
+        const int who = __ffs(__ballot_sync(full, min(k0, k1) == least)) - 1;
+        const int second = __shfl_sync(full, (int)(k0 != least), who);
+        const int64_t id = (nb << 6) + who + 32 * second;
+        const int s0 = __ldg(&start[id]), e0 = min(__ldg(&start[id + 1]), s0 + 4);
+        w.nev += e0 - s0;
+        for (int q = s0; q < e0; ++q) consider(w.b, __ldg(&pts[q]), q, w.px, w.py);
     }
 }
 
-// Far pass over the worklist: one warp per group of 32 slots (handed out by a counter;
-// all slots of a group belong to one tile).  Each lane seeds its bound (its
-// best site so far, else the nearest non-empty block's closest bin, else the
-// nearest non-empty superblock) and the warp searches the union of the bound
-// discs cooperatively.
+template <bool k32, bool kCta>
+__device__ __forceinline__ bool far_run(FarWork& w, const TileParams& T, const int4* pts_all, const int* start_all,
+                                        const uint64_t* bmask_all, const uint64_t* smask_all, FarBuf* buf,
+                                        volatile unsigned long long* s_bound, int most) {
+    FarLane<k32> b{w.px, w.py, (typename FarNum<k32>::D)w.b.d2, w.b.gid, w.b.z, w.b.idx};
+    const bool done = far_search<k32, kCta>(T.bg, pts_all + T.srt_off, start_all + T.bin_off, bmask_all + T.blk_off,
+                                            smask_all + T.sup_off, b, w.nev, buf, s_bound, most);
+    w.b.d2 = (long long)b.d2;
+    w.b.gid = b.gid;
+    w.b.z = b.z;
+    w.b.idx = b.idx;
+    return done;
+}
+
+__device__ __forceinline__ bool far_small(const FarWork& w, const TileParams& T) {
+    const long long r = w.b.d2 < (1LL << 31) ? (long long)sqrt_est((float)w.b.d2) + 2 : LLONG_MAX / 4;
+    return __all_sync(0xffffffffu, far_fits32(r, T.bg.bs, T.cs));
+}
+
+__device__ __forceinline__ void far_settle(const FarWork& w, const TileParams& T, int2* __restrict__ pix,
+                                           uint32_t* __restrict__ site, Scalars* __restrict__ sc, const FarLayout& far,
+                                           int slot) {
+    int R2 = -1;
+    if (w.act) {
+        R2 = r2_of(w.b.d2, (long long)T.cs * T.cs, T.r2cap);
+        settle_pixel(T, w.i, w.j, w.b, R2, pix, site);
+    }
+    StatAcc acc;
+    acc.add(T, R2, w.act ? (int)w.nev : 0);
+    acc.flush(sc + w.t, slot, true);
+    const int m = __reduce_max_sync(0xffffffffu, R2);
+    if ((threadIdx.x & 31) == 0 && m > T.rs * T.rs) atomicMax(&far.rtmax[w.rt], m);
+}
+
+// Far pass over the worklist: one warp per group, handed out by a counter
+// (groups differ in cost by orders of magnitude: a lake's centre against its
+// shore).  Groups that need more than kFarDefer blocks go, with the sites
+// found so far, to the heavy list (in the span items' place, which are listed
+// later; at most 64 groups per raster tile).
 __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4* __restrict__ pts_all,
                                                      const int* __restrict__ start_all,
                                                      const uint64_t* __restrict__ bmask_all,
@@ -949,69 +1127,73 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
                                                      FarLayout far, int2* __restrict__ pix,
                                                      uint32_t* __restrict__ site, Scalars* __restrict__ sc,
                                                      BatchCounters* __restrict__ ctr, int far_blocks) {
+    __shared__ FarBuf s_buf[8];
     const int count = ctr->nfar;
+    if (far_all_heavy(count)) return;
     const int lane = threadIdx.x & 31;
-    // groups differ in cost by orders of magnitude (a lake's centre against
-    // its shore), so each warp takes the next group from a counter instead of
-    // a fixed stride
+    FarBuf* buf = &s_buf[threadIdx.x >> 5];
+    const int most = count < (int)gridDim.x * 32 ? kFarDeferFew : kFarDefer;
+    int* heavy = (int*)far.items;
     for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&ctr->far_next, 1);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= count) break;
-        const int4 head = *reinterpret_cast<const int4*>(&far.groups[base]);
-        const int own = far.groups[base].idx[lane];
-        const int t = head.x;
-        const TileParams& T = bt.tiles[t];
-        const BinGrid g = T.bg;
-        const int4* pts = pts_all + T.srt_off;
-        const int* start = start_all + T.bin_off;
-        const uint64_t* bmask = bmask_all + T.blk_off;
-        const uint64_t* smask = smask_all + T.sup_off;
-        const bool act = own != kFarIdle;
-        int i = 0, j = 0, px = 0, py = 0;
-        Best b{LLONG_MAX, 0xFFFFFFFFu, INT_MAX, -1, 0};
-        if (act) {
-            int di, dj;
-            far_lane(far_blocks, lane, di, dj);
-            i = head.z + di;
-            j = head.w + dj;
-            px = (T.rx0 + i) * T.cs;
-            py = (T.ry0 + j) * T.cs;
-            if (own >= 0) {
-                consider(b, __ldg(&pts[own]), own, px, py);
-                b.nev += 1;
+        int k = 0;
+        if (lane == 0) k = atomicAdd(&ctr->far_next, 1);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= count) break;
+        FarWork w;
+        far_load(w, bt, far, k, far_blocks, pts_all, start_all, bmask_all, near_all);
+        const TileParams& T = bt.tiles[w.t];
+        const bool done = far_small(w, T)
+                              ? far_run<true, false>(w, T, pts_all, start_all, bmask_all, smask_all, buf, nullptr, most)
+                              : far_run<false, false>(w, T, pts_all, start_all, bmask_all, smask_all, buf, nullptr, most);
+        if (done) {
+            far_settle(w, T, pix, site, sc, far, blockIdx.x * 3 + (threadIdx.x >> 5));
+        } else {
+            if (w.act) far.groups[k].idx[lane] = w.b.idx;
+            if (lane == 0) heavy[atomicAdd(&ctr->nheavy, 1)] = k;
+        }
+    }
+}
+
+// The heavy groups, one CTA of eight warps each.
+__global__ void __launch_bounds__(256, 4) k_near_far_heavy(BatchTables bt, const int4* __restrict__ pts_all,
+                                                           const int* __restrict__ start_all,
+                                                           const uint64_t* __restrict__ bmask_all,
+                                                           const uint64_t* __restrict__ smask_all,
+                                                           const int64_t* __restrict__ near_all, FarLayout far,
+                                                           int2* __restrict__ pix, uint32_t* __restrict__ site,
+                                                           Scalars* __restrict__ sc, BatchCounters* __restrict__ ctr,
+                                                           int far_blocks) {
+    __shared__ unsigned long long s_bound[32];
+    __shared__ Best s_best[8][32];
+    __shared__ FarBuf s_buf[8];
+    __shared__ int s_k;
+    const bool all = far_all_heavy(ctr->nfar);
+    const int count = all ? ctr->nfar : ctr->nheavy;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int* heavy = (const int*)far.items;
+    for (;;) {
+        __syncthreads();                 // the previous group's readers are done
+        if (threadIdx.x == 0) s_k = atomicAdd(&ctr->heavy_next, 1);
+        __syncthreads();
+        if (s_k >= count) break;
+        FarWork w;
+        far_load(w, bt, far, all ? s_k : heavy[s_k], far_blocks, pts_all, start_all, bmask_all, near_all);
+        if (warp == 0) s_bound[lane] = (unsigned long long)w.b.d2;
+        __syncthreads();
+        const TileParams& T = bt.tiles[w.t];
+        if (far_small(w, T)) far_run<true, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], s_bound, 0);
+        else far_run<false, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], s_bound, 0);
+        w.b.nev = (int)w.nev;
+        s_best[warp][lane] = w.b;
+        __syncthreads();
+        if (warp == 0) {
+            for (int v = 1; v < 8; ++v) {
+                const Best o = s_best[v][lane];
+                w.nev += (unsigned)o.nev;
+                if (o.d2 < w.b.d2 || (o.d2 == w.b.d2 && (o.gid < w.b.gid || (o.gid == w.b.gid && o.z < w.b.z)))) w.b = o;
             }
-            int bx = udiv32((long long)px - g.gx0, g.bs), by = udiv32((long long)py - g.gy0, g.bs);
-            bx = bx < g.nbx - 1 ? bx : g.nbx - 1;
-            by = by < g.nby - 1 ? by : g.nby - 1;
-            const int64_t nb = __ldg(&near_all[T.blk_off + (int64_t)(by >> 3) * (g.nbx >> 3) + (bx >> 3)]);
-            if (nb >= 0) seed_from_block(g, pts, start, bmask, nb, px, py, b);
-            if (b.d2 == LLONG_MAX) seed_from_superblocks(g, pts, start, bmask, smask, px, py, b);
+            far_settle(w, T, pix, site, sc, far, blockIdx.x);
         }
-        // the seeds of the group's corner lanes are candidates for every
-        // pixel of the group: a lane whose own seed came from a distant
-        // block starts the disc search with a tighter bound
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int src = (k & 1 ? 7 : 0) + (k & 2 ? 24 : 0);
-            const int q = __shfl_sync(0xffffffffu, b.idx, src);
-            if (act && q >= 0) {
-                consider(b, __ldg(&pts[q]), q, px, py);
-                b.nev += 1;
-            }
-        }
-        search_disc_warp(g, pts, start, bmask, smask, act, px, py, b);
-        int R2 = -1;
-        if (act) {
-            R2 = r2_of(b.d2, (long long)T.cs * T.cs, T.r2cap);
-            settle_pixel(T, i, j, b, R2, pix, site);
-        }
-        StatAcc acc;
-        acc.add(T, R2, b.nev);
-        acc.flush(sc + t, blockIdx.x * 3 + (threadIdx.x >> 5), true);
-        const int m = __reduce_max_sync(0xffffffffu, R2);
-        if (lane == 0 && m > T.rs * T.rs) atomicMax(&far.rtmax[head.y], m);
     }
 }
 
