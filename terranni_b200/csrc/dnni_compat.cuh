@@ -290,11 +290,11 @@ static dnni_status compat_run(dnni_ctx* c, const dnni_compat_settings* s, const 
     const long long per = (span / kCpTile + 2) * (span / kCpTile + 2);
     const int64_t list_n = std::max<int64_t>(n * per, 1);
     dnni_status rs;
-    // scratch: the pixel keys in the context's span-word buffer, the tile
+    // scratch: the pixel keys in the context's late buffer, the tile
     // counts, offsets and cursors in its bin-count buffer, the per-tile point
     // lists in its rank buffer; points and outputs in its staging buffers
     const size_t tbytes = sizeof(long long) * (size_t)(nt + 1) + 2 * sizeof(int) * (size_t)nt;
-    if ((rs = dnni_ensure(c, c->scr.D, sizeof(unsigned long long) * (size_t)(xp * yp))) ||
+    if ((rs = dnni_ensure(c, c->scr.late, sizeof(unsigned long long) * (size_t)(xp * yp))) ||
         (rs = dnni_ensure(c, c->scr.cnt, tbytes)) ||
         (rs = dnni_ensure(c, c->scr.list, sizeof(uint32_t) * (size_t)list_n)) ||
         (!device && ((rs = dnni_ensure(c, c->in_xyz, sizeof(double) * 3 * (size_t)std::max<int64_t>(n, 1))) ||
@@ -304,7 +304,7 @@ static dnni_status compat_run(dnni_ctx* c, const dnni_compat_settings* s, const 
     const double* dxyz = device ? xyz : (const double*)c->in_xyz.p;
     float* dh = device ? h_out : (float*)c->out_h.p;
     int32_t* dres = res_out ? (device ? res_out : (int32_t*)c->out_site.p) : nullptr;
-    unsigned long long* key = (unsigned long long*)c->scr.D.p;
+    unsigned long long* key = (unsigned long long*)c->scr.late.p;
     long long* toff = (long long*)c->scr.cnt.p;
     int* tcnt = (int*)(toff + nt + 1);
     int* tcur = tcnt + nt;

@@ -53,15 +53,21 @@ struct DeviceGuard {
     }
 };
 
+size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
+
 // Every scratch array a batch needs, in bytes.
 struct ScratchSizes {
     size_t sorted, cnt, bsum, bmask, smask, rownear, near, pix, far, D, Dc, sc, ctr, tables;
+    size_t part;                     // the points grouped by region
+    size_t late() const { return al256(pix) + al256(far) + al256(D) + al256(Dc); }
+    size_t late_part() const { return std::max(late(), al256(part)); }
 };
 
 ScratchSizes scratch_sizes(const HostBatch& hb) {
     const int n = (int)hb.tiles.size();
     ScratchSizes z;
     z.sorted = sizeof(int4) * std::max<int64_t>(hb.n_pts, 1);
+    z.part = z.sorted;
     z.cnt = sizeof(int) * std::max<int64_t>(hb.n_bins, 1);
     z.bsum = sizeof(int) * std::max<int64_t>(hb.scan_base.back(), 1);
     z.bmask = sizeof(uint64_t) * std::max<int64_t>(hb.blk_base.back(), 1);
@@ -78,15 +84,36 @@ ScratchSizes scratch_sizes(const HostBatch& hb) {
     return z;
 }
 
+// Lays out the arrays of the phases after the binning in `bytes` at base, and
+// over them, where they are large enough for it, the points grouped by region.
+void carve_late(void* base, size_t bytes, const ScratchSizes& z, DevArrays& a) {
+    unsigned char* p = (unsigned char*)base;
+    a.part = bytes >= z.part ? (int4*)p : nullptr;
+    a.pix = (int2*)p;
+    p += al256(z.pix);
+    a.far = (int4*)p;
+    p += al256(z.far);
+    a.D = (unsigned long long*)p;
+    p += al256(z.D);
+    a.Dc = (int*)p;
+}
+
+// The late arrays with room for the grouped points, or, where that would pass
+// the context's budget or the device's memory, without.
+dnni_status ensure_late(dnni_ctx* c, DevBuf& b, size_t with_part, size_t plain) {
+    if (dnni_ensure(c, b, with_part) == DNNI_OK) return DNNI_OK;
+    c->err.clear();
+    return dnni_ensure(c, b, plain);
+}
+
 dnni_status ensure_scratch(dnni_ctx* c, Scratch& s, const ScratchSizes& z, DevArrays& a) {
     dnni_status rs;
     if ((rs = dnni_ensure(c, s.sorted, z.sorted)) || (rs = dnni_ensure(c, s.cnt, z.cnt)) || (rs = dnni_ensure(c, s.start, z.cnt)) ||
         (rs = dnni_ensure(c, s.bsum, z.bsum)) || (rs = dnni_ensure(c, s.bmask, z.bmask)) ||
         (rs = dnni_ensure(c, s.smask, z.smask)) || (rs = dnni_ensure(c, s.rownear, z.rownear)) ||
-        (rs = dnni_ensure(c, s.near, z.near)) || (rs = dnni_ensure(c, s.pix, z.pix)) ||
-        (rs = dnni_ensure(c, s.far, z.far)) || (rs = dnni_ensure(c, s.D, z.D)) || (rs = dnni_ensure(c, s.Dc, z.Dc)) ||
+        (rs = dnni_ensure(c, s.near, z.near)) ||
         (rs = dnni_ensure(c, s.sc, z.sc)) || (rs = dnni_ensure(c, s.ctr, z.ctr)) ||
-        (rs = dnni_ensure(c, s.tables, z.tables)))
+        (rs = dnni_ensure(c, s.tables, z.tables)) || (rs = ensure_late(c, s.late, z.late_part(), z.late())))
         return rs;
     a.sorted = (int4*)s.sorted.p;
     a.cnt = (int*)s.cnt.p;
@@ -96,10 +123,7 @@ dnni_status ensure_scratch(dnni_ctx* c, Scratch& s, const ScratchSizes& z, DevAr
     a.smask = (uint64_t*)s.smask.p;
     a.rownear = (int*)s.rownear.p;
     a.near = (int64_t*)s.near.p;
-    a.pix = (int2*)s.pix.p;
-    a.far = (int4*)s.far.p;
-    a.D = (unsigned long long*)s.D.p;
-    a.Dc = (int*)s.Dc.p;
+    carve_late(s.late.p, s.late.cap, z, a);
     a.sc = (Scalars*)s.sc.p;
     a.ctr = (BatchCounters*)s.ctr.p;
     a.tables = (unsigned char*)s.tables.p;
@@ -108,7 +132,7 @@ dnni_status ensure_scratch(dnni_ctx* c, Scratch& s, const ScratchSizes& z, DevAr
 
 void release_scratch(dnni_ctx* c, Scratch& s) {
     DevBuf* bufs[] = {&s.sorted, &s.list, &s.cnt, &s.start, &s.bsum, &s.bmask, &s.smask, &s.rownear,
-                      &s.near, &s.pix, &s.far, &s.D, &s.Dc, &s.sc, &s.ctr, &s.tables};
+                      &s.near, &s.late, &s.sc, &s.ctr, &s.tables};
     for (DevBuf* b : bufs) dnni_release(*b, c);
 }
 
@@ -135,6 +159,10 @@ void set_dense_smem_attr() {
     if (dev >= 0 && dev < 64 && !done[dev]) {
         cudaFuncSetAttribute(k_near_dense<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem);
         cudaFuncSetAttribute(k_near_dense<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem);
+        cudaFuncSetAttribute(k_region_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(int) * (kMaxBins / kBinsPerSuper)));
+        cudaFuncSetAttribute(k_region_part, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(int) * (kMaxBins / kBinsPerSuper)));
         cudaFuncSetAttribute(k_scatter_window, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(sizeof(unsigned long long) * kSpanWindowMaxWords));
         done[dev] = true;
@@ -158,9 +186,10 @@ void launch_spans(const HostBatch& hb, const BatchTables& bt, const DevArrays& a
 void launch_prologue(const HostBatch& hb, const BatchTables& bt, const DevArrays& a, const int32_t* d_xyz,
                      cudaStream_t st, bool bbox = true) {
     const int n = (int)hb.tiles.size();
-    k_init_scalars<<<n, 256, 0, st>>>(bt, a.sc, a.ctr, far_layout(a.far, hb.n_far, hb.rt_base.back()).rtmax);
+    k_init_scalars<<<n, 256, 0, st>>>(bt, a.sc, a.ctr, far_layout(a.far, hb.n_far, hb.rt_base.back()).rtmax,
+                                      bbox ? nullptr : a.cnt);
     const int nchunk = hb.chunk_base.back();
-    if (bbox && nchunk > 0) k_bbox<<<nchunk, 256, 0, st>>>(bt, d_xyz, a.sc, a.ctr);
+    if (bbox && nchunk > 0) k_bbox<<<nchunk, kChunkThreads, 0, st>>>(bt, d_xyz, a.sc, a.ctr);
 }
 
 // Launch sequence, part 2: binning, nearest sites, spans, stencil, finalize.
@@ -173,23 +202,43 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
                  const cudaEvent_t* ev, bool bbox_in_count = false, bool sites_only = false) {
     const int nchunk = hb.chunk_base.back();
     const int64_t nblk = hb.blk_base.back(), nsup = hb.sup_base.back();
-    if (nchunk > 0) {
-        cudaMemsetAsync(a.cnt, 0, sizeof(int) * hb.n_bins, st);
-        k_bin_count<<<nchunk, 256, 0, st>>>(bt, d_xyz, a.cnt, a.sc, a.ctr, bbox_in_count ? 1 : 0);
-        const int nscan = hb.scan_base.back();
-        k_scan_partial<<<nscan, kScanThreads, 0, st>>>(bt, a.cnt, a.bsum);
-        k_scan_bsum<<<(int)hb.tiles.size(), 1024, 0, st>>>(bt, a.bsum);
-        k_scan_final<<<nscan, kScanThreads, 0, st>>>(bt, a.cnt, a.bsum, a.start);
-        k_bin_scatter<<<nchunk, 256, 0, st>>>(bt, d_xyz, d_gid, a.start, a.cnt, a.sorted);
-        if (nblk > 0) k_block_masks<<<(int)((nblk * 32 + 255) / 256), 256, 0, st>>>(bt, a.start, a.bmask);
-        if (nsup > 0) k_super_masks<<<(int)((nsup * 32 + 255) / 256), 256, 0, st>>>(bt, a.bmask, a.smask);
-        const int nrow1 = hb.row1_base.back();
-        if (nrow1 > 0) k_block_rows<<<(nrow1 + 127) / 128, 128, 0, st>>>(bt, a.bmask, a.rownear);
-        if (nblk > 0) k_block_near<<<(int)((nblk + 255) / 256), 256, 0, st>>>(bt, a.rownear, a.near);
-    }
-    if (ev) cudaEventRecord(ev[0], st);
     const int nrt = hb.rt_base.back();
     const FarLayout far = far_layout(a.far, hb.n_far, nrt);
+    if (nchunk > 0) {
+        if (a.part) {
+            const size_t hist = sizeof(int) * hb.max_reg;
+            // a single work package's region counts start at zero here (its
+            // bins were not planned when k_init_scalars ran)
+            const bool partition = hb.max_reg > 1;
+            if (partition && !bbox_in_count) cudaMemsetAsync(a.cnt, 0, sizeof(int) * hb.max_reg, st);
+            if (partition || bbox_in_count)
+                k_region_count<<<nchunk, kChunkThreads, hist, st>>>(bt, d_xyz, a.cnt, a.sc, a.ctr, bbox_in_count ? 1 : 0);
+            if (partition) {
+                k_region_scan<<<(int)hb.tiles.size(), 1024, 0, st>>>(bt, a.cnt);
+                k_region_part<<<nchunk, kChunkThreads, hist, st>>>(bt, d_xyz, d_gid, a.cnt, a.part);
+            }
+            if (hb.strip_base.back() > 0)
+                k_region_sort<9><<<hb.strip_base.back(), 256, 0, st>>>(bt, d_xyz, d_gid, a.cnt, a.part, a.start, a.sorted,
+                                                                       a.bmask, a.smask);
+            if (hb.whole_base.back() > 0)
+                k_region_sort<12><<<hb.whole_base.back(), 1024, 0, st>>>(bt, d_xyz, d_gid, a.cnt, a.part, a.start,
+                                                                         a.sorted, a.bmask, a.smask);
+        } else {
+            cudaMemsetAsync(a.cnt, 0, sizeof(int) * hb.n_bins, st);
+            k_bin_count<<<nchunk, kChunkThreads, 0, st>>>(bt, d_xyz, a.cnt, a.sc, a.ctr, bbox_in_count ? 1 : 0);
+            const int nscan = hb.scan_base.back();
+            k_scan_partial<<<nscan, kScanThreads, 0, st>>>(bt, a.cnt, a.bsum);
+            k_scan_bsum<<<(int)hb.tiles.size(), 1024, 0, st>>>(bt, a.bsum);
+            k_scan_final<<<nscan, kScanThreads, 0, st>>>(bt, a.cnt, a.bsum, a.start);
+            k_bin_scatter<<<nchunk, kChunkThreads, 0, st>>>(bt, d_xyz, d_gid, a.start, a.cnt, a.sorted);
+            if (nblk > 0) k_block_masks<<<(int)((nblk * 32 + 255) / 256), 256, 0, st>>>(bt, a.start, a.bmask);
+            if (nsup > 0) k_super_masks<<<(int)((nsup * 32 + 255) / 256), 256, 0, st>>>(bt, a.bmask, a.smask);
+        }
+        const int nrow1 = hb.row1_base.back();
+        if (nrow1 > 0) k_block_rows<<<(nrow1 + 3) / 4, 128, 0, st>>>(bt, a.bmask, a.rownear);
+        if (nblk > 0) k_block_near<<<(int)((nblk + 255) / 256), 256, 0, st>>>(bt, a.rownear, a.near, far.rtmax);
+    }
+    if (ev) cudaEventRecord(ev[0], st);
     // a raster tile goes to several CTAs while the tiles alone leave the SMs
     // (four CTAs each) without two rounds of work
     int split = 1;
@@ -315,10 +364,11 @@ static dnni_status run_device(dnni_ctx* c, const dnni_workpackage* wp, const int
     plan_bins(bb, 0, c->s.bin_target, t);
     HostBatch hb;
     hb.rs = c->s.small_radius;
+    set_chunk(hb, n);
     batch_add(hb, t, 0, 0, d_site ? 0 : -1);
     DevArrays a;
     if ((rs = ensure_scratch(c, c->scr, scratch_sizes(hb), a))) return rs;
-    BatchTables bt = device_tables(a.tables, 1);
+    BatchTables bt = device_tables(a.tables, hb);
     if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
     if (timing) CK(cudaEventRecord(c->ev[0], st));
     launch_prologue(hb, bt, a, d_xyz, st);
@@ -331,9 +381,10 @@ static dnni_status run_device(dnni_ctx* c, const dnni_workpackage* wp, const int
         plan_bins(c->h_sc->bbox, n, c->s.bin_target, t);
         hb = HostBatch();
         hb.rs = c->s.small_radius;
+        set_chunk(hb, n);
         batch_add(hb, t, 0, 0, d_site ? 0 : -1);
         if ((rs = ensure_scratch(c, c->scr, scratch_sizes(hb), a))) return rs;
-        bt = device_tables(a.tables, 1);
+        bt = device_tables(a.tables, hb);
         if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
     }
     launch_body(hb, bt, a, d_xyz, d_gid, d_h, d_site, c->sm_count, st, timing ? &c->ev[1] : nullptr);
@@ -424,6 +475,9 @@ static dnni_status plan_batch(dnni_ctx* c, const dnni_tile* tiles, int32_t ntile
     hb.win_words = ww_;
     hb.far_blocks = fb_;
     hb.dense_band = db_;
+    int64_t points = 0;
+    for (const TileParams& t : plan) points += t.npts;
+    set_chunk(hb, points);
     for (int k : order) batch_add(hb, plan[k], tiles[k].pt_offset, tiles[k].out_offset, tiles[k].site_offset);
     if (hb.too_big) return set_err(c, DNNI_E_INVAL, "batch too large for one launch sequence: split it");
     return DNNI_OK;
@@ -637,7 +691,7 @@ dnni_status dnni_batch_create(dnni_ctx* c, const dnni_tile* tiles, int32_t ntile
     }
     dnni_status rs = ensure_scratch(c, b->scr, scratch_sizes(b->hb), b->arr);
     if (!rs) {
-        b->bt = device_tables(b->arr.tables, ntiles);
+        b->bt = device_tables(b->arr.tables, b->hb);
         rs = stage_tables(c, b->hb, b->arr.tables, c->stream);
         if (!rs && cudaStreamSynchronize(c->stream) != cudaSuccess) rs = cuda_err(c, cudaGetLastError(), "upload");
     }
@@ -787,29 +841,38 @@ static dnni_status plan_slices(dnni_batch* b) {
             }
         if (sl.site0 == INT64_MAX) sl.site0 = sl.site1 = 0;
         if ((rs = dnni_ensure(c, sl.tables, TableLayout((int)part.size()).total))) return rs;
-        sl.bt = device_tables((const unsigned char*)sl.tables.p, (int)part.size());
+        sl.bt = device_tables((const unsigned char*)sl.tables.p, sl.hb);
         if ((rs = stage_tables(c, sl.hb, (unsigned char*)sl.tables.p, c->stream))) return rs;
         b->slices.push_back(std::move(sl));
         k0 = k1;
     }
+    // each slice works in its own part of the batch's scratch, so that
+    // consecutive slices can compute on two streams at once
+    const int ns = (int)b->slices.size();
+    dnni_status rs;
+    if ((rs = dnni_ensure(c, b->slice_ctrs, sizeof(BatchCounters) * (size_t)ns))) return rs;
+    ScratchSizes full_z = scratch_sizes(b->hb);
+    size_t with_part = 0, plain = 0;
+    for (const BatchSlice& sl : b->slices) {
+        const ScratchSizes z = scratch_sizes(sl.hb);
+        with_part += z.late_part();
+        plain += z.late();
+    }
+    if ((rs = ensure_late(c, b->scr.late, std::max(with_part, full_z.late_part()), std::max(plain, full_z.late())))) return rs;
     // the full batch's view of its scratch (the graph captured for it is
     // rebuilt if the arrays moved)
     DevArrays full;
-    dnni_status rs = ensure_scratch(c, b->scr, scratch_sizes(b->hb), full);
-    if (rs) return rs;
+    if ((rs = ensure_scratch(c, b->scr, full_z, full))) return rs;
     full.tables = b->arr.tables;
     if (full.sorted != b->arr.sorted || full.pix != b->arr.pix) {
         if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
         if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
     }
     b->arr = full;
-    const int ns = (int)b->slices.size();
-    // each slice works in its own part of the batch's scratch (the parts add
-    // up to the whole batch's sizes), so that consecutive slices can compute
-    // on two streams at once
-    if ((rs = dnni_ensure(c, b->slice_ctrs, sizeof(BatchCounters) * (size_t)ns))) return rs;
     {
-        int64_t pts = 0, bins = 0, scan = 0, blk = 0, sup = 0, pix = 0, far = 0, cells = 0, tiles = 0;
+        const bool parts = b->scr.late.cap >= with_part;
+        unsigned char* late = (unsigned char*)b->scr.late.p;
+        int64_t pts = 0, bins = 0, scan = 0, blk = 0, sup = 0, tiles = 0;
         for (int s = 0; s < ns; ++s) {
             BatchSlice& sl = b->slices[s];
             const HostBatch& h = sl.hb;
@@ -822,10 +885,10 @@ static dnni_status plan_slices(dnni_batch* b) {
             v.smask += sup;
             v.rownear += blk;
             v.near += blk;
-            v.pix += pix;
-            v.far += far;
-            v.D += cells;
-            v.Dc += cells;
+            const ScratchSizes z = scratch_sizes(h);
+            const size_t bytes = parts ? z.late_part() : z.late();
+            carve_late(late, bytes, z, v);
+            late += bytes;
             v.sc += tiles;
             v.ctr = (BatchCounters*)b->slice_ctrs.p + s;
             v.tables = (unsigned char*)sl.tables.p;
@@ -835,9 +898,6 @@ static dnni_status plan_slices(dnni_batch* b) {
             scan += h.scan_base.back();
             blk += h.blk_base.back();
             sup += h.sup_base.back();
-            pix += h.n_pix;
-            far += h.n_far;
-            cells += h.n_cells;
             tiles += (int64_t)h.tiles.size();
         }
     }
@@ -1022,7 +1082,7 @@ dnni_status dnni_batch_autotune(dnni_ctx* c, const dnni_tile* tiles, int32_t nti
         dnni_status rs = plan_batch(c, smp.data(), m, o, hb, order);
         if (rs) return rs;
         if ((rs = ensure_scratch(c, tscr, scratch_sizes(hb), a))) return rs;
-        const BatchTables bt = device_tables(a.tables, m);
+        const BatchTables bt = device_tables(a.tables, hb);
         if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
         for (int r = 0; r < 3; ++r) {            // one warm-up run, two timed
             if (r == 1) CK(cudaEventRecord(c->ev[0], st));
@@ -1173,9 +1233,9 @@ dnni_status noalloc_base(int dev, unsigned char** out) {
     return DNNI_OK;
 }
 
-// Carves one work package's scratch out of the array; false when it does
-// not fit.
-bool carve_noalloc(unsigned char* base, const ScratchSizes& z, DevArrays& a) {
+// Carves one work package's scratch out of the array, with room for the
+// points grouped by region if with_part; false when it does not fit.
+bool carve_noalloc(unsigned char* base, const ScratchSizes& z, bool with_part, DevArrays& a) {
     size_t off = 0;
     auto take = [&](size_t bytes) {
         unsigned char* p = base + off;
@@ -1185,10 +1245,8 @@ bool carve_noalloc(unsigned char* base, const ScratchSizes& z, DevArrays& a) {
     a.tables = take(z.tables);
     a.sc = (Scalars*)take(z.sc);
     a.ctr = (BatchCounters*)take(z.ctr);
-    a.pix = (int2*)take(z.pix);
-    a.far = (int4*)take(z.far);
-    a.D = (unsigned long long*)take(z.D);
-    a.Dc = (int*)take(z.Dc);
+    const size_t late = with_part ? z.late_part() : z.late();
+    carve_late(take(late), late, z, a);
     a.sorted = (int4*)take(z.sorted);
     a.cnt = (int*)take(z.cnt);
     a.start = (int*)take(z.cnt);
@@ -1229,7 +1287,8 @@ extern "C" dnni_status dnni_interpolate_segment_device_noalloc(const dnni_workpa
     HostBatch hb;
     batch_add(hb, t, 0, 0, d_site ? 0 : -1);
     DevArrays a;
-    if (!carve_noalloc(base, scratch_sizes(hb), a)) return DNNI_E_SCRATCH;
+    if (!carve_noalloc(base, scratch_sizes(hb), true, a) && !carve_noalloc(base, scratch_sizes(hb), false, a))
+            return DNNI_E_SCRATCH;
     // the one-tile tables go up from pageable host memory: the copy has
     // taken the bytes when cudaMemcpyAsync returns, so the buffer can be
     // repacked at once
@@ -1237,7 +1296,7 @@ extern "C" dnni_status dnni_interpolate_segment_device_noalloc(const dnni_workpa
     pack_tables(hb, tbl.data());
     if (cudaMemcpyAsync(a.tables, tbl.data(), tbl.size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
         return DNNI_E_CUDA;
-    BatchTables bt = device_tables(a.tables, 1);
+    BatchTables bt = device_tables(a.tables, hb);
     // the array keeps the previous call's contents: the scalars, bin counts
     // and span words are cleared by the launch sequence itself
     launch_prologue(hb, bt, a, d_xyz, st);
@@ -1252,11 +1311,12 @@ extern "C" dnni_status dnni_interpolate_segment_device_noalloc(const dnni_workpa
         plan_bins(hsc.bbox, n, 0.0, t);
         hb = HostBatch();
         batch_add(hb, t, 0, 0, d_site ? 0 : -1);
-        if (!carve_noalloc(base, scratch_sizes(hb), a)) return DNNI_E_SCRATCH;
+        if (!carve_noalloc(base, scratch_sizes(hb), true, a) && !carve_noalloc(base, scratch_sizes(hb), false, a))
+            return DNNI_E_SCRATCH;
         pack_tables(hb, tbl.data());
         if (cudaMemcpyAsync(a.tables, tbl.data(), tbl.size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
             return DNNI_E_CUDA;
-        bt = device_tables(a.tables, 1);
+        bt = device_tables(a.tables, hb);
     }
     launch_body(hb, bt, a, d_xyz, d_gid, d_h, d_site, sms, st, nullptr);
     if (cudaGetLastError() != cudaSuccess) return DNNI_E_CUDA;

@@ -20,14 +20,18 @@ struct DevBuf {
 };
 
 // Device scratch of one batch (or of the context's single work packages);
-// `list` serves only the reference-default mode (its per-tile point lists).
+// `list` serves only the reference-default mode (its per-tile point lists);
+// `late` holds what the phases after the binning use (pixel records,
+// worklist, span words and counts: carve_late), and before that the points
+// grouped by region.
 struct Scratch {
-    DevBuf sorted, list, cnt, start, bsum, bmask, smask, rownear, near, pix, far, D, Dc, sc, ctr, tables;
+    DevBuf sorted, list, cnt, start, bsum, bmask, smask, rownear, near, late, sc, ctr, tables;
 };
 
 // Raw device pointers of a scratch set for one launch sequence.
 struct DevArrays {
     int4* sorted = nullptr;
+    int4* part = nullptr;            // points grouped by region, over pix .. Dc; null: no room, bin directly
     int* cnt = nullptr;
     int* start = nullptr;
     int* bsum = nullptr;

@@ -15,6 +15,7 @@ namespace dnni {
 
 constexpr int64_t kMaxBins = 1LL << 26;
 constexpr int kMaxSide = 32767;
+constexpr int64_t kRegionDirect = 8192;   // points one CTA bins without a partition pass
 
 // Validates the work package (nni::WorkPackage, nni.h:66-70, in LAS units)
 // and fills the geometry part of t.  On failure returns the status and sets
@@ -101,6 +102,11 @@ inline void plan_bins(const int32_t bbox[6], int64_t n, double bin_target, TileP
     t.bg.n2x = (int32_t)(nbx / kBinsPerSuperEdge);
     t.bg.n2y = (int32_t)(nby / kBinsPerSuperEdge);
     t.bg.nbins = nbx * nby;
+    // binning regions: one for a small tile (a single CTA bins it straight from
+    // the input), strips of 512 bins up to 2048 of them (a chunk of 4096 points
+    // then still finds several to a strip), superblocks beyond
+    const int64_t nsup = t.bg.nbins / kBinsPerSuper;
+    t.rsh = nsup > 256 || (nsup == 1 && n <= kRegionDirect) ? 12 : 9;
     // the ring search's bands: halved while the window of an average place
     // (evenly spread points) would pass the shared-memory arrays' sizes; a
     // denser place halves its band further in the kernel
@@ -130,6 +136,9 @@ struct HostBatch {
     std::vector<TileParams> tiles;
     std::vector<int> chunk_base{0}, scan_base{0}, row1_base{0}, rt_base{0}, ct_base{0}, grow_base{0}, band_base{0};
     std::vector<int64_t> blk_base{0}, sup_base{0};
+    std::vector<int> strip_base{0}, whole_base{0};   // binning regions of 512 bins, of 4096 bins
+    int max_reg = 1;                     // most regions of a tile
+    int chunk = kChunkSmall;             // points per block in the point passes (set_chunk)
     int64_t n_rows = 0;                  // input point rows the tiles reference
     int64_t n_pts = 0, n_bins = 0, n_pix = 0, n_cells = 0, n_far = 0;
     int64_t out_end = 0, site_end = 0;   // extent of the caller's output arrays used
@@ -146,6 +155,12 @@ struct HostBatch {
 inline int64_t far_slots(const TileParams& t) {
     return (int64_t)((t.rw + kTileX - 1) / kTileX * kTileX) * ((t.rh + kTileY - 1) / kTileY * kTileY);
 }
+
+// Before the first tile is added: the points per block of the point passes,
+// from all points of the batch.  Large chunks reserve more points per global
+// atomic of the partition; small ones keep the SMs busy when points are few
+// (1 M points: 245 large chunks are less than two to an SM).
+inline void set_chunk(HostBatch& hb, int64_t points) { hb.chunk = points >= (2 << 20) ? kChunkLarge : kChunkSmall; }
 
 // Appends a tile whose geometry and bin grid are set; its point range starts
 // at pt_off of the batch's point arrays and its heights at out_off of the
@@ -170,7 +185,10 @@ inline void batch_add(HostBatch& hb, TileParams t, int64_t pt_off, int64_t out_o
         if (x > kMaxLaunchIndex) hb.too_big = true;
         v.push_back((int)std::min<int64_t>(x, kMaxLaunchIndex));
     };
-    add(hb.chunk_base, (t.npts + kChunk - 1) / kChunk);
+    add(hb.chunk_base, (t.npts + hb.chunk - 1) / hb.chunk);
+    add(hb.strip_base, t.rsh == 9 ? nbins >> 9 : 0);
+    add(hb.whole_base, t.rsh == 12 ? nbins >> 12 : 0);
+    hb.max_reg = std::max<int>(hb.max_reg, (int)(nbins >> t.rsh));
     add(hb.scan_base, (nbins + 1 + kScanTile - 1) / kScanTile);
     add(hb.row1_base, t.npts > 0 ? (t.bg.nby >> 3) : 0);
     add(hb.rt_base, (int64_t)((t.rw + kTileX - 1) / kTileX) * ((t.rh + kTileY - 1) / kTileY));
@@ -243,7 +261,7 @@ inline std::vector<double> edt_2d(const unsigned char* occ, int nx, int ny) {
 
 // Byte layout of the device copy of a batch's tables (one upload).
 struct TableLayout {
-    size_t tiles, chunk, scan, blk, sup, row1, rt, ct, grow, band, total;
+    size_t tiles, chunk, scan, blk, sup, row1, rt, ct, grow, band, strip, whole, total;
     explicit TableLayout(int n) {
         size_t o = 0;
         auto take = [&](size_t b) { const size_t r = o; o = (o + b + 15) & ~(size_t)15; return r; };
@@ -257,6 +275,8 @@ struct TableLayout {
         ct = take(sizeof(int) * (n + 1));
         grow = take(sizeof(int) * (n + 1));
         band = take(sizeof(int) * (n + 1));
+        strip = take(sizeof(int) * (n + 1));
+        whole = take(sizeof(int) * (n + 1));
         total = o;
     }
 };
@@ -275,12 +295,16 @@ inline void pack_tables(const HostBatch& hb, unsigned char* dst) {
     memcpy(dst + L.ct, hb.ct_base.data(), sizeof(int) * (n + 1));
     memcpy(dst + L.grow, hb.grow_base.data(), sizeof(int) * (n + 1));
     memcpy(dst + L.band, hb.band_base.data(), sizeof(int) * (n + 1));
+    memcpy(dst + L.strip, hb.strip_base.data(), sizeof(int) * (n + 1));
+    memcpy(dst + L.whole, hb.whole_base.data(), sizeof(int) * (n + 1));
 }
 
 // Device view of tables uploaded to `dev` (laid out as TableLayout).
-inline BatchTables device_tables(const unsigned char* dev, int n) {
+inline BatchTables device_tables(const unsigned char* dev, const HostBatch& hb) {
+    const int n = (int)hb.tiles.size();
     const TableLayout L(n);
     BatchTables bt;
+    bt.chunk = hb.chunk;
     bt.tiles = (const TileParams*)(dev + L.tiles);
     bt.ntiles = n;
     bt.chunk_base = (const int*)(dev + L.chunk);
@@ -292,6 +316,8 @@ inline BatchTables device_tables(const unsigned char* dev, int n) {
     bt.ct_base = (const int*)(dev + L.ct);
     bt.grow_base = (const int*)(dev + L.grow);
     bt.band_base = (const int*)(dev + L.band);
+    bt.strip_base = (const int*)(dev + L.strip);
+    bt.whole_base = (const int*)(dev + L.whole);
     return bt;
 }
 

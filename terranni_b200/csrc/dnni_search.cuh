@@ -71,7 +71,7 @@ struct TileParams {
     int32_t r2cap;               // no pixel/cell pair is farther apart (cell units^2)
     int32_t rs;                  // small-disc radius of the stencil path
     int32_t band;                // ring search: most pixel rows whose window is expected to fit
-    int32_t pad;
+    int32_t rsh;                 // binning: a region is 2^rsh bins (one superblock or an eighth of one)
     int32_t has_gid;
     int64_t npts;
     double z_scale, z_offset;
@@ -442,6 +442,15 @@ DNNI_HD int floor_div_est(int x, int u, float inv_u) {
     q -= q * u > x ? 1 : 0;
     q += (q + 1) * u <= x ? 1 : 0;
     return q;
+}
+
+// The same for 0 <= x < 2^32 and a quotient below 2^20 (its float estimate is
+// then within one), (q + 1) u < 2^32.
+DNNI_HD int floor_div_u32(unsigned x, unsigned u, float inv_u) {
+    unsigned q = (unsigned)((float)x * inv_u);
+    q -= q * u > x ? 1u : 0u;
+    q += (q + 1) * u <= x ? 1u : 0u;
+    return (int)q;
 }
 
 // Bin rings 0..kRingsBins around the pixel on a window that fits 32 bits;

@@ -609,7 +609,7 @@ dnni_status segment_run(dnni_ctx* c, const dnni_segment& s, const int32_t* h_xyz
         }
         if ((rs = plan_batch(c, tl.data(), ng, bo, hb, order))) return rs;
         if ((rs = ensure_scratch(c, scr, scratch_sizes(hb), a))) return rs;
-        const BatchTables bt = device_tables(a.tables, ng);
+        const BatchTables bt = device_tables(a.tables, hb);
         if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
         launch_prologue(hb, bt, a, (const int32_t*)B.gxyz.p, st, false);
         launch_body(hb, bt, a, (const int32_t*)B.gxyz.p, (const uint32_t*)B.ggid.p, gout, gsite, c->sm_count, st,

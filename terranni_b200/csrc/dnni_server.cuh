@@ -211,8 +211,6 @@ bool srv_plan(dnni_server* s, uint64_t ticket, const SrvReq& q, std::vector<SegC
     return true;
 }
 
-size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
-
 // Device bytes a batch needs in a slot arena: staging plus scratch.
 size_t srv_footprint(const HostBatch& hb, int64_t pts, int64_t out, int64_t site, size_t nchunks) {
     const ScratchSizes z = scratch_sizes(hb);
@@ -257,10 +255,8 @@ dnni_status srv_launch(dnni_server* s, SrvSlot& sl, std::vector<SrvItem>& items,
     a.tables = take(z.tables);
     a.sc = (Scalars*)take(z.sc);
     a.ctr = (BatchCounters*)take(z.ctr);
-    a.pix = (int2*)take(z.pix);
-    a.far = (int4*)take(z.far);
-    a.D = (unsigned long long*)take(z.D);
-    a.Dc = (int*)take(z.Dc);
+    // (no room beyond the admitted footprint: denser batches bin directly)
+    carve_late(take(z.late()), z.late(), z, a);
     a.sorted = (int4*)take(z.sorted);
     a.cnt = (int*)take(z.cnt);
     a.start = (int*)take(z.cnt);
@@ -305,7 +301,7 @@ dnni_status srv_launch(dnni_server* s, SrvSlot& sl, std::vector<SrvItem>& items,
                                                          gxyz, ggid);
     }
     if (nt) {
-        const BatchTables bt = device_tables(a.tables, nt);
+        const BatchTables bt = device_tables(a.tables, hb);
         launch_prologue(hb, bt, a, gxyz, st, false);
         launch_body(hb, bt, a, gxyz, ggid, gout, site ? gsite : nullptr, c->sm_count, st, nullptr, true);
         CK(cudaMemcpyAsync(sl.h_sc, a.sc, sizeof(Scalars) * nt, cudaMemcpyDeviceToHost, st));

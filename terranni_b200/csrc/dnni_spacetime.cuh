@@ -410,7 +410,7 @@ static dnni_status spacetime_run(dnni_ctx* c, const dnni_workpackage* wp, const 
         if ((rs = plan_batch(c, tiles.data(), V, bo, vb, order))) return rs;
         DevArrays va;
         if ((rs = ensure_scratch(c, c->st.scr, scratch_sizes(vb), va))) return rs;
-        const BatchTables vbt = device_tables(va.tables, V);
+        const BatchTables vbt = device_tables(va.tables, vb);
         if ((rs = stage_tables(c, vb, va.tables, st))) return rs;
         const int32_t* dx = m > 0 ? (const int32_t*)c->st.xyz.p : nullptr;
         launch_prologue(vb, vbt, va, dx, st, false);
@@ -428,7 +428,7 @@ static dnni_status spacetime_run(dnni_ctx* c, const dnni_workpackage* wp, const 
     batch_add(hb, T, 0, 0, -1);
     DevArrays a;
     if ((rs = ensure_scratch(c, c->scr, scratch_sizes(hb), a))) return rs;
-    BatchTables bt = device_tables(a.tables, 1);
+    BatchTables bt = device_tables(a.tables, hb);
     if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
     int2* pix = (int2*)c->st.pix.p;
     const int64_t lifts = (int64_t)S * npix;
@@ -439,7 +439,7 @@ static dnni_status spacetime_run(dnni_ctx* c, const dnni_workpackage* wp, const 
     const FarLayout far = far_layout(a.far, 0, (int64_t)S * nrt);
     static_assert((2 * kStMaxRadius + 1) * (4 + 8 * kSpanItemsPerTile) + 512 <= kTileX * kTileY * kFarSlotBytes,
                   "the slices' span work items fit the worklist buffer");
-    k_init_scalars<<<1, 256, 0, st>>>(bt, a.sc, a.ctr, nullptr);
+    k_init_scalars<<<1, 256, 0, st>>>(bt, a.sc, a.ctr, nullptr, nullptr);
     CK(cudaMemsetAsync(far.rtmax, 0xFF, sizeof(int) * (size_t)S * nrt, st));
     k_st_lift<<<(unsigned)((lifts + 255) / 256), 256, 0, st>>>(T, P, (const uint32_t*)c->st.site.p, dxyz, pix, a.sc,
                                                                far.rtmax, nrt);
