@@ -160,9 +160,9 @@ void set_dense_smem_attr() {
         cudaFuncSetAttribute(k_near_dense<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem);
         cudaFuncSetAttribute(k_near_dense<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem);
         cudaFuncSetAttribute(k_region_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(int) * (kMaxBins / kBinsPerSuper)));
+                             (int)(sizeof(int) * kMaxRegions));
         cudaFuncSetAttribute(k_region_part, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(int) * (kMaxBins / kBinsPerSuper)));
+                             (int)(sizeof(int) * kMaxRegions));
         cudaFuncSetAttribute(k_scatter_window, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(sizeof(unsigned long long) * kSpanWindowMaxWords));
         done[dev] = true;
@@ -197,9 +197,10 @@ void launch_prologue(const HostBatch& hb, const BatchTables& bt, const DevArrays
 // ev[0..2] (optional) mark the ends of binning, nearest sites and spans, and
 // ev[4] the end of the ring search (k_near_dense) inside the nearest sites.
 // sites_only: stop after the nearest-site kernels (the site map is the result).
+// unique_gid: no two points share a gid (the engine's own input indices).
 void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a, const int32_t* d_xyz,
                  const uint32_t* d_gid, float* d_h, uint32_t* d_site, int sms, cudaStream_t st,
-                 const cudaEvent_t* ev, bool bbox_in_count = false, bool sites_only = false) {
+                 const cudaEvent_t* ev, bool bbox_in_count = false, bool sites_only = false, bool unique_gid = false) {
     const int nchunk = hb.chunk_base.back();
     const int64_t nblk = hb.blk_base.back(), nsup = hb.sup_base.back();
     const int nrt = hb.rt_base.back();
@@ -243,7 +244,7 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
     // (four CTAs each) without two rounds of work
     int split = 1;
     while (split < kTileY / 8 && (int64_t)nrt * split < 8 * (int64_t)sms) split *= 2;
-    const auto dense = d_gid ? k_near_dense<true> : k_near_dense<false>;
+    const auto dense = d_gid && !unique_gid ? k_near_dense<true> : k_near_dense<false>;
     dense<<<nrt * split, 256, kDenseSmem, st>>>(bt, a.sorted, a.start, a.pix, d_site, far, a.sc, a.ctr, hb.far_blocks,
                                                 hb.dense_band, split);
     if (ev) cudaEventRecord(ev[4], st);

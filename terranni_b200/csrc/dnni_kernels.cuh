@@ -129,28 +129,22 @@ __global__ void __launch_bounds__(256) k_init_scalars(BatchTables bt, Scalars* s
 
 // Bounding box of each tile's points relative to its origin, with range checks
 // (the coordinate range, and the declared extent where the caller gave one):
-// bbox_point per point, bbox_flush once per warp.
+// bbox_point per point on the input coordinates, bbox_flush once per block; a
+// point is out of range exactly when the block's box is.
 struct BBoxAcc {
     int mnx = INT_MAX, mxx = INT_MIN, mny = INT_MAX, mxy = INT_MIN, mnz = INT_MAX, mxz = INT_MIN;
-    unsigned bad = 0;
 };
 
-__device__ __forceinline__ void bbox_point(const TileParams& T, int xr, int yr, int zr, BBoxAcc& acc) {
-    const long long x = (long long)xr - T.ox, y = (long long)yr - T.oy, z = zr;
-    if (x <= -kCoordLimit || x >= kCoordLimit || y <= -kCoordLimit || y >= kCoordLimit || z <= -kCoordLimit ||
-        z >= kCoordLimit || (T.has_ext && (x < T.ex0 || x > T.ex1 || y < T.ey0 || y > T.ey1))) {
-        acc.bad = 1;
-        return;
-    }
-    acc.mnx = min(acc.mnx, (int)x); acc.mxx = max(acc.mxx, (int)x);
-    acc.mny = min(acc.mny, (int)y); acc.mxy = max(acc.mxy, (int)y);
-    acc.mnz = min(acc.mnz, (int)z); acc.mxz = max(acc.mxz, (int)z);
+__device__ __forceinline__ void bbox_point(int x, int y, int z, BBoxAcc& acc) {
+    acc.mnx = min(acc.mnx, x); acc.mxx = max(acc.mxx, x);
+    acc.mny = min(acc.mny, y); acc.mxy = max(acc.mxy, y);
+    acc.mnz = min(acc.mnz, z); acc.mxz = max(acc.mxz, z);
 }
 
 // One reduction per block (kChunkThreads threads), so that a tile's blocks
 // meet in its six words once each: with one per warp the same-address atomics
 // took 0.34 ms of the 0.38 ms pass over 20 M points.
-__device__ __forceinline__ void bbox_flush(BBoxAcc& acc, Scalars* s, BatchCounters* ctr) {
+__device__ __forceinline__ void bbox_flush(const TileParams& T, const BBoxAcc& acc, Scalars* s, BatchCounters* ctr) {
     __shared__ int red[6][kChunkThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int v[6] = {acc.mnx, acc.mxx, acc.mny, acc.mxy, acc.mnz, acc.mxz};
@@ -159,14 +153,22 @@ __device__ __forceinline__ void bbox_flush(BBoxAcc& acc, Scalars* s, BatchCounte
         const int r = k & 1 ? __reduce_max_sync(0xffffffffu, v[k]) : __reduce_min_sync(0xffffffffu, v[k]);
         if (lane == 0) red[k][warp] = r;
     }
-    acc.bad = __reduce_or_sync(0xffffffffu, acc.bad);
-    if (lane == 0 && acc.bad) { atomicOr(&s->err, kErrRange); atomicOr(&ctr->err, kErrRange); }
     __syncthreads();
     if (warp < 6) {
+        // warp 0..5: least and greatest x, y, z of the block
+        const bool top = warp & 1;
         const int x = red[warp][lane & (kChunkThreads / 32 - 1)];
-        const int r = warp & 1 ? __reduce_max_sync(0xffffffffu, x) : __reduce_min_sync(0xffffffffu, x);
+        const int r = top ? __reduce_max_sync(0xffffffffu, x) : __reduce_min_sync(0xffffffffu, x);
         if (lane == 0) {
-            if (warp & 1) atomicMax(&s->bbox[warp], r); else atomicMin(&s->bbox[warp], r);
+            const long long o = warp < 2 ? T.ox : (warp < 4 ? T.oy : 0), rel = (long long)r - o;
+            bool bad = top ? rel >= kCoordLimit : rel <= -kCoordLimit;
+            if (T.has_ext && warp < 4) {
+                const int e = warp < 2 ? (top ? T.ex1 : T.ex0) : (top ? T.ey1 : T.ey0);
+                bad |= top ? rel > e : rel < e;
+            }
+            if (bad) { atomicOr(&s->err, kErrRange); atomicOr(&ctr->err, kErrRange); }
+            const int c = (int)min(max(rel, -kCoordLimit), kCoordLimit);
+            if (top) atomicMax(&s->bbox[warp], c); else atomicMin(&s->bbox[warp], c);
         }
     }
 }
@@ -193,9 +195,9 @@ __global__ void __launch_bounds__(kChunkThreads) k_bbox(BatchTables bt, const in
         }
 #pragma unroll
         for (int k = 0; k < kB; ++k)
-            if (b + k * kChunkThreads + threadIdx.x < c1) bbox_point(T, x[k], y[k], z[k], acc);
+            if (b + k * kChunkThreads + threadIdx.x < c1) bbox_point(x[k], y[k], z[k], acc);
     }
-    bbox_flush(acc, sc + t, ctr);
+    bbox_flush(T, acc, sc + t, ctr);
 }
 
 // A tile's points outside its bin grid (possible only when the caller's
@@ -280,12 +282,12 @@ __global__ void __launch_bounds__(kChunkThreads) k_region_count(BatchTables bt, 
 #pragma unroll
         for (int k = 0; k < kB; ++k) {
             if (b + k * kChunkThreads + threadIdx.x >= c1) continue;
-            if (with_bbox) bbox_point(T, x[k], y[k], z[k], acc);
+            if (with_bbox) bbox_point(x[k], y[k], z[k], acc);
             const int64_t id = point_bin_est(g, inv_bs, rel_coord(x[k], T.ox), rel_coord(y[k], T.oy), bad);
             if (nreg > 1) atomicAdd(&hist[id >> rsh], 1);
         }
     }
-    if (with_bbox) bbox_flush(acc, sc + t, ctr);
+    if (with_bbox) bbox_flush(T, acc, sc + t, ctr);
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&ctr->err, kErrRange);
     if (nreg == 1) return;
     __syncthreads();
@@ -532,11 +534,11 @@ __global__ void __launch_bounds__(kChunkThreads) k_bin_count(BatchTables bt, con
     BBoxAcc acc;
     for (int64_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
         const int xr = p[3 * i], yr = p[3 * i + 1];
-        if (with_bbox) bbox_point(T, xr, yr, p[3 * i + 2], acc);
+        if (with_bbox) bbox_point(xr, yr, p[3 * i + 2], acc);
         const int64_t id = point_bin_checked(T.bg, rel_coord(xr, T.ox), rel_coord(yr, T.oy), bad);
         atomicAdd(&c[id], 1);
     }
-    if (with_bbox) bbox_flush(acc, sc + t, ctr);
+    if (with_bbox) bbox_flush(T, acc, sc + t, ctr);
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&ctr->err, kErrRange);
 }
 

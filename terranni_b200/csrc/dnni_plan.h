@@ -16,6 +16,7 @@ namespace dnni {
 constexpr int64_t kMaxBins = 1LL << 26;
 constexpr int kMaxSide = 32767;
 constexpr int64_t kRegionDirect = 8192;   // points one CTA bins without a partition pass
+constexpr int64_t kMaxRegions = kMaxBins / kBinsPerSuper;   // of one tile
 
 // Validates the work package (nni::WorkPackage, nni.h:66-70, in LAS units)
 // and fills the geometry part of t.  On failure returns the status and sets
@@ -103,10 +104,13 @@ inline void plan_bins(const int32_t bbox[6], int64_t n, double bin_target, TileP
     t.bg.n2y = (int32_t)(nby / kBinsPerSuperEdge);
     t.bg.nbins = nbx * nby;
     // binning regions: one for a small tile (a single CTA bins it straight from
-    // the input), strips of 512 bins up to 2048 of them (a chunk of 4096 points
-    // then still finds several to a strip), superblocks beyond
+    // the input), strips of 512 bins up to the 16384 of them whose counters
+    // fit a chunk's shared-memory histogram, superblocks beyond.  20 M points,
+    // 9800 strips against 1225 superblocks: partition 429 against 290 us, sort
+    // 213 against 429 us; nine tiles of 3.1 M points, 1800 strips each:
+    // partition 507 against 457 us, sort 504 against 915 us
     const int64_t nsup = t.bg.nbins / kBinsPerSuper;
-    t.rsh = nsup > 256 || (nsup == 1 && n <= kRegionDirect) ? 12 : 9;
+    t.rsh = nsup > kMaxRegions / 8 || (nsup == 1 && n <= kRegionDirect) ? 12 : 9;
     // the ring search's bands: halved while the window of an average place
     // (evenly spread points) would pass the shared-memory arrays' sizes; a
     // denser place halves its band further in the kernel

@@ -7,7 +7,7 @@
 // (terranni.cpp:203-368, border copies terranni.cpp:271-302), the loop over
 // work packages (binRun, terranni.cpp:394-426) and the grid assembly
 // (terranni.cpp:430-488).  Here the points go to HBM once and are bucketed
-// there (buckets of 256 x 256 cells, row-major, so one row of buckets is one
+// there (buckets of 128 x 128 cells, row-major, so one row of buckets is one
 // contiguous range of the bucketed points); each tile gathers the buckets of
 // its point box into a staging area and a batch of tiles runs through the
 // ordinary launch sequence.
@@ -15,8 +15,9 @@
 
 namespace dnni {
 
-constexpr int kSegBucketCells = 256;        // bucket side in cells
-constexpr int kSegGatherChunk = 1 << 16;    // points per gather block
+constexpr int kSegBucketCells = 128;        // bucket side in cells (a tile gathers whole buckets around its halo:
+                                            // with 256, 5000 x 4200 cells in nine tiles took 5 % more device time)
+constexpr int kSegGatherChunk = 1 << 12;    // points per gather block
 
 struct SegGrid {
     long long ox, oy;   // LAS origin of cell (0,0)
@@ -24,19 +25,56 @@ struct SegGrid {
     int nbx, nby;
 };
 
+// max(r, 0) / w, for r < 2^32 (inv_w = 1 / w): a float estimate with an exact
+// correction for quotients below 2^20 of 31-bit numbers, which all but far
+// points' are; a 64-bit divide costs twenty times more.
+__device__ __forceinline__ long long seg_div(long long r, long long w, float inv_w) {
+    if (r < 0) return 0;
+    if (r < (1LL << 31) && w < (1LL << 31) && (float)r * inv_w < 1048576.0f)
+        return floor_div_u32((unsigned)r, (unsigned)w, inv_w);
+    return r / w;
+}
+
 // Bucket of a point; points beyond the grid fall into the edge buckets.
 __device__ __forceinline__ int seg_bucket(const SegGrid& g, int x, int y) {
     const long long rx = (long long)x - g.ox, ry = (long long)y - g.oy;
-    long long bx = rx >= 0 ? rx / g.w : 0, by = ry >= 0 ? ry / g.w : 0;
+    const float inv_w = 1.0f / (float)g.w;
+    long long bx = seg_div(rx, g.w, inv_w), by = seg_div(ry, g.w, inv_w);
     bx = bx < g.nbx - 1 ? bx : g.nbx - 1;
     by = by < g.nby - 1 ? by : g.nby - 1;
     return (int)(by * g.nbx + bx);
 }
 
-__global__ void __launch_bounds__(256) k_seg_count(SegGrid g, const int32_t* __restrict__ xyz, int64_t n,
+// Points per bucket: a shared-memory histogram per CTA while the buckets fit
+// one (nh of them; 24 M points met in 340 global counters: 4.58 ms, now 0.11 ms),
+// else global reductions, which then spread over many counters.
+constexpr int kSegHist = 8192;
+__global__ void __launch_bounds__(512) k_seg_count(SegGrid g, const int32_t* __restrict__ xyz, int64_t n, int nh,
                                                    unsigned* __restrict__ cnt) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd(&cnt[seg_bucket(g, xyz[3 * i], xyz[3 * i + 1])], 1u);
+    extern __shared__ unsigned seg_hist[];
+    for (int k = threadIdx.x; k < nh; k += blockDim.x) seg_hist[k] = 0;
+    __syncthreads();
+    constexpr int kB = 4;                       // points in flight
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < n; b += kB * step) {
+        int x[kB], y[kB];
+#pragma unroll
+        for (int k = 0; k < kB; ++k)
+            if (b + k * step < n) {
+                x[k] = xyz[3 * (b + k * step)];
+                y[k] = xyz[3 * (b + k * step) + 1];
+            }
+#pragma unroll
+        for (int k = 0; k < kB; ++k)
+            if (b + k * step < n) {
+                const int q = seg_bucket(g, x[k], y[k]);
+                if (nh) atomicAdd(&seg_hist[q], 1u); else atomicAdd(&cnt[q], 1u);
+            }
+    }
+    if (!nh) return;
+    __syncthreads();
+    for (int k = threadIdx.x; k < nh; k += blockDim.x)
+        if (seg_hist[k]) atomicAdd(&cnt[k], seg_hist[k]);
 }
 
 // Bucketing by partition in two passes, each staged in shared memory: a CTA
@@ -54,7 +92,10 @@ constexpr int kSegPer = kSegPart / 256;     // per thread
 constexpr int kSegKeys = 2048;              // most keys one pass-2 CTA stages
 constexpr int kSegRowKeys = 4096;           // most row groups of pass 1
 
-__device__ __forceinline__ int seg_row(const SegGrid& g, int x, int y) { return seg_bucket(g, x, y) / g.nbx; }
+__device__ __forceinline__ int seg_row(const SegGrid& g, int x, int y) {
+    const long long by = seg_div((long long)y - g.oy, g.w, 1.0f / (float)g.w);
+    return (int)(by < g.nby - 1 ? by : g.nby - 1);
+}
 
 // Exclusive prefix of cnt[0..nk) into off[] by 256 threads (each sums a run
 // of consecutive keys); reserves each non-empty key's range from cur[key0 +
@@ -188,11 +229,14 @@ __global__ void __launch_bounds__(256) k_seg_part_buckets(SegGrid g, const int4*
 
 // One block per bucket: bounding box {minx, miny, maxx, maxy} of its points
 // (INT_MAX, INT_MAX, INT_MIN, INT_MIN when empty).
-__global__ void __launch_bounds__(256) k_seg_bbox(const int32_t* __restrict__ sxyz, const long long* __restrict__ start,
-                                                  int4* __restrict__ bbox) {
-    __shared__ int red[4][8];
+constexpr int kSegBoxThreads = 512;
+__global__ void __launch_bounds__(kSegBoxThreads) k_seg_bbox(const int32_t* __restrict__ sxyz,
+                                                             const long long* __restrict__ start,
+                                                             int4* __restrict__ bbox) {
+    __shared__ int red[4][kSegBoxThreads / 32];
     const long long s0 = start[blockIdx.x], s1 = start[blockIdx.x + 1];
     int mnx = INT_MAX, mny = INT_MAX, mxx = INT_MIN, mxy = INT_MIN;
+#pragma unroll 4
     for (long long i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
         const int x = sxyz[3 * i], y = sxyz[3 * i + 1];
         mnx = min(mnx, x); mxx = max(mxx, x);
@@ -205,7 +249,7 @@ __global__ void __launch_bounds__(256) k_seg_bbox(const int32_t* __restrict__ sx
     __syncthreads();
     if (threadIdx.x == 0) {
         int4 b = make_int4(INT_MAX, INT_MAX, INT_MIN, INT_MIN);
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < kSegBoxThreads / 32; ++k) {
             b.x = min(b.x, red[0][k]); b.y = min(b.y, red[1][k]);
             b.z = max(b.z, red[2][k]); b.w = max(b.w, red[3][k]);
         }
@@ -214,16 +258,42 @@ __global__ void __launch_bounds__(256) k_seg_bbox(const int32_t* __restrict__ sx
 }
 
 // Occupancy of the fine blocks (fw LAS units square) that partition the
-// grid; points beyond the grid are left out.
-__global__ void __launch_bounds__(256) k_seg_occ(SegGrid g, long long fw, int nfx, int nfy,
-                                                 const int32_t* __restrict__ xyz, int64_t n,
+// grid; points beyond the grid are left out.  A CTA of a bucket marks the
+// blocks that the bucket's cells meet (m a side; seg_occ_side) in shared memory
+// and then in occ; with blocks too small for that (m = 0), and for the points
+// that an edge bucket holds from beyond the grid, each point marks its block.
+// (Every point marking its byte of occ in global memory took 0.50 ms for 24 M
+// points, their 82 KB of bytes contended for by every SM.)
+constexpr int kSegOccSide = 96;
+__global__ void __launch_bounds__(512) k_seg_occ(SegGrid g, long long fw, int nfx, int nfy, int m,
+                                                 const int32_t* __restrict__ xyz, const long long* __restrict__ start,
                                                  unsigned char* __restrict__ occ) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    __shared__ unsigned char own[kSegOccSide * kSegOccSide];
+    // grid.y CTAs share a bucket's points (clusters fill some buckets tenfold)
+    const long long b0 = start[blockIdx.x], len = start[blockIdx.x + 1] - b0;
+    const long long s0 = b0 + len * blockIdx.y / gridDim.y, s1 = b0 + len * (blockIdx.y + 1) / gridDim.y;
+    if (s0 == s1) return;
+    const int bx = blockIdx.x % g.nbx, by = blockIdx.x / g.nbx;
+    const long long fx0 = bx * g.w / fw, fy0 = by * g.w / fw;
+    const float inv_fw = 1.0f / (float)fw;
+    for (int k = threadIdx.x; k < m * m; k += blockDim.x) own[k] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (long long i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
         const long long rx = (long long)xyz[3 * i] - g.ox, ry = (long long)xyz[3 * i + 1] - g.oy;
-        if (rx < 0 || ry < 0) continue;
-        const long long fx = rx / fw, fy = ry / fw;
-        if (fx < nfx && fy < nfy) occ[fy * nfx + fx] = 1;
+        const long long fx = seg_div(rx, fw, inv_fw), fy = seg_div(ry, fw, inv_fw), lx = fx - fx0, ly = fy - fy0;
+        if (rx < 0 || ry < 0 || fx >= nfx || fy >= nfy) continue;
+        if (lx < m && ly < m) own[ly * m + lx] = 1;      // (never below fx0, fy0: the bucket starts there)
+        else occ[fy * nfx + fx] = 1;
     }
+    __syncthreads();
+    for (int k = threadIdx.x; k < m * m; k += blockDim.x)
+        if (own[k]) occ[(fy0 + k / m) * nfx + fx0 + k % m] = 1;
+}
+
+inline int seg_occ_side(const SegGrid& g, long long fw) {
+    const long long m = g.w / fw + 2;
+    return m <= kSegOccSide ? (int)m : 0;
 }
 
 // Bounding box {minx, miny, maxx, maxy} of n points (ext pre-set to empty).
@@ -278,13 +348,15 @@ struct SegChunk {
     int count, pad;
 };
 
-__global__ void __launch_bounds__(256) k_seg_gather(const SegChunk* __restrict__ ch, const int32_t* __restrict__ sxyz,
+__global__ void __launch_bounds__(512) k_seg_gather(const SegChunk* __restrict__ ch, const int32_t* __restrict__ sxyz,
                                                     const uint32_t* __restrict__ sgid, int32_t* __restrict__ dxyz,
                                                     uint32_t* __restrict__ dgid) {
     const SegChunk c = ch[blockIdx.x];
     const int32_t* s = sxyz + 3 * c.src;
     int32_t* d = dxyz + 3 * c.dst;
+#pragma unroll 8
     for (int k = threadIdx.x; k < 3 * c.count; k += blockDim.x) d[k] = s[k];
+#pragma unroll 8
     for (int k = threadIdx.x; k < c.count; k += blockDim.x) dgid[c.dst + k] = sgid[c.src + k];
 }
 
@@ -332,7 +404,9 @@ dnni_status bucket_uploaded(dnni_ctx* c, cudaStream_t st, const SegGrid& G, int6
         return rs;
     CK(cudaMemsetAsync(B.cnt.p, 0, 4 * (size_t)nb, st));
     const int grid = c->sm_count * 8;
-    if (n > 0) k_seg_count<<<grid, 256, 0, st>>>(G, (const int32_t*)B.xin.p, n, (unsigned*)B.cnt.p);
+    const int nh = nb <= kSegHist ? nb : 0;
+    if (n > 0)
+        k_seg_count<<<grid / 2, 512, sizeof(unsigned) * nh, st>>>(G, (const int32_t*)B.xin.p, n, nh, (unsigned*)B.cnt.p);
     std::vector<unsigned> cnt(nb);
     start.assign(nb + 1, 0);
     CK(cudaMemcpyAsync(cnt.data(), B.cnt.p, 4 * (size_t)nb, cudaMemcpyDeviceToHost, st));
@@ -358,7 +432,7 @@ dnni_status bucket_uploaded(dnni_ctx* c, cudaStream_t st, const SegGrid& G, int6
         k_seg_part_buckets<<<nblk, 256, sm2, st>>>(G, (const int4*)B.part.p, n, (unsigned long long*)B.cur.p,
                                                    (int32_t*)B.sxyz.p, (uint32_t*)B.sgid.p);
     }
-    k_seg_bbox<<<nb, 256, 0, st>>>((const int32_t*)B.sxyz.p, (const long long*)B.start.p, (int4*)B.bbox.p);
+    k_seg_bbox<<<nb, kSegBoxThreads, 0, st>>>((const int32_t*)B.sxyz.p, (const long long*)B.start.p, (int4*)B.bbox.p);
     bbox.resize(nb);
     CK(cudaMemcpyAsync(bbox.data(), B.bbox.p, 16 * (size_t)nb, cudaMemcpyDeviceToHost, st));
     CK(cudaEventRecord(c->ev[2], st));
@@ -391,8 +465,8 @@ dnni_status occupancy_edt(dnni_ctx* c, cudaStream_t st, const SegGrid& G, long l
     std::vector<unsigned char> occ((size_t)nfx * nfy);
     cudaError_t e = cudaMemsetAsync(occ_d.p, 0, occ.size(), st);
     if (e == cudaSuccess && n > 0)
-        k_seg_occ<<<c->sm_count * 8, 256, 0, st>>>(G, fw, nfx, nfy, (const int32_t*)B.sxyz.p, n,
-                                                   (unsigned char*)occ_d.p);
+        k_seg_occ<<<dim3(G.nbx * G.nby, 2), 512, 0, st>>>(G, fw, nfx, nfy, seg_occ_side(G, fw), (const int32_t*)B.sxyz.p,
+                                                 (const long long*)B.start.p, (unsigned char*)occ_d.p);
     if (e == cudaSuccess) e = cudaMemcpyAsync(occ.data(), occ_d.p, occ.size(), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_err(c, e, "occupancy");
@@ -603,7 +677,7 @@ dnni_status segment_run(dnni_ctx* c, const dnni_segment& s, const int32_t* h_xyz
         uint32_t* gsite = h_site ? (uint32_t*)B.gsite[ob].p : nullptr;
         if (!chunks.empty()) {
             CK(cudaMemcpyAsync(B.chunks.p, chunks.data(), sizeof(SegChunk) * chunks.size(), cudaMemcpyHostToDevice, st));
-            k_seg_gather<<<(int)chunks.size(), 256, 0, st>>>((const SegChunk*)B.chunks.p, (const int32_t*)B.sxyz.p,
+            k_seg_gather<<<(int)chunks.size(), 512, 0, st>>>((const SegChunk*)B.chunks.p, (const int32_t*)B.sxyz.p,
                                                              (const uint32_t*)B.sgid.p, (int32_t*)B.gxyz.p,
                                                              (uint32_t*)B.ggid.p);
         }
@@ -613,7 +687,7 @@ dnni_status segment_run(dnni_ctx* c, const dnni_segment& s, const int32_t* h_xyz
         if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
         launch_prologue(hb, bt, a, (const int32_t*)B.gxyz.p, st, false);
         launch_body(hb, bt, a, (const int32_t*)B.gxyz.p, (const uint32_t*)B.ggid.p, gout, gsite, c->sm_count, st,
-                    nullptr, true);
+                    nullptr, true, false, true);
         CK(cudaGetLastError());
         hsc.resize(ng);
         ring.resize(4 * (size_t)ng);
