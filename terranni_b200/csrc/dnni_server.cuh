@@ -18,6 +18,8 @@ double now_s() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
+constexpr double kSrvGather = 100e-6;   // seconds
+
 struct SrvReq {
     dnni_request r{};
     double t_submit = 0, t_launch = 0, t_done = 0;
@@ -297,13 +299,13 @@ dnni_status srv_launch(dnni_server* s, SrvSlot& sl, std::vector<SrvItem>& items,
     if (nt) CK(cudaMemcpyAsync(a.tables, sl.h_tab, tbytes, cudaMemcpyHostToDevice, st));
     if (!chunks.empty()) {
         CK(cudaMemcpyAsync(dch, sl.h_tab + tbytes, sizeof(SegChunk) * chunks.size(), cudaMemcpyHostToDevice, st));
-        k_seg_gather<<<(int)chunks.size(), 256, 0, st>>>(dch, (const int32_t*)s->B.sxyz.p, (const uint32_t*)s->B.sgid.p,
+        k_seg_gather<<<(int)chunks.size(), 512, 0, st>>>(dch, (const int32_t*)s->B.sxyz.p, (const uint32_t*)s->B.sgid.p,
                                                          gxyz, ggid);
     }
     if (nt) {
         const BatchTables bt = device_tables(a.tables, hb);
         launch_prologue(hb, bt, a, gxyz, st, false);
-        launch_body(hb, bt, a, gxyz, ggid, gout, site ? gsite : nullptr, c->sm_count, st, nullptr, true);
+        launch_body(hb, bt, a, gxyz, ggid, gout, site ? gsite : nullptr, c->sm_count, st, nullptr, true, false, true);
         CK(cudaMemcpyAsync(sl.h_sc, a.sc, sizeof(Scalars) * nt, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(sl.h_ctr, a.ctr, sizeof(BatchCounters), cudaMemcpyDeviceToHost, st));
     }
@@ -476,6 +478,12 @@ void srv_loop(dnni_server* s) {
         // fill free slots from the queue, in arrival order
         for (SrvSlot& sl : s->slots) {
             if (sl.busy || s->queue.empty()) continue;
+            // while another batch runs, a request waits up to kSrvGather for
+            // company: requests submitted together then share a batch however
+            // short a batch has become
+            if (any_busy && !s->stop && (int)s->queue.size() < s->o.max_batch &&
+                now_s() - s->reqs[s->queue.front()].t_submit < kSrvGather)
+                break;
             std::vector<SrvItem> items;
             chunks.clear();
             int64_t pt = 0, out = 0, site = 0;
