@@ -1968,6 +1968,14 @@ __device__ __forceinline__ float finalize_height(long long Z, long long C, doubl
     return __double2float_rn(__dadd_rn(__dmul_rn(q, zs), zo));
 }
 
+// Lattice points within H of the origin.
+constexpr int stencil_taps(int H) {
+    int n = 0;
+    for (int dy = -H; dy <= H; ++dy)
+        for (int dx = -H; dx <= H; ++dx) n += dx * dx + dy * dy <= H * H ? 1 : 0;
+    return n;
+}
+
 // Row scan, stencil and finalize in one pass: one CTA (32 x 16 threads) per
 // band of 16 grid rows of a work package, walking the band's columns in
 // chunks of 32.  Each warp owns one row: it prefix-sums the row's span words
@@ -1975,46 +1983,75 @@ __device__ __forceinline__ float finalize_height(long long Z, long long C, doubl
 // the running sum in a register, so the prefix is never written back; each
 // cell then gathers the small discs (R2 <= H^2) of the pixels within H from
 // the chunk's pixel records in shared memory, adds its prefix, and divides.
+//
+// A launch of fewer bands than SMs cuts them into segments of seg_cols columns,
+// a CTA each (segs of them): a segment's rows start from the sum of the words
+// before it, read once more.
+//
+// Bound by instruction issue (about 270 warp instructions per 32 cells, the
+// double-precision quotient and the row scan more than the stencil) and the
+// latency of the chunk chain.  512^2 cells (32 bands) 24.7 -> 12.0 us, mostly
+// from sixteen segments; 1500 x 1400 cells 63.6 -> 45.2 us; 1024 mixed tiles 2.98 ->
+// 2.61 ms from the chunk's record addresses formed once per band and stencil
+// taps summed as one word.
 template <int H>
 __global__ void __launch_bounds__(512) k_rows_final(BatchTables bt, const int2* __restrict__ pix,
                                                     Scalars* __restrict__ sc,
                                                     const unsigned long long* __restrict__ S_all,
-                                                    const int* __restrict__ Sc_all, float* __restrict__ h_all) {
+                                                    const int* __restrict__ Sc_all, float* __restrict__ h_all, int segs,
+                                                    int seg_cols) {
     constexpr int TX = 32, TY = 16, SW = TX + 2 * H, SH = TY + 2 * H;
     constexpr int NL = (SW * SH + TX * TY - 1) / (TX * TY);   // pixel records each thread loads per chunk
     __shared__ int2 tile[2][SH][SW];                          // double buffer: this chunk and the next
-    const int t = find_tile(bt.band_base, bt.ntiles, blockIdx.x);
+    const int band = blockIdx.x / segs, c_begin = (blockIdx.x - band * segs) * seg_cols;
+    const int t = find_tile(bt.band_base, bt.ntiles, band);
     const TileParams T = bt.tiles[t];
-    const int cy0 = (blockIdx.x - __ldg(&bt.band_base[t])) * TY;
+    if (c_begin >= T.ncols) return;
+    const int c_end = min(c_begin + seg_cols, T.ncols);
+    const int cy0 = (band - __ldg(&bt.band_base[t])) * TY;
     const int2* P = pix + T.pix_off;
     Scalars* s = sc + t;
     const bool packed = s->packed != 0;
     const int K = s->kbits;
     const long long zbase = s->zbase;
+    // a record's place in the stencil: (z - zbase) * 2^KB + 1 and its R2, -1
+    // when the span path has it, so that a cell sums its taps' values and counts
+    // in one 32-bit word; where the sum could overflow (`wide`), z itself
+    constexpr int TAPS = stencil_taps(H), KB = TAPS < 32 ? 5 : (TAPS < 64 ? 6 : 7);
+    const long long zabs = max((long long)s->bbox[5] - zbase, zbase - (long long)s->bbox[4]);
+    const bool wide = zabs >= (1LL << (31 - KB)) / (TAPS + 1);
+    const int zb32 = (int)zbase;
     const int lane = threadIdx.x, tid = threadIdx.y * TX + threadIdx.x;
     const int qy = cy0 + threadIdx.y;
     const bool row_in = qy < T.nrows;
     // the chunk starting at column cx: this thread's pixel records (into
     // registers) and its cell's span words
     int2 rec[NL];
+    const int2* src[NL];                 // the record at column cx = 0, its raster column there, its place in a buffer
+    int col[NL], at[NL];
+#pragma unroll
+    for (int k = 0; k < NL; ++k) {
+        const int idx = tid + k * TX * TY, ly = idx / SW, lx = idx - ly * SW;
+        const int ryi = cy0 - H + ly - T.ry0;
+        at[k] = idx;
+        col[k] = idx < SW * SH && ryi >= 0 && ryi < T.rh ? lx - H - T.rx0 : INT_MIN / 2;   // never inside
+        src[k] = P + ((int64_t)ryi * T.rw + col[k]);
+    }
     auto load_tile = [&](int cx) {
 #pragma unroll
         for (int k = 0; k < NL; ++k) {
-            const int idx = tid + k * TX * TY;
             int2 v = make_int2(0, -1);
-            if (idx < SW * SH) {
-                const int ly = idx / SW, lx = idx - ly * SW;
-                const int rxi = cx - H + lx - T.rx0, ryi = cy0 - H + ly - T.ry0;
-                if (rxi >= 0 && rxi < T.rw && ryi >= 0 && ryi < T.rh) v = P[(int64_t)ryi * T.rw + rxi];
-            }
+            if ((unsigned)(col[k] + cx) < (unsigned)T.rw) v = src[k][cx];
             rec[k] = v;
         }
     };
     auto store_tile = [&](int b) {
 #pragma unroll
         for (int k = 0; k < NL; ++k) {
-            const int idx = tid + k * TX * TY;
-            if (idx < SW * SH) tile[b][idx / SW][idx % SW] = rec[k];
+            int2 v = rec[k];
+            if (v.y > H * H) v.y = -1;
+            if (!wide) v.x = (v.x - zb32) * (1 << KB) + 1;
+            if (k < NL - 1 || at[k] < SW * SH) (&tile[b][0][0])[at[k]] = v;
         }
     };
     auto load_words = [&](int cx, unsigned long long& w, int& wc) {
@@ -2029,15 +2066,29 @@ __global__ void __launch_bounds__(512) k_rows_final(BatchTables bt, const int2* 
     unsigned nod = 0;
     unsigned long long w;
     int wc;
-    load_tile(0);
+    load_tile(c_begin);
     store_tile(0);
-    load_words(0, w, wc);
+    load_words(c_begin, w, wc);
+    if (c_begin > 0 && row_in) {
+        // the words before this segment
+        const int64_t q = T.cell_off + (int64_t)qy * T.ncols;
+#pragma unroll 4
+        for (int c = lane; c < c_begin; c += TX) {
+            carry += S_all[q + c];
+            if (!packed) carry_c += Sc_all[q + c];
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            carry += __shfl_xor_sync(0xffffffffu, carry, o);
+            carry_c += __shfl_xor_sync(0xffffffffu, carry_c, o);
+        }
+    }
     __syncthreads();
     int b = 0;
 #pragma unroll 1
-    for (int cx0 = 0; cx0 < T.ncols; cx0 += TX, b ^= 1) {
+    for (int cx0 = c_begin; cx0 < c_end; cx0 += TX, b ^= 1) {
         // the next chunk's loads are in flight while this one computes
-        const bool more = cx0 + TX < T.ncols;
+        const bool more = cx0 + TX < c_end;
         unsigned long long w_next = 0;
         int wc_next = 0;
         if (more) {
@@ -2047,25 +2098,42 @@ __global__ void __launch_bounds__(512) k_rows_final(BatchTables bt, const int2* 
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned long long y = __shfl_up_sync(0xffffffffu, w, o);
-            const int yc = __shfl_up_sync(0xffffffffu, wc, o);
-            if (lane >= o) {
-                w += y;
-                wc += yc;
-            }
+            if (lane >= o) w += y;
         }
         w += carry;
-        wc += carry_c;
         carry = __shfl_sync(0xffffffffu, w, 31);
-        carry_c = __shfl_sync(0xffffffffu, wc, 31);
-        long long Z = 0, C = 0;
+        if (!packed) {
 #pragma unroll
-        for (int dy = -H; dy <= H; ++dy)
-#pragma unroll
-            for (int dx = -H; dx <= H; ++dx) {
-                if (dx * dx + dy * dy > H * H) continue;
-                const int2 p = tile[b][threadIdx.y + H + dy][lane + H + dx];
-                if (p.y >= dx * dx + dy * dy && p.y <= H * H) { Z += p.x; C += 1; }
+            for (int o = 1; o < 32; o <<= 1) {
+                const int yc = __shfl_up_sync(0xffffffffu, wc, o);
+                if (lane >= o) wc += yc;
             }
+            wc += carry_c;
+            carry_c = __shfl_sync(0xffffffffu, wc, 31);
+        }
+        long long Z = 0, C = 0;
+        if (!wide) {
+            int sum = 0;
+#pragma unroll
+            for (int dy = -H; dy <= H; ++dy)
+#pragma unroll
+                for (int dx = -H; dx <= H; ++dx) {
+                    if (dx * dx + dy * dy > H * H) continue;
+                    const int2 p = tile[b][threadIdx.y + H + dy][lane + H + dx];
+                    if (p.y >= dx * dx + dy * dy) sum += p.x;
+                }
+            C = sum & ((1 << KB) - 1);
+            Z = (long long)(sum >> KB) + C * zbase;
+        } else {
+#pragma unroll 1
+            for (int dy = -H; dy <= H; ++dy)
+#pragma unroll 1
+                for (int dx = -H; dx <= H; ++dx) {
+                    const int d2 = dx * dx + dy * dy;
+                    const int2 p = tile[b][threadIdx.y + H + dy][lane + H + dx];
+                    if (d2 <= H * H && p.y >= d2) { Z += p.x; C += 1; }
+                }
+        }
         const int qx = cx0 + lane;
         if (row_in && qx < T.ncols) {
             if (packed) {
