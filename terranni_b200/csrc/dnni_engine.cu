@@ -195,7 +195,18 @@ void launch_prologue(const HostBatch& hb, const BatchTables& bt, const DevArrays
     k_init_scalars<<<n, 256, 0, st>>>(bt, a.sc, a.ctr, far_layout(a.far, hb.n_far, hb.rt_base.back()).rtmax,
                                       bbox ? nullptr : a.cnt);
     const int nchunk = hb.chunk_base.back();
-    if (bbox && nchunk > 0) k_bbox<<<nchunk, kChunkThreads, 0, st>>>(bt, d_xyz, a.sc, a.ctr);
+    if (bbox && nchunk > 0) k_bbox<<<nchunk, kChunkThreads, 0, st>>>(bt, d_xyz, a.sc, a.ctr, nullptr);
+}
+
+// A single work package's tables (and, with scalars, its scalars and counters;
+// with nreg its region counts), written by a kernel from its arguments.
+void launch_one_tables(const HostBatch& hb, const DevArrays& a, bool scalars, int nreg, cudaStream_t st) {
+    OneTable tab{};
+    const size_t bytes = TableLayout(1).total;
+    static_assert(sizeof(TileParams) + 13 * 16 + 16 <= sizeof(OneTable), "one tile's tables fit the kernel argument");
+    pack_tables(hb, (unsigned char*)&tab);
+    k_init_one<<<1 + nreg / 4096, 256, 0, st>>>(tab, (uint4*)a.tables, (int)(bytes / 16), scalars ? 1 : 0, a.sc, a.ctr, a.cnt,
+                                                nreg);
 }
 
 // Launch sequence, part 2: binning, nearest sites, spans, stencil, finalize.
@@ -204,9 +215,13 @@ void launch_prologue(const HostBatch& hb, const BatchTables& bt, const DevArrays
 // ev[4] the end of the ring search (k_near_dense) inside the nearest sites.
 // sites_only: stop after the nearest-site kernels (the site map is the result).
 // unique_gid: no two points share a gid (the engine's own input indices).
+// packed_sure: the span words hold the counts whatever the search finds, so
+// the separate counts are never read.
+// A single work package's region counts are zero on entry (launch_one_tables).
 void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a, const int32_t* d_xyz,
                  const uint32_t* d_gid, float* d_h, uint32_t* d_site, int sms, cudaStream_t st,
-                 const cudaEvent_t* ev, bool bbox_in_count = false, bool sites_only = false, bool unique_gid = false) {
+                 const cudaEvent_t* ev, bool bbox_in_count = false, bool sites_only = false, bool unique_gid = false,
+                 bool packed_sure = false) {
     const int nchunk = hb.chunk_base.back();
     const int64_t nblk = hb.blk_base.back(), nsup = hb.sup_base.back();
     const int nrt = hb.rt_base.back();
@@ -214,16 +229,10 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
     if (nchunk > 0) {
         if (a.part) {
             const size_t hist = sizeof(int) * hb.max_reg;
-            // a single work package's region counts start at zero here (its
-            // bins were not planned when k_init_scalars ran)
             const bool partition = hb.max_reg > 1;
-            if (partition && !bbox_in_count) cudaMemsetAsync(a.cnt, 0, sizeof(int) * hb.max_reg, st);
             if (partition || bbox_in_count)
                 k_region_count<<<nchunk, kChunkThreads, hist, st>>>(bt, d_xyz, a.cnt, a.sc, a.ctr, bbox_in_count ? 1 : 0);
-            if (partition) {
-                k_region_scan<<<(int)hb.tiles.size(), 1024, 0, st>>>(bt, a.cnt);
-                k_region_part<<<nchunk, kChunkThreads, hist, st>>>(bt, d_xyz, d_gid, a.cnt, a.part);
-            }
+            if (partition) k_region_part<<<nchunk, kChunkThreads, hist, st>>>(bt, d_xyz, d_gid, a.cnt, a.part);
             if (hb.strip_base.back() > 0)
                 k_region_sort<9><<<hb.strip_base.back(), 256, 0, st>>>(bt, d_xyz, d_gid, a.cnt, a.part, a.start, a.sorted,
                                                                        a.bmask, a.smask);
@@ -242,8 +251,8 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
             if (nsup > 0) k_super_masks<<<(int)((nsup * 32 + 255) / 256), 256, 0, st>>>(bt, a.bmask, a.smask);
         }
         const int nrow1 = hb.row1_base.back();
-        if (nrow1 > 0) k_block_rows<<<(nrow1 + 3) / 4, 128, 0, st>>>(bt, a.bmask, a.rownear);
-        if (nblk > 0) k_block_near<<<(int)((nblk + 255) / 256), 256, 0, st>>>(bt, a.rownear, a.near, far.rtmax);
+        if (nrow1 > 0 && hb.max_n2x > kNearMaskCols) k_block_rows<<<(nrow1 + 3) / 4, 128, 0, st>>>(bt, a.bmask, a.rownear);
+        if (nblk > 0) k_block_near<<<(int)((nblk + 255) / 256), 256, 0, st>>>(bt, a.smask, a.rownear, a.near, far.rtmax);
     }
     if (ev) cudaEventRecord(ev[0], st);
     // a raster tile goes to several CTAs while the tiles alone leave the SMs
@@ -254,17 +263,25 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
     dense<<<nrt * split, 256, kDenseSmem, st>>>(bt, a.sorted, a.start, a.pix, d_site, far, a.sc, a.ctr, hb.far_blocks,
                                                 hb.dense_band, split);
     if (ev) cudaEventRecord(ev[4], st);
+    // with as many heavy CTAs as the rasters have groups, they take them all
+    const bool decide_there = nchunk > 0 && !sites_only && hb.tiles.size() == 1 && nrt <= 2048;
     if (nchunk > 0) {
-        k_near_far<<<sms * kFarCtasPerSm, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site,
-                                            a.sc, a.ctr, hb.far_blocks);
-        k_near_far_heavy<<<sms * kFarCtasPerSm, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site,
-                                                  a.sc, a.ctr, hb.far_blocks);
+        if (hb.n_far / 32 > (int64_t)sms * kFarCtasPerSm)
+            k_near_far<<<sms * kFarCtasPerSm, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix,
+                                                            d_site, a.sc, a.ctr, hb.far_blocks);
+        k_near_far_heavy<<<sms * kFarCtasPerSm, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix,
+                                                              d_site, a.sc, a.ctr, hb.far_blocks, a.D,
+                                                              sites_only ? 0 : hb.n_cells, a.Dc,
+                                                              sites_only || packed_sure ? 0 : hb.n_cells,
+                                                              decide_there ? hb.win_words : 0);
     }
     if (sites_only) return;
-    k_decide<<<(int)hb.tiles.size(), 256, 0, st>>>(bt, a.sc, far, a.ctr, hb.win_words);
+    if (!decide_there) k_decide<<<(int)hb.tiles.size(), 256, 0, st>>>(bt, a.sc, far, a.ctr, hb.win_words);
     if (ev) cudaEventRecord(ev[1], st);
-    cudaMemsetAsync(a.D, 0, sizeof(unsigned long long) * hb.n_cells, st);
-    cudaMemsetAsync(a.Dc, 0, sizeof(int) * hb.n_cells, st);
+    if (nchunk == 0) {
+        cudaMemsetAsync(a.D, 0, sizeof(unsigned long long) * hb.n_cells, st);
+        cudaMemsetAsync(a.Dc, 0, sizeof(int) * hb.n_cells, st);
+    }
     launch_spans(hb, bt, a, a.pix, far, 0, 0, sms, st);
     if (ev) cudaEventRecord(ev[2], st);
     launch_rows_final(hb, bt, a.pix, a.sc, a.D, a.Dc, d_h, sms, st);
@@ -376,12 +393,12 @@ static dnni_status run_device(dnni_ctx* c, const dnni_workpackage* wp, const int
     DevArrays a;
     if ((rs = ensure_scratch(c, c->scr, scratch_sizes(hb), a))) return rs;
     BatchTables bt = device_tables(a.tables, hb);
-    if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
     if (timing) CK(cudaEventRecord(c->ev[0], st));
-    launch_prologue(hb, bt, a, d_xyz, st);
-    CK(cudaGetLastError());
+    launch_one_tables(hb, a, true, 0, st);
+    bool packed_sure = false;
     if (n > 0) {
-        CK(cudaMemcpyAsync(c->h_sc, a.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
+        k_bbox<<<hb.chunk_base.back(), kChunkThreads, 0, st>>>(bt, d_xyz, a.sc, a.ctr, c->h_sc);
+        CK(cudaGetLastError());
         CK(cudaStreamSynchronize(st));
         if (c->h_sc->err & kErrRange)
             return set_err(c, DNNI_E_RANGE, "a point lies beyond +-2^30 LAS units of the work-package origin");
@@ -392,9 +409,16 @@ static dnni_status run_device(dnni_ctx* c, const dnni_workpackage* wp, const int
         batch_add(hb, t, 0, 0, d_site ? 0 : -1);
         if ((rs = ensure_scratch(c, c->scr, scratch_sizes(hb), a))) return rs;
         bt = device_tables(a.tables, hb);
-        if ((rs = stage_tables(c, hb, a.tables, st))) return rs;
+        launch_one_tables(hb, a, false, hb.max_reg, st);
+        int packed, K;
+        long long zbase;
+        decide_packing(t.r2cap, (long long)t.rw * t.rh, c->h_sc->bbox[4], c->h_sc->bbox[5], packed, K, zbase);
+        packed_sure = packed != 0;
+    } else {
+        launch_prologue(hb, bt, a, d_xyz, st);
     }
-    launch_body(hb, bt, a, d_xyz, d_gid, d_h, d_site, c->sm_count, st, timing ? &c->ev[1] : nullptr);
+    launch_body(hb, bt, a, d_xyz, d_gid, d_h, d_site, c->sm_count, st, timing ? &c->ev[1] : nullptr, false, false, false,
+                packed_sure);
     CK(cudaGetLastError());
     if (timing) CK(cudaEventRecord(c->ev[4], st));
     if (stats) k_span_hist<<<hb.rt_base.back(), dim3(32, 8), 0, st>>>(bt, a.pix, a.sc);
@@ -1324,6 +1348,8 @@ extern "C" dnni_status dnni_interpolate_segment_device_noalloc(const dnni_workpa
         if (cudaMemcpyAsync(a.tables, tbl.data(), tbl.size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
             return DNNI_E_CUDA;
         bt = device_tables(a.tables, hb);
+        if (hb.max_reg > 1 && a.part && cudaMemsetAsync(a.cnt, 0, sizeof(int) * hb.max_reg, st) != cudaSuccess)
+            return DNNI_E_CUDA;
     }
     launch_body(hb, bt, a, d_xyz, d_gid, d_h, d_site, sms, st, nullptr);
     if (cudaGetLastError() != cudaSuccess) return DNNI_E_CUDA;

@@ -70,7 +70,7 @@ struct BatchCounters {
     int span_next;               // next span work item to hand out
     int nheavy;                  // far groups left to the heavy pass
     int heavy_next;              // next of them to hand out
-    int pad;
+    int ticket;                  // blocks of the bounding-box pass, then of the heavy pass, that have finished
 };
 
 template <typename B>
@@ -117,14 +117,47 @@ __global__ void __launch_bounds__(256) k_init_scalars(BatchTables bt, Scalars* s
         s->bbox[0] = INT_MAX; s->bbox[1] = INT_MIN;
         s->bbox[2] = INT_MAX; s->bbox[3] = INT_MIN;
         s->bbox[4] = INT_MAX; s->bbox[5] = INT_MIN;
-        s->err = 0; s->packed = 0; s->kbits = 0; s->zbase = 0;
-        if (t == 0) { ctr->nfar = 0; ctr->err = 0; ctr->far_next = 0; ctr->nspan = 0; ctr->span_next = 0; ctr->nheavy = 0; ctr->heavy_next = 0; }
+        s->err = 0; s->packed = 0; s->kbits = 0; s->ticket = 0; s->zbase = 0;
+        if (t == 0) { ctr->nfar = 0; ctr->err = 0; ctr->far_next = 0; ctr->nspan = 0; ctr->span_next = 0; ctr->nheavy = 0; ctr->heavy_next = 0; ctr->ticket = 0; }
     }
     if (l < kStatSlots) {
         s->max_r2[l] = -1; s->big_pixels[l] = 0; s->spans[l] = 0; s->nodata[l] = 0;
         s->evals_dense[l] = 0; s->evals_far[l] = 0;
     }
     if (l < kSpanHistBuckets) s->span_hist[l] = 0;
+}
+
+// A single work package's tables, passed by value: no staging buffer, copy or
+// wait between the host's plan and the kernels that read it.
+struct OneTable {
+    uint4 w[32];
+};
+
+__device__ __forceinline__ bool last_block(int* ticket, int blocks) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == blocks - 1;
+    __syncthreads();
+    return last != 0;
+}
+
+// Writes the tables; scalars: and starts the scalars and counters, as
+// k_init_scalars does; nreg: and starts that many region counts at zero.
+__global__ void __launch_bounds__(256) k_init_one(OneTable tab, uint4* __restrict__ tables, int words, int scalars, Scalars* s,
+                                                  BatchCounters* ctr, int* __restrict__ cnt, int nreg) {
+    const int l = threadIdx.x;
+    if (blockIdx.x == 0) {
+        if (l < words) tables[l] = tab.w[l];
+        if (scalars) {
+            for (int k = l; k < (int)(sizeof(Scalars) / sizeof(int)); k += blockDim.x) ((int*)s)[k] = 0;
+            if (l < (int)(sizeof(BatchCounters) / sizeof(int))) ((int*)ctr)[l] = 0;
+            __syncthreads();
+            if (l < kStatSlots) s->max_r2[l] = -1;
+            if (l < 6) s->bbox[l] = l & 1 ? INT_MIN : INT_MAX;
+        }
+    }
+    for (int k = blockIdx.x * blockDim.x + l; k < nreg; k += gridDim.x * blockDim.x) cnt[k] = 0;
 }
 
 // Bounding box of each tile's points relative to its origin, with range checks
@@ -173,8 +206,10 @@ __device__ __forceinline__ void bbox_flush(const TileParams& T, const BBoxAcc& a
     }
 }
 
+// host (optional, one tile): where the last block to finish leaves the box and
+// the error bits for the host, in its mapped memory.
 __global__ void __launch_bounds__(kChunkThreads) k_bbox(BatchTables bt, const int32_t* __restrict__ xyz, Scalars* sc,
-                                                        BatchCounters* ctr) {
+                                                        BatchCounters* ctr, Scalars* host) {
     const int t = find_tile(bt.chunk_base, bt.ntiles, blockIdx.x);
     const TileParams& T = bt.tiles[t];
     const int64_t c0 = (int64_t)(blockIdx.x - __ldg(&bt.chunk_base[t])) * bt.chunk;
@@ -198,6 +233,12 @@ __global__ void __launch_bounds__(kChunkThreads) k_bbox(BatchTables bt, const in
             if (b + k * kChunkThreads + threadIdx.x < c1) bbox_point(x[k], y[k], z[k], acc);
     }
     bbox_flush(T, acc, sc + t, ctr);
+    if (host && last_block(&ctr->ticket, gridDim.x)) {
+        if (threadIdx.x < 6) host->bbox[threadIdx.x] = __ldcg(&sc->bbox[threadIdx.x]);
+        if (threadIdx.x == 6) host->err = __ldcg(&sc->err);
+        if (threadIdx.x == 7) ctr->ticket = 0;
+        __threadfence_system();
+    }
 }
 
 // A tile's points outside its bin grid (possible only when the caller's
@@ -217,8 +258,7 @@ __device__ __forceinline__ int64_t point_bin_checked(const BinGrid& g, int xr, i
 //
 // A region is a run of 2^rsh bins (a superblock or an eighth of one: a strip of
 // 64 x 8 bins), so its points are one range of the sorted array.  k_region_count
-// counts the points per region, k_region_scan turns the counts into ranges,
-// k_region_part groups the points by region (into a part of the scratch that
+// counts the points per region and turns the counts into ranges, k_region_part groups the points by region (into a part of the scratch that
 // later phases use: the span words, pixel records and worklist), and
 // k_region_sort sorts one region's points by bin with the counters in shared
 // memory, writing the bin starts and the occupancy masks on the way.  A tile of
@@ -291,41 +331,34 @@ __global__ void __launch_bounds__(kChunkThreads) k_region_count(BatchTables bt, 
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&ctr->err, kErrRange);
     if (nreg == 1) return;
     __syncthreads();
-    int* cnt = region_arrays(T, bins).cnt;
-    for (int k = threadIdx.x; k < nreg; k += kChunkThreads)
-        if (hist[k]) atomicAdd(&cnt[k], hist[k]);
-}
-
-// One block per tile: the regions' ranges.
-__global__ void __launch_bounds__(1024) k_region_scan(BatchTables bt, int* __restrict__ bins) {
-    __shared__ int wsum[32];
-    const TileParams& T = bt.tiles[blockIdx.x];
-    const int n = (int)(T.bg.nbins >> T.rsh);
-    if (n == 1) return;
     const RegionArrays r = region_arrays(T, bins);
+    for (int k = threadIdx.x; k < nreg; k += kChunkThreads)
+        if (hist[k]) atomicAdd(&r.cnt[k], hist[k]);
+    // the tile's last block turns the counts into the regions' ranges
+    const int blocks = __ldg(&bt.chunk_base[t + 1]) - __ldg(&bt.chunk_base[t]);
+    if (!last_block(&sc[t].ticket, blocks)) return;
+    __shared__ int wsum[kChunkThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int carry = 0;
-    for (int b = 0; b < n; b += 1024) {
-        const int k = b + threadIdx.x;
-        const int v = k < n ? r.cnt[k] : 0;
-        int x = v;
+    for (int b = 0; b < nreg; b += 2 * kChunkThreads) {
+        const int k = b + 2 * threadIdx.x;
+        const int v0 = k < nreg ? __ldcg(&r.cnt[k]) : 0, v1 = k + 1 < nreg ? __ldcg(&r.cnt[k + 1]) : 0;
+        int x = v0 + v1;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
         if (lane == 31) wsum[warp] = x;
         __syncthreads();
-        int w = wsum[lane];
+        int w = lane < kChunkThreads / 32 ? wsum[lane] : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += y; }
-        const int before = warp ? __shfl_sync(0xffffffffu, w, warp - 1) : 0;
-        const int total = __shfl_sync(0xffffffffu, w, 31);
-        if (k < n) {
-            r.start[k] = carry + before + x - v;
-            r.cur[k] = carry + before + x - v;
-        }
+        const int before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31), total = __shfl_sync(0xffffffffu, w, 31);
+        const int run = carry + (warp ? before : 0) + x - v0 - v1;
+        if (k < nreg) { r.start[k] = run; r.cur[k] = run; }
+        if (k + 1 < nreg) { r.start[k + 1] = run + v0; r.cur[k + 1] = run + v0; }
         carry += total;
         __syncthreads();
     }
-    if (threadIdx.x == 0) r.start[n] = carry;
+    if (threadIdx.x == 0) r.start[nreg] = carry;
 }
 
 // A chunk's points to their regions: ranks from a shared-memory histogram, one
@@ -753,8 +786,9 @@ __global__ void __launch_bounds__(128) k_block_rows(BatchTables bt, const uint64
 
 // Also starts the raster tiles' largest R2 at none (the binning's grouped
 // points lay over them until now).
-__global__ void k_block_near(BatchTables bt, const int* __restrict__ rownear, int64_t* __restrict__ near,
-                             int* __restrict__ rtmax) {
+constexpr int kNearMaskCols = 8;     // superblock columns up to which k_block_near needs no row sweep
+__global__ void k_block_near(BatchTables bt, const uint64_t* __restrict__ smask, const int* __restrict__ rownear,
+                             int64_t* __restrict__ near, int* __restrict__ rtmax) {
     const int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     for (int64_t k = w; k < bt.rt_base[bt.ntiles]; k += (int64_t)gridDim.x * blockDim.x) rtmax[k] = -1;
     if (w >= __ldg(&bt.blk_base[bt.ntiles])) return;
@@ -768,6 +802,32 @@ __global__ void k_block_near(BatchTables bt, const int* __restrict__ rownear, in
     const int64_t k = w - T.blk_off;
     const int cx = (int)(k % n1x), cy = (int)(k / n1x);
     const int* rn = rownear + T.blk_off;
+    if (T.bg.n2x <= kNearMaskCols) {
+        // a row of at most 64 blocks is one word, put together from the
+        // superblocks' masks: no row sweep
+        long long best = LLONG_MAX;
+        int bxn = -1, byn = -1;
+        for (int d = 0; d < n1y && (long long)d * d <= best; ++d)
+            for (int sgn = -1; sgn <= 1; sgn += 2) {
+                const int y = cy + sgn * d;
+                if ((d == 0 && sgn > 0) || y < 0 || y >= n1y) continue;
+                uint64_t row = 0;
+                for (int sx = 0; sx < T.bg.n2x; ++sx)
+                    row |= ((__ldg(&smask[T.sup_off + (y >> 3) * T.bg.n2x + sx]) >> (8 * (y & 7))) & 0xFF) << (8 * sx);
+                const uint64_t below = row & (~0ull >> (63 - cx)), above = row & (~0ull << cx);
+                int x = -1;
+                if (below) x = 63 - __clzll((long long)below);
+                if (above) {
+                    const int a = ffs64(above);
+                    if (x < 0 || a - cx < cx - x) x = a;
+                }
+                if (x < 0) continue;
+                const long long v = (long long)(x - cx) * (x - cx) + (long long)d * d;
+                if (v < best) { best = v; bxn = x; byn = y; }
+            }
+        near[w] = bxn >= 0 ? block_index(T.bg, bxn, byn) : -1;
+        return;
+    }
     long long best = LLONG_MAX;
     int bxn = -1, byn = -1;
     for (int d = 0; d < n1y; ++d) {
@@ -1528,53 +1588,6 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
     }
 }
 
-// The heavy groups, one CTA of eight warps each.
-__global__ void __launch_bounds__(256, 4) k_near_far_heavy(BatchTables bt, const int4* __restrict__ pts_all,
-                                                           const int* __restrict__ start_all,
-                                                           const uint64_t* __restrict__ bmask_all,
-                                                           const uint64_t* __restrict__ smask_all,
-                                                           const int64_t* __restrict__ near_all, FarLayout far,
-                                                           int2* __restrict__ pix, uint32_t* __restrict__ site,
-                                                           Scalars* __restrict__ sc, BatchCounters* __restrict__ ctr,
-                                                           int far_blocks) {
-    __shared__ unsigned long long s_bound[32];
-    __shared__ Best s_best[8][32];
-    __shared__ FarBuf s_buf[8];
-    __shared__ int s_k;
-    const bool all = far_all_heavy(ctr->nfar);
-    const int count = all ? ctr->nfar : ctr->nheavy;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int* heavy = (const int*)far.items;
-    for (;;) {
-        __syncthreads();                 // the previous group's readers are done
-        if (threadIdx.x == 0) s_k = atomicAdd(&ctr->heavy_next, 1);
-        __syncthreads();
-        if (s_k >= count) break;
-        FarWork w;
-        far_load(w, bt, far, all ? s_k : heavy[s_k], far_blocks, pts_all, start_all, bmask_all, near_all);
-        if (warp == 0) s_bound[lane] = (unsigned long long)w.b.d2;
-        __syncthreads();
-        const TileParams& T = bt.tiles[w.t];
-        if (far_small(w, T)) far_run<true, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], s_bound, 0);
-        else far_run<false, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], s_bound, 0);
-        w.b.nev = (int)w.nev;
-        s_best[warp][lane] = w.b;
-        __syncthreads();
-        if (warp == 0) {
-            for (int v = 1; v < 8; ++v) {
-                const Best o = s_best[v][lane];
-                w.nev += (unsigned)o.nev;
-                if (o.d2 < w.b.d2 || (o.d2 == w.b.d2 && (o.gid < w.b.gid || (o.gid == w.b.gid && o.z < w.b.z)))) w.b = o;
-            }
-            far_settle(w, T, pix, site, sc, far, blockIdx.x);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// scatter-accumulate and finalize
-// ---------------------------------------------------------------------------
-
 constexpr int kSpanWindowWords = 4096;      // default: 32 KB per CTA (two int32 arrays)
 constexpr int kSpanWindowMaxWords = 26624;  // 208 KB, the most one CTA may take
 constexpr int kSpanChunksPerItem = 2;       // window chunks of one span work item, at least
@@ -1641,7 +1654,7 @@ __device__ __forceinline__ void list_span_items(const BatchTables& bt, int t, in
         int n = 0;
         SpanWindow w;
         if (k < nrt * layers) {
-            const int r2 = far.rtmax[b0 + k];
+            const int r2 = __ldcg(&far.rtmax[b0 + k]);
             if (r2 > rs2) {
                 w = span_window(T, k % nrt, r2, win_words, direct);
                 if (w.c0 <= w.c1 && w.r0 <= w.r1) n = (w.r1 - w.r0 + w.per) / w.per;
@@ -1661,15 +1674,15 @@ __device__ __forceinline__ void list_span_items(const BatchTables& bt, int t, in
 }
 
 // Per tile: the accumulator form of the span path (see decide_packing) and
-// its work items.
-__global__ void __launch_bounds__(256) k_decide(BatchTables bt, Scalars* sc, FarLayout far, BatchCounters* ctr,
-                                                int win_words) {
+// its work items (one block of 256 threads).
+__device__ __forceinline__ void decide_tile(const BatchTables& bt, int t, Scalars* sc, const FarLayout& far,
+                                            BatchCounters* ctr, int win_words) {
     __shared__ int direct;
-    const int t = blockIdx.x, l = threadIdx.x;
+    const int l = threadIdx.x;
     const TileParams& T = bt.tiles[t];
     Scalars* s = sc + t;
     if (l < 32) {
-        int mx = s->max_r2[l];
+        int mx = __ldcg(&s->max_r2[l]);
         mx = __reduce_max_sync(0xffffffffu, mx);
         if (l == 0) {
             int packed, K;
@@ -1684,6 +1697,66 @@ __global__ void __launch_bounds__(256) k_decide(BatchTables bt, Scalars* sc, Far
     __syncthreads();
     list_span_items(bt, t, 1, direct != 0, win_words, far, ctr);
 }
+
+__global__ void __launch_bounds__(256) k_decide(BatchTables bt, Scalars* sc, FarLayout far, BatchCounters* ctr,
+                                                int win_words) {
+    decide_tile(bt, blockIdx.x, sc, far, ctr, win_words);
+}
+
+// The heavy groups, one CTA of eight warps each.  On the way it clears the span
+// words (D, n64 of them) and counts (Dc, n32), which no later phase needs before,
+// and with win_words the last block to finish decides the first tile's
+// accumulator form and lists its work items (k_decide, for a single work
+// package whose raster tiles one block lists quickly).
+__global__ void __launch_bounds__(256, 4) k_near_far_heavy(BatchTables bt, const int4* __restrict__ pts_all,
+                                                           const int* __restrict__ start_all,
+                                                           const uint64_t* __restrict__ bmask_all,
+                                                           const uint64_t* __restrict__ smask_all,
+                                                           const int64_t* __restrict__ near_all, FarLayout far,
+                                                           int2* __restrict__ pix, uint32_t* __restrict__ site,
+                                                           Scalars* __restrict__ sc, BatchCounters* __restrict__ ctr,
+                                                           int far_blocks, unsigned long long* __restrict__ D, int64_t n64,
+                                                           int* __restrict__ Dc, int64_t n32, int win_words) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n64; k += (int64_t)gridDim.x * blockDim.x) D[k] = 0;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n32; k += (int64_t)gridDim.x * blockDim.x) Dc[k] = 0;
+    __shared__ unsigned long long s_bound[32];
+    __shared__ Best s_best[8][32];
+    __shared__ FarBuf s_buf[8];
+    __shared__ int s_k;
+    const bool all = far_all_heavy(ctr->nfar);
+    const int count = all ? ctr->nfar : ctr->nheavy;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int* heavy = (const int*)far.items;
+    for (;;) {
+        __syncthreads();                 // the previous group's readers are done
+        if (threadIdx.x == 0) s_k = atomicAdd(&ctr->heavy_next, 1);
+        __syncthreads();
+        if (s_k >= count) break;
+        FarWork w;
+        far_load(w, bt, far, all ? s_k : heavy[s_k], far_blocks, pts_all, start_all, bmask_all, near_all);
+        if (warp == 0) s_bound[lane] = (unsigned long long)w.b.d2;
+        __syncthreads();
+        const TileParams& T = bt.tiles[w.t];
+        if (far_small(w, T)) far_run<true, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], s_bound, 0);
+        else far_run<false, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], s_bound, 0);
+        w.b.nev = (int)w.nev;
+        s_best[warp][lane] = w.b;
+        __syncthreads();
+        if (warp == 0) {
+            for (int v = 1; v < 8; ++v) {
+                const Best o = s_best[v][lane];
+                w.nev += (unsigned)o.nev;
+                if (o.d2 < w.b.d2 || (o.d2 == w.b.d2 && (o.gid < w.b.gid || (o.gid == w.b.gid && o.z < w.b.z)))) w.b = o;
+            }
+            far_settle(w, T, pix, site, sc, far, blockIdx.x);
+        }
+    }
+    if (win_words && last_block(&ctr->ticket, gridDim.x)) decide_tile(bt, 0, sc, far, ctr, win_words);
+}
+
+// ---------------------------------------------------------------------------
+// scatter-accumulate and finalize
+// ---------------------------------------------------------------------------
 
 __device__ __forceinline__ void emit_span(int row, int a, int b, int ncols, int nrows, bool packed,
                                           unsigned long long v, long long z,

@@ -143,6 +143,7 @@ struct HostBatch {
     std::vector<int> strip_base{0}, whole_base{0};   // binning regions of 512 bins, of 4096 bins
     int max_reg = 1;                     // most regions of a tile
     int max_cols = 1;                    // most grid columns of a tile
+    int max_n2x = 1;                     // most superblock columns of a tile
     int chunk = kChunkSmall;             // points per block in the point passes (set_chunk)
     int64_t n_rows = 0;                  // input point rows the tiles reference
     int64_t n_pts = 0, n_bins = 0, n_pix = 0, n_cells = 0, n_far = 0;
@@ -201,6 +202,7 @@ inline void batch_add(HostBatch& hb, TileParams t, int64_t pt_off, int64_t out_o
     add(hb.grow_base, t.nrows);
     add(hb.band_base, (t.nrows + 15) / 16);
     hb.max_cols = std::max(hb.max_cols, t.ncols);
+    hb.max_n2x = std::max(hb.max_n2x, t.bg.n2x);
     hb.n_rows = std::max<int64_t>(hb.n_rows, pt_off + t.npts);
     hb.n_pts += t.npts;
     hb.n_pix += (int64_t)t.rw * t.rh;

@@ -99,7 +99,7 @@ struct Scalars {
     int32_t err;
     int32_t packed;              // decided after the nearest-site pass
     int32_t kbits;
-    int32_t pad;
+    int32_t ticket;              // blocks of the region count that have finished
     long long zbase;
     int32_t max_r2[kStatSlots];
     unsigned long long big_pixels[kStatSlots];
