@@ -1225,9 +1225,6 @@ __device__ __forceinline__ I interval_gap(I a0, I a1, I b0, I b1) {
     return m > 0 ? m : 0;
 }
 
-// A candidate block with at most this many points is scanned whole, which
-// costs less than its bin rows.
-constexpr int kFarWholeBlock = 24;
 // A warp leaves a group to the heavy pass once it has searched this many
 // blocks for it and more remain: fewer while the groups leave warps without
 // work (below four to a warp), and none at all below one group per CTA of the
@@ -1237,22 +1234,14 @@ constexpr int kFarCtasPerSm = 4;
 __device__ __forceinline__ bool far_all_heavy(int groups) { return groups <= (int)gridDim.x; }
 constexpr int kFarPixels = 32;   // a group spans at most this many cells in x and y
 
-// A warp's buffer of candidate points: lanes fetch one point each, all in
-// flight at once, and every lane then evaluates all of them.
+// A warp's buffer of candidate points, and the circles that hold the discs of
+// each eighth of its pixels (2 x 2, or 4 x 1 in row groups): centre relative to
+// the group's corner and squared radius, rounded up; a negative radius where no
+// pixel is active.
 struct FarBuf {
     int4 p[32];
     int q[32];
-    __device__ __forceinline__ void put(int k, const int4 v, int pos) {
-        p[k] = v;
-        q[k] = pos;
-    }
-    template <typename L>
-    __device__ __forceinline__ void consider_all(L& b, int n) const {
-        __syncwarp();
-#pragma unroll 4
-        for (int k = 0; k < n; ++k) b.consider(p[k], q[k]);
-        __syncwarp();
-    }
+    float4 circle[8];
 };
 
 // 32-bit arithmetic serves a search whose bound is `reach` (per lane, the
@@ -1269,10 +1258,12 @@ __device__ __forceinline__ bool far_fits32(long long reach, int bs, int cs) {
 // group's own; a superblock's blocks, two to a lane, are tested against the
 // group's box at once and searched nearest first, so that the bounds tighten
 // early; in a block, the bins within the largest bound form one run per row
-// (tested the same way), and a run some lane's disc touches is one range of
-// points, evaluated by every lane.  Every test is a lower bound of the
-// distance against an upper bound of what is sought, so nothing that could
-// hold an equally near site is left out.  Uniform control flow in the warp.
+// (tested the same way), and the runs that some lane's disc touches are ranges
+// of points: one point per lane is fetched, and those inside the circle of some
+// eighth of the pixels are evaluated by every lane.  Every test is a lower bound
+// of the distance against an upper bound of what is sought, so nothing that
+// could hold an equally near site is left out.  Uniform control flow in the
+// warp.
 //
 // kCta: the eight warps of a CTA search one group; warp w takes the blocks of
 // one residue class, and the lanes' bounds meet in s_bound.  Otherwise the
@@ -1280,7 +1271,7 @@ __device__ __forceinline__ bool far_fits32(long long reach, int bs, int cs) {
 template <bool k32, bool kCta>
 __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restrict__ pts, const int* __restrict__ start,
                                            const uint64_t* __restrict__ bmask, const uint64_t* __restrict__ smask,
-                                           FarLane<k32>& b, unsigned& nev, FarBuf* buf,
+                                           FarLane<k32>& b, bool act, unsigned& nev, FarBuf* buf, int far_blocks,
                                            volatile unsigned long long* s_bound, int most) {
     using N = FarNum<k32>;
     using I = typename N::I;
@@ -1296,7 +1287,67 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
         const unsigned long long s = s_bound[lane];
         return s < (unsigned long long)b.d2 ? (D)s : b.d2;
     };
-    D maxd = N::warp_max(bound());
+    // the circles of the pixels' eighths; float rounding (a few 2^-23 of the
+    // distances involved) stays inside the factors
+    const int step2 = far_blocks ? 8 : 2;
+    float cx0 = act ? (float)(b.px - X0) : 3e38f, cx1 = act ? (float)(b.px - X0) : -3e38f;
+    float cy0 = act ? (float)(b.py - Y0) : 3e38f, cy1 = act ? (float)(b.py - Y0) : -3e38f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int x = k ? step2 : 1;
+        cx0 = fminf(cx0, __shfl_xor_sync(full, cx0, x));
+        cx1 = fmaxf(cx1, __shfl_xor_sync(full, cx1, x));
+        cy0 = fminf(cy0, __shfl_xor_sync(full, cy0, x));
+        cy1 = fmaxf(cy1, __shfl_xor_sync(full, cy1, x));
+    }
+    const bool none_active = cx0 > cx1;
+    const float ccx = 0.5f * (cx0 + cx1), ccy = 0.5f * (cy0 + cy1);
+    const float half = (0.5f * (cx1 - cx0) + 0.5f * (cy1 - cy0));       // at least half the diagonal
+    const bool writes = !(lane & (1 | step2));
+    const int eighth = far_blocks ? ((lane >> 1) & 3) + 4 * (lane >> 4) : lane >> 2;
+    D maxd;
+    auto new_bounds = [&]() {
+        D m = act ? bound() : (D)0;
+        maxd = N::warp_max(m);
+        D o = __shfl_xor_sync(full, m, 1);
+        m = o > m ? o : m;
+        o = __shfl_xor_sync(full, m, step2);
+        m = o > m ? o : m;
+        const float r = (sqrt_est((float)m) + half) * 1.00001f + 1.0f;
+        if (writes) buf->circle[eighth] = make_float4(ccx, ccy, none_active ? -1.0f : r * r * 1.00001f, 0.0f);
+        __syncwarp();
+    };
+    new_bounds();
+    // one candidate point to a lane, fetched all at once; those inside a circle
+    // are evaluated by every lane
+    auto round = [&](int q, bool in) {
+        int4 p = make_int4(0, 0, 0, 0);
+        if (in) p = __ldg(&pts[q]);
+        const float x = (float)((I)p.x - X0), y = (float)((I)p.y - Y0);
+        bool hit = false;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float4 c = buf->circle[k];
+            const float dx = x - c.x, dy = y - c.y;
+            hit |= fmaf(dx, dx, dy * dy) <= c.z;
+        }
+        in = in && hit;
+        const unsigned got = __ballot_sync(full, in);
+        if (!got) return;
+        if (in) {
+            const int k = __popc(got & ((1u << lane) - 1u));
+            buf->p[k] = p;
+            buf->q[k] = q;
+        }
+        __syncwarp();
+        const int n = __popc(got);
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) b.consider(buf->p[k], buf->q[k]);
+        nev += n;
+        if (kCta && (unsigned long long)b.d2 < s_bound[lane])
+            atomicMin((unsigned long long*)&s_bound[lane], (unsigned long long)b.d2);
+        new_bounds();                    // (its barrier also ends the buffer's use)
+    };
     const I reach = N::reach(maxd);
     auto cell = [&](I v, I o, int n) {   // superblock column (row) of v, clamped to the grid
         const long long c = (long long)v - o;
@@ -1380,16 +1431,18 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
             const int* st = start + (((int64_t)sidx << 6) + m << 6);
             const int bp0 = __shfl_sync(full, second ? first1 : first0, who);
             const int bp1 = __shfl_sync(full, second ? last1 : last0, who);
-            if (bp1 - bp0 <= kFarWholeBlock) {
-                // few points: the block's range whole (its bins are consecutive)
-                if (lane < bp1 - bp0) buf->put(lane, __ldg(&pts[bp0 + lane]), bp0 + lane);
-                buf->consider_all(b, bp1 - bp0);
-                nev += bp1 - bp0;
-            } else {
-                const int t0 = __ldg(&st[lane]), t1 = __ldg(&st[lane + 32]);
+            // the block's runs of points, dealt to the lanes one after the other:
+            // the whole block when it has few points (its bins are
+            // consecutive), else the rows' runs, first to last bin, that some
+            // disc touches
+            uint64_t run = 0;
+            int t0 = 0, t1 = 0, s0 = bp0, e0 = bp1;
+            if (bp1 - bp0 > 32) {
+                e0 = bp0;
+                t0 = __ldg(&st[lane]);
+                t1 = __ldg(&st[lane + 32]);
                 const unsigned bm0 = __shfl_sync(full, second ? (unsigned)mask1 : (unsigned)mask0, who);
                 const unsigned bm1 = __shfl_sync(full, second ? (unsigned)(mask1 >> 32) : (unsigned)(mask0 >> 32), who);
-                uint64_t run;
                 {
                     const I qx = BX0 + (I)(lane & 7) * bs, qy = BY0 + (I)(lane >> 3) * bs;
                     I dx = interval_gap(X0, X1, qx, qx + bs - 1);
@@ -1403,38 +1456,34 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
                     const unsigned hi = __ballot_sync(full, (D)(dx * dx) + (D)(ey * ey) <= maxd);
                     run = (uint64_t)(bm0 & lo) | ((uint64_t)(bm1 & hi) << 32);
                 }
-                // the rows' runs, first to last bin, that some disc touches;
-                // lanes 4r .. 4r + 3 take row r's run of points
-                int ia = 0, ie = 0;
-                while (run) {
-                    const int r = ffs64(run) >> 3;
-                    const unsigned bits = (unsigned)(run >> (8 * r)) & 0xFFu;
-                    run &= ~(0xFFull << (8 * r));
-                    const int a = __ffs(bits) - 1, e = 31 - __clz(bits);
-                    const I qx = BX0 + (I)a * bs, qy = BY0 + (I)r * bs;
-                    I dx = interval_gap((I)b.px, (I)b.px, qx, qx + (I)(e - a + 1) * bs - 1);
-                    I dy = interval_gap((I)b.py, (I)b.py, qy, qy + bs - 1);
-                    if (k32) { dx = dx < 46340 ? dx : 46340; dy = dy < 46340 ? dy : 46340; }
-                    if (__any_sync(full, (D)(dx * dx) + (D)(dy * dy) <= bd) && (lane >> 2) == r) {
-                        ia = 8 * r + a;
-                        ie = 8 * r + e + 1;
-                    }
-                }
-                const int sa0 = __shfl_sync(full, t0, ia & 31), sa1 = __shfl_sync(full, t1, ia & 31);
-                const int se0 = __shfl_sync(full, t0, ie & 31), se1 = __shfl_sync(full, t1, ie & 31);
-                const int e0 = ie == 64 ? bp1 : (ie < 32 ? se0 : se1);
-                for (int q = (ia < 32 ? sa0 : sa1) + (lane & 3); ; q += 4) {
-                    const bool in = q < e0 && ie != 0;
-                    const unsigned got = __ballot_sync(full, in);
-                    if (!got) break;
-                    if (in) buf->put(__popc(got & ((1u << lane) - 1u)), __ldg(&pts[q]), q);
-                    buf->consider_all(b, __popc(got));
-                    nev += __popc(got);
-                }
             }
-            if (kCta && (unsigned long long)b.d2 < s_bound[lane])
-                atomicMin((unsigned long long*)&s_bound[lane], (unsigned long long)b.d2);
-            maxd = N::warp_max(bound());
+            for (;;) {
+                int fill = 0, q = 0;
+                while (fill < 32) {
+                    if (s0 == e0) {
+                        if (!run) break;
+                        const int r = ffs64(run) >> 3;
+                        const unsigned bits = (unsigned)(run >> (8 * r)) & 0xFFu;
+                        run &= ~(0xFFull << (8 * r));
+                        const int a = __ffs(bits) - 1, e = 31 - __clz(bits);
+                        const I qx = BX0 + (I)a * bs, qy = BY0 + (I)r * bs;
+                        I dx = interval_gap((I)b.px, (I)b.px, qx, qx + (I)(e - a + 1) * bs - 1);
+                        I dy = interval_gap((I)b.py, (I)b.py, qy, qy + bs - 1);
+                        if (k32) { dx = dx < 46340 ? dx : 46340; dy = dy < 46340 ? dy : 46340; }
+                        if (!__any_sync(full, (D)(dx * dx) + (D)(dy * dy) <= bd)) continue;
+                        const int ia = 8 * r + a, ie = 8 * r + e + 1;
+                        s0 = __shfl_sync(full, ia < 32 ? t0 : t1, ia & 31);
+                        e0 = __shfl_sync(full, ie < 32 ? t0 : t1, ie & 31);
+                        if (ie == 64) e0 = bp1;
+                    }
+                    const int take = min(32 - fill, e0 - s0);
+                    if ((unsigned)(lane - fill) < (unsigned)take) q = s0 + lane - fill;
+                    fill += take;
+                    s0 += take;
+                }
+                if (fill) round(q, lane < fill);
+                if (fill < 32) break;
+            }
         }
     }
     return true;
@@ -1516,11 +1565,11 @@ __device__ __forceinline__ void far_load(FarWork& w, const BatchTables& bt, cons
 
 template <bool k32, bool kCta>
 __device__ __forceinline__ bool far_run(FarWork& w, const TileParams& T, const int4* pts_all, const int* start_all,
-                                        const uint64_t* bmask_all, const uint64_t* smask_all, FarBuf* buf,
+                                        const uint64_t* bmask_all, const uint64_t* smask_all, FarBuf* buf, int far_blocks,
                                         volatile unsigned long long* s_bound, int most) {
     FarLane<k32> b{w.px, w.py, (typename FarNum<k32>::D)w.b.d2, w.b.gid, w.b.z, w.b.idx};
     const bool done = far_search<k32, kCta>(T.bg, pts_all + T.srt_off, start_all + T.bin_off, bmask_all + T.blk_off,
-                                            smask_all + T.sup_off, b, w.nev, buf, s_bound, most);
+                                            smask_all + T.sup_off, b, w.act, w.nev, buf, far_blocks, s_bound, most);
     w.b.d2 = (long long)b.d2;
     w.b.gid = b.gid;
     w.b.z = b.z;
@@ -1550,8 +1599,10 @@ __device__ __forceinline__ void far_settle(const FarWork& w, const TileParams& T
 
 // Far pass over the worklist: one warp per group, handed out by a counter
 // (groups differ in cost by orders of magnitude: a lake's centre against its
-// shore).  Groups that need more than kFarDefer blocks go, with the sites
-// found so far, to the heavy list (in the span items' place, which are listed
+// shore).  Groups that need more than kFarDefer blocks, or 64-bit arithmetic
+// (this kernel then holds one search, which fits the instruction cache: with
+// both, and the candidate round in four places, a warp waited four issue slots
+// for instructions), go, with the sites found so far, to the heavy list (in the span items' place, which are listed
 // later; at most 64 groups per raster tile).
 __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4* __restrict__ pts_all,
                                                      const int* __restrict__ start_all,
@@ -1576,9 +1627,8 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
         FarWork w;
         far_load(w, bt, far, k, far_blocks, pts_all, start_all, bmask_all, near_all);
         const TileParams& T = bt.tiles[w.t];
-        const bool done = far_small(w, T)
-                              ? far_run<true, false>(w, T, pts_all, start_all, bmask_all, smask_all, buf, nullptr, most)
-                              : far_run<false, false>(w, T, pts_all, start_all, bmask_all, smask_all, buf, nullptr, most);
+        const bool done = far_small(w, T) &&
+                          far_run<true, false>(w, T, pts_all, start_all, bmask_all, smask_all, buf, far_blocks, nullptr, most);
         if (done) {
             far_settle(w, T, pix, site, sc, far, blockIdx.x * 3 + (threadIdx.x >> 5));
         } else {
@@ -1737,8 +1787,8 @@ __global__ void __launch_bounds__(256, 4) k_near_far_heavy(BatchTables bt, const
         if (warp == 0) s_bound[lane] = (unsigned long long)w.b.d2;
         __syncthreads();
         const TileParams& T = bt.tiles[w.t];
-        if (far_small(w, T)) far_run<true, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], s_bound, 0);
-        else far_run<false, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], s_bound, 0);
+        if (far_small(w, T)) far_run<true, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], far_blocks, s_bound, 0);
+        else far_run<false, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], far_blocks, s_bound, 0);
         w.b.nev = (int)w.nev;
         s_best[warp][lane] = w.b;
         __syncthreads();
