@@ -940,8 +940,20 @@ constexpr int kFarBlocksDefault = 1;   // far groups of 8 x 4 pixels
 // shared memory use the global arrays.  Pixels the rings do not settle go to
 // the far worklist, 32 to a group: the warp's 8 x 4 block, or a 32 x 1 row.
 // With no points every pixel is settled as "no site".
+//
+// Bound by instruction issue (79 % of the issue slots; 4096^2, 20 M points:
+// 1400 warp instructions per 32 pixels, a third of them staging and settling,
+// the rest the candidate loops at 22 of 32 lanes).  Visiting a row or column
+// of bins only while the gap to it allows a nearer site, two candidates per
+// loop turn, quotients from float estimates and bands sized from the plan took
+// it from 1074 to 808 us there, and three CTAs per SM with windows of 3584
+// points in place of four with 2560 (taller bands, fewer points staged twice)
+// to 752 us (1024 mixed tiles 9.97 -> 9.33 ms).  split: a launch with too few
+// raster tiles to fill the SMs twice (eight CTAs per SM) cuts them into strips
+// of down to 8 rows; the 512^2 case (128 tiles) 66 -> 24 us, the 96 x 80 case (6
+// tiles) 41 -> 10 us.
 template <bool kDup>
-__global__ void __launch_bounds__(256, 4) k_near_dense(BatchTables bt, const int4* __restrict__ pts_all,
+__global__ void __launch_bounds__(256, 3) k_near_dense(BatchTables bt, const int4* __restrict__ pts_all,
                                                        const int* __restrict__ start_all, int2* __restrict__ pix,
                                                        uint32_t* __restrict__ site, FarLayout far,
                                                        Scalars* __restrict__ sc, BatchCounters* __restrict__ ctr,
