@@ -136,16 +136,39 @@ void release_scratch(dnni_ctx* c, Scratch& s) {
     for (DevBuf* b : bufs) dnni_release(*b, c);
 }
 
+// A kernel launch; chain: as a link of a chain whose kernels start with chained(),
+// so that the next one's blocks are placed before this one has drained.
+template <typename... P, typename... A>
+void launch(bool chain, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    if (!chain) {
+        kernel<<<grid, block, smem, st>>>(P(args)...);
+        return;
+    }
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Row scan, stencil and finalize, for the batch's stencil radius; fewer bands
 // than SMs go in as many segments as it takes for four CTAs per SM (256 bands of
 // 4096 columns: 304 us whole, 315 us in three segments each).
 void launch_rows_final(const HostBatch& hb, const BatchTables& bt, const int2* pix, Scalars* sc,
-                       const unsigned long long* S, const int* Sc, float* h, int sms, cudaStream_t st) {
+                       const unsigned long long* S, const int* Sc, float* h, int sms, cudaStream_t st, bool chain) {
     const int bands = hb.band_base.back(), cols = (hb.max_cols + 31) / 32;      // in chunks of 32
     int segs = bands >= sms ? 1 : std::max(1, std::min(cols, (4 * sms + bands - 1) / std::max(bands, 1)));
     const int seg_cols = 32 * ((cols + segs - 1) / segs);
     segs = (hb.max_cols + seg_cols - 1) / seg_cols;
-    const auto run = [&](auto kernel) { kernel<<<bands * segs, dim3(32, 16), 0, st>>>(bt, pix, sc, S, Sc, h, segs, seg_cols); };
+    const auto run = [&](auto kernel) {
+        launch(chain, kernel, bands * segs, dim3(32, 16), 0, st, bt, pix, sc, S, Sc, h, segs, seg_cols);
+    };
     switch (hb.rs) {
         case 1: run(k_rows_final<1>); break;
         case 2: run(k_rows_final<2>); break;
@@ -179,11 +202,11 @@ void set_dense_smem_attr() {
 // that k_decide listed (layers: stacked rasters of nrt_layer raster tiles and
 // lstride records each, 0 = one).
 void launch_spans(const HostBatch& hb, const BatchTables& bt, const DevArrays& a, const int2* pix, const FarLayout& far,
-                  int nrt_layer, int64_t lstride, int sms, cudaStream_t st) {
+                  int nrt_layer, int64_t lstride, int sms, cudaStream_t st, bool chain = false) {
     const size_t smem = sizeof(unsigned long long) * hb.win_words;
     const int per_sm = std::max(1, std::min(6, (int)((220u << 10) / (smem + 1024))));
-    k_scatter_window<<<sms * per_sm, dim3(32, 8), smem, st>>>(bt, pix, a.sc, a.D, a.Dc, hb.win_words, far, a.ctr,
-                                                             nrt_layer, lstride);
+    launch(chain, k_scatter_window, sms * per_sm, dim3(32, 8), smem, st, bt, pix, a.sc, a.D, a.Dc, hb.win_words, far, a.ctr,
+           nrt_layer, lstride);
 }
 
 // Launch sequence, part 1: per-tile scalars and (with bbox) the point
@@ -205,8 +228,8 @@ void launch_one_tables(const HostBatch& hb, const DevArrays& a, bool scalars, in
     const size_t bytes = TableLayout(1).total;
     static_assert(sizeof(TileParams) + 13 * 16 + 16 <= sizeof(OneTable), "one tile's tables fit the kernel argument");
     pack_tables(hb, (unsigned char*)&tab);
-    k_init_one<<<1 + nreg / 4096, 256, 0, st>>>(tab, (uint4*)a.tables, (int)(bytes / 16), scalars ? 1 : 0, a.sc, a.ctr, a.cnt,
-                                                nreg);
+    launch(true, k_init_one, 1 + nreg / 4096, 256, 0, st, tab, (uint4*)a.tables, (int)(bytes / 16), scalars ? 1 : 0, a.sc, a.ctr,
+           a.cnt, nreg);
 }
 
 // Launch sequence, part 2: binning, nearest sites, spans, stencil, finalize.
@@ -221,7 +244,7 @@ void launch_one_tables(const HostBatch& hb, const DevArrays& a, bool scalars, in
 void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a, const int32_t* d_xyz,
                  const uint32_t* d_gid, float* d_h, uint32_t* d_site, int sms, cudaStream_t st,
                  const cudaEvent_t* ev, bool bbox_in_count = false, bool sites_only = false, bool unique_gid = false,
-                 bool packed_sure = false) {
+                 bool packed_sure = false, bool chain = false) {
     const int nchunk = hb.chunk_base.back();
     const int64_t nblk = hb.blk_base.back(), nsup = hb.sup_base.back();
     const int nrt = hb.rt_base.back();
@@ -231,14 +254,12 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
             const size_t hist = sizeof(int) * hb.max_reg;
             const bool partition = hb.max_reg > 1;
             if (partition || bbox_in_count)
-                k_region_count<<<nchunk, kChunkThreads, hist, st>>>(bt, d_xyz, a.cnt, a.sc, a.ctr, bbox_in_count ? 1 : 0);
-            if (partition) k_region_part<<<nchunk, kChunkThreads, hist, st>>>(bt, d_xyz, d_gid, a.cnt, a.part);
+                launch(chain, k_region_count, nchunk, kChunkThreads, hist, st, bt, d_xyz, a.cnt, a.sc, a.ctr, bbox_in_count ? 1 : 0);
+            if (partition) launch(chain, k_region_part, nchunk, kChunkThreads, hist, st, bt, d_xyz, d_gid, a.cnt, a.part);
             if (hb.strip_base.back() > 0)
-                k_region_sort<9><<<hb.strip_base.back(), 256, 0, st>>>(bt, d_xyz, d_gid, a.cnt, a.part, a.start, a.sorted,
-                                                                       a.bmask, a.smask);
+                launch(chain, k_region_sort<9>, hb.strip_base.back(), 256, 0, st, bt, d_xyz, d_gid, a.cnt, a.part, a.start, a.sorted, a.bmask, a.smask);
             if (hb.whole_base.back() > 0)
-                k_region_sort<12><<<hb.whole_base.back(), 1024, 0, st>>>(bt, d_xyz, d_gid, a.cnt, a.part, a.start,
-                                                                         a.sorted, a.bmask, a.smask);
+                launch(chain, k_region_sort<12>, hb.whole_base.back(), 1024, 0, st, bt, d_xyz, d_gid, a.cnt, a.part, a.start, a.sorted, a.bmask, a.smask);
         } else {
             cudaMemsetAsync(a.cnt, 0, sizeof(int) * hb.n_bins, st);
             k_bin_count<<<nchunk, kChunkThreads, 0, st>>>(bt, d_xyz, a.cnt, a.sc, a.ctr, bbox_in_count ? 1 : 0);
@@ -251,8 +272,8 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
             if (nsup > 0) k_super_masks<<<(int)((nsup * 32 + 255) / 256), 256, 0, st>>>(bt, a.bmask, a.smask);
         }
         const int nrow1 = hb.row1_base.back();
-        if (nrow1 > 0 && hb.max_n2x > kNearMaskCols) k_block_rows<<<(nrow1 + 3) / 4, 128, 0, st>>>(bt, a.bmask, a.rownear);
-        if (nblk > 0) k_block_near<<<(int)((nblk + 255) / 256), 256, 0, st>>>(bt, a.smask, a.rownear, a.near, far.rtmax);
+        if (nrow1 > 0 && hb.max_n2x > kNearMaskCols) launch(chain, k_block_rows, (nrow1 + 3) / 4, 128, 0, st, bt, a.bmask, a.rownear);
+        if (nblk > 0) launch(chain, k_block_near, (int)((nblk + 255) / 256), 256, 0, st, bt, a.smask, a.rownear, a.near, far.rtmax);
     }
     if (ev) cudaEventRecord(ev[0], st);
     // a raster tile goes to several CTAs while the tiles alone leave the SMs
@@ -260,31 +281,25 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
     int split = 1;
     while (split < kTileY / 8 && (int64_t)nrt * split < 8 * (int64_t)sms) split *= 2;
     const auto dense = d_gid && !unique_gid ? k_near_dense<true> : k_near_dense<false>;
-    dense<<<nrt * split, 256, kDenseSmem, st>>>(bt, a.sorted, a.start, a.pix, d_site, far, a.sc, a.ctr, hb.far_blocks,
-                                                hb.dense_band, split);
+    launch(chain, dense, nrt * split, 256, kDenseSmem, st, bt, a.sorted, a.start, a.pix, d_site, far, a.sc, a.ctr, hb.far_blocks, hb.dense_band, split);
     if (ev) cudaEventRecord(ev[4], st);
     // with as many heavy CTAs as the rasters have groups, they take them all
     const bool decide_there = nchunk > 0 && !sites_only && hb.tiles.size() == 1 && nrt <= 2048;
     if (nchunk > 0) {
         if (hb.n_far / 32 > (int64_t)sms * kFarCtasPerSm)
-            k_near_far<<<sms * kFarCtasPerSm, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix,
-                                                            d_site, a.sc, a.ctr, hb.far_blocks);
-        k_near_far_heavy<<<sms * kFarCtasPerSm, 256, 0, st>>>(bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix,
-                                                              d_site, a.sc, a.ctr, hb.far_blocks, a.D,
-                                                              sites_only ? 0 : hb.n_cells, a.Dc,
-                                                              sites_only || packed_sure ? 0 : hb.n_cells,
-                                                              decide_there ? hb.win_words : 0);
+            launch(chain, k_near_far, sms * kFarCtasPerSm, 256, 0, st, bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site, a.sc, a.ctr, hb.far_blocks);
+        launch(chain, k_near_far_heavy, sms * kFarCtasPerSm, 256, 0, st, bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site, a.sc, a.ctr, hb.far_blocks, a.D, sites_only ? 0 : hb.n_cells, a.Dc, sites_only || packed_sure ? 0 : hb.n_cells, decide_there ? hb.win_words : 0);
     }
     if (sites_only) return;
-    if (!decide_there) k_decide<<<(int)hb.tiles.size(), 256, 0, st>>>(bt, a.sc, far, a.ctr, hb.win_words);
+    if (!decide_there) launch(chain, k_decide, (int)hb.tiles.size(), 256, 0, st, bt, a.sc, far, a.ctr, hb.win_words);
     if (ev) cudaEventRecord(ev[1], st);
     if (nchunk == 0) {
         cudaMemsetAsync(a.D, 0, sizeof(unsigned long long) * hb.n_cells, st);
         cudaMemsetAsync(a.Dc, 0, sizeof(int) * hb.n_cells, st);
     }
-    launch_spans(hb, bt, a, a.pix, far, 0, 0, sms, st);
+    launch_spans(hb, bt, a, a.pix, far, 0, 0, sms, st, chain);
     if (ev) cudaEventRecord(ev[2], st);
-    launch_rows_final(hb, bt, a.pix, a.sc, a.D, a.Dc, d_h, sms, st);
+    launch_rows_final(hb, bt, a.pix, a.sc, a.D, a.Dc, d_h, sms, st, chain);
 }
 
 // Sums the per-tile scalars into dnni_stats.
@@ -397,7 +412,7 @@ static dnni_status run_device(dnni_ctx* c, const dnni_workpackage* wp, const int
     launch_one_tables(hb, a, true, 0, st);
     bool packed_sure = false;
     if (n > 0) {
-        k_bbox<<<hb.chunk_base.back(), kChunkThreads, 0, st>>>(bt, d_xyz, a.sc, a.ctr, c->h_sc);
+        launch(true, k_bbox, hb.chunk_base.back(), kChunkThreads, 0, st, bt, d_xyz, a.sc, a.ctr, c->h_sc);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(st));
         if (c->h_sc->err & kErrRange)
@@ -418,7 +433,7 @@ static dnni_status run_device(dnni_ctx* c, const dnni_workpackage* wp, const int
         launch_prologue(hb, bt, a, d_xyz, st);
     }
     launch_body(hb, bt, a, d_xyz, d_gid, d_h, d_site, c->sm_count, st, timing ? &c->ev[1] : nullptr, false, false, false,
-                packed_sure);
+                packed_sure, true);
     CK(cudaGetLastError());
     if (timing) CK(cudaEventRecord(c->ev[4], st));
     if (stats) k_span_hist<<<hb.rt_base.back(), dim3(32, 8), 0, st>>>(bt, a.pix, a.sc);

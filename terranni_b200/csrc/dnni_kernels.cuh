@@ -73,6 +73,15 @@ struct BatchCounters {
     int ticket;                  // blocks of the bounding-box pass, then of the heavy pass, that have finished
 };
 
+// First statement of the kernels that a single work package's call launches as a
+// chain: waits until the kernel before has finished and its writes are visible,
+// then lets the next one's blocks be placed while this one runs (they wait here
+// in turn).  Without the launch attribute both do nothing.
+__device__ __forceinline__ void chained() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+
 template <typename B>
 __device__ __forceinline__ int find_tile(const B* __restrict__ base, int ntiles, long long k) {
     int lo = 0, hi = ntiles - 1;   // last tile with base[t] <= k
@@ -146,6 +155,7 @@ __device__ __forceinline__ bool last_block(int* ticket, int blocks) {
 // k_init_scalars does; nreg: and starts that many region counts at zero.
 __global__ void __launch_bounds__(256) k_init_one(OneTable tab, uint4* __restrict__ tables, int words, int scalars, Scalars* s,
                                                   BatchCounters* ctr, int* __restrict__ cnt, int nreg) {
+    chained();
     const int l = threadIdx.x;
     if (blockIdx.x == 0) {
         if (l < words) tables[l] = tab.w[l];
@@ -210,6 +220,7 @@ __device__ __forceinline__ void bbox_flush(const TileParams& T, const BBoxAcc& a
 // the error bits for the host, in its mapped memory.
 __global__ void __launch_bounds__(kChunkThreads) k_bbox(BatchTables bt, const int32_t* __restrict__ xyz, Scalars* sc,
                                                         BatchCounters* ctr, Scalars* host) {
+    chained();
     const int t = find_tile(bt.chunk_base, bt.ntiles, blockIdx.x);
     const TileParams& T = bt.tiles[t];
     const int64_t c0 = (int64_t)(blockIdx.x - __ldg(&bt.chunk_base[t])) * bt.chunk;
@@ -293,6 +304,7 @@ __device__ __forceinline__ int64_t point_bin_est(const BinGrid& g, float inv_bs,
 __global__ void __launch_bounds__(kChunkThreads) k_region_count(BatchTables bt, const int32_t* __restrict__ xyz,
                                                                 int* __restrict__ bins, Scalars* sc, BatchCounters* ctr,
                                                                 int with_bbox) {
+    chained();
     extern __shared__ int hist[];
     const int t = find_tile(bt.chunk_base, bt.ntiles, blockIdx.x);
     const TileParams& T = bt.tiles[t];
@@ -366,6 +378,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_region_count(BatchTables bt, 
 __global__ void __launch_bounds__(kChunkThreads, 2) k_region_part(BatchTables bt, const int32_t* __restrict__ xyz,
                                                                const uint32_t* __restrict__ gid, int* __restrict__ bins,
                                                                int4* __restrict__ part) {
+    chained();
     extern __shared__ int hist[];
     constexpr int kPer = kChunkLarge / kChunkThreads;
     const int t = find_tile(bt.chunk_base, bt.ntiles, blockIdx.x);
@@ -428,6 +441,7 @@ __global__ void __launch_bounds__(kRsh == 9 ? 256 : 1024, kRsh == 9 ? 6 : 2) k_r
                                                               const int4* __restrict__ part, int* __restrict__ start_all,
                                                               int4* __restrict__ sorted, uint64_t* __restrict__ bmask,
                                                               uint64_t* __restrict__ smask) {
+    chained();
     constexpr int kSortThreads = kRsh == 9 ? 256 : 1024, nb = 1 << kRsh, mask = nb - 1;
     constexpr int kHold = kRsh == 9 ? 8 : 0, kB = 4;     // kB: loads in flight before the first atomic
     __shared__ int cnt[nb + 1];
@@ -753,6 +767,7 @@ __global__ void __launch_bounds__(256) k_super_masks(BatchTables bt, const uint6
 // blocks one by one, took 90 us for 20 M points on 4096^2 cells).
 __global__ void __launch_bounds__(128) k_block_rows(BatchTables bt, const uint64_t* __restrict__ bmask,
                                                     int* __restrict__ rownear) {
+    chained();
     const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (r >= __ldg(&bt.row1_base[bt.ntiles])) return;
     const int t = find_tile(bt.row1_base, bt.ntiles, r);
@@ -789,6 +804,7 @@ __global__ void __launch_bounds__(128) k_block_rows(BatchTables bt, const uint64
 constexpr int kNearMaskCols = 8;     // superblock columns up to which k_block_near needs no row sweep
 __global__ void k_block_near(BatchTables bt, const uint64_t* __restrict__ smask, const int* __restrict__ rownear,
                              int64_t* __restrict__ near, int* __restrict__ rtmax) {
+    chained();
     const int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     for (int64_t k = w; k < bt.rt_base[bt.ntiles]; k += (int64_t)gridDim.x * blockDim.x) rtmax[k] = -1;
     if (w >= __ldg(&bt.blk_base[bt.ntiles])) return;
@@ -958,6 +974,7 @@ __global__ void __launch_bounds__(256, 3) k_near_dense(BatchTables bt, const int
                                                        uint32_t* __restrict__ site, FarLayout far,
                                                        Scalars* __restrict__ sc, BatchCounters* __restrict__ ctr,
                                                        int far_blocks, int band0, int split) {
+    chained();
     extern __shared__ int4 smem[];
     int4* s_pts = smem;
     int* s_lstart = (int*)(smem + kWinMaxPts + 1);
@@ -1624,6 +1641,7 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
                                                      FarLayout far, int2* __restrict__ pix,
                                                      uint32_t* __restrict__ site, Scalars* __restrict__ sc,
                                                      BatchCounters* __restrict__ ctr, int far_blocks) {
+    chained();
     __shared__ FarBuf s_buf[8];
     const int count = ctr->nfar;
     if (far_all_heavy(count)) return;
@@ -1762,6 +1780,7 @@ __device__ __forceinline__ void decide_tile(const BatchTables& bt, int t, Scalar
 
 __global__ void __launch_bounds__(256) k_decide(BatchTables bt, Scalars* sc, FarLayout far, BatchCounters* ctr,
                                                 int win_words) {
+    chained();
     decide_tile(bt, blockIdx.x, sc, far, ctr, win_words);
 }
 
@@ -1779,6 +1798,7 @@ __global__ void __launch_bounds__(256, 4) k_near_far_heavy(BatchTables bt, const
                                                            Scalars* __restrict__ sc, BatchCounters* __restrict__ ctr,
                                                            int far_blocks, unsigned long long* __restrict__ D, int64_t n64,
                                                            int* __restrict__ Dc, int64_t n32, int win_words) {
+    chained();
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n64; k += (int64_t)gridDim.x * blockDim.x) D[k] = 0;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n32; k += (int64_t)gridDim.x * blockDim.x) Dc[k] = 0;
     __shared__ unsigned long long s_bound[32];
@@ -1905,6 +1925,7 @@ __global__ void __launch_bounds__(256) k_scatter_window(BatchTables bt, const in
                                                         int* __restrict__ Dc_all, int win_words, FarLayout far,
                                                         BatchCounters* __restrict__ ctr, int nrt_layer,
                                                         int64_t lstride) {
+    chained();
     extern __shared__ int swin[];              // 2 x win_words: z - zbase sums, then counts
     __shared__ int s_item;
     const int count = ctr->nspan;
@@ -2135,6 +2156,7 @@ __global__ void __launch_bounds__(512) k_rows_final(BatchTables bt, const int2* 
                                                     const unsigned long long* __restrict__ S_all,
                                                     const int* __restrict__ Sc_all, float* __restrict__ h_all, int segs,
                                                     int seg_cols) {
+    chained();
     constexpr int TX = 32, TY = 16, SW = TX + 2 * H, SH = TY + 2 * H;
     constexpr int NL = (SW * SH + TX * TY - 1) / (TX * TY);   // pixel records each thread loads per chunk
     __shared__ int2 tile[2][SH][SW];                          // double buffer: this chunk and the next
