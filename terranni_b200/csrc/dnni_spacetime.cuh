@@ -510,7 +510,7 @@ static dnni_status spacetime_run(dnni_ctx* c, const dnni_workpackage* wp, const 
         const int32_t* dx = m > 0 ? (const int32_t*)c->st.xyz.p : nullptr;
         launch_prologue(vb, vbt, va, dx, st, false);
         launch_body(vb, vbt, va, dx, (const uint32_t*)c->st.idx.p, nullptr, (uint32_t*)c->st.site.p, c->sm_count, st,
-                    nullptr, true, true, true);
+                    nullptr, true, true, true, false, true);
         CK(cudaGetLastError());
     }
     if (timing) CK(cudaEventRecord(c->ev[1], st));
