@@ -40,8 +40,8 @@ sys.path.insert(0, ROOT)
 
 METRIC = "DEM cells/s batched vs plain GPU NNI at ≤1e-4 m err vs FP64; p50/p99 tile latency"
 UNIT = "cells/s"
-KERNELS_PER_CALL = 16      # own kernel launches per single-work-package call with points
-KERNELS_PER_BATCH = 15     # per batch run (the bounding boxes come with the bin counts)
+KERNELS_PER_CALL = 14      # own kernel launches of a 4096^2-cell call (smaller ones merge up to five of them)
+KERNELS_PER_BATCH = 12     # per batch run, at least (a row sweep and a second region size where tiles need them)
 FALLBACK_HBM_GBS = 6650.0
 BASE_SEED = 20261203
 
@@ -975,7 +975,7 @@ def run_engine_spacetime(args, world, rank, local):
             # per call: grouping (3), the per-value nearest-site batch (12), the
             # lift and packing decision (3), one span pass per slice, the row scan
             # and the gather-and-divide
-            "gpu_launches": args.steps * (20 + 2 * rt + 1),
+            "gpu_launches": args.steps * 17,
             "cpu_baseline": cpu, "accuracy": acc, "clocks": clk.summary(),
         }), flush=True)
     eng.close()

@@ -6,7 +6,7 @@
 // Replaces, per work package:
 //   nni.cpp:722-790 renderInputPoints / nni.cpp:171-230 drawPlane (the GL
 //     depth-tested site planes that leave each pixel's nearest site in the
-//     colour buffer)                       -> k_bin_* + k_nearest
+//     colour buffer)                       -> k_region_* + k_near_dense/far
 //   nni.cpp:794-820 performNNIQueries / nni.cpp:483-534 makeBlocks and
 //     cuda_nni.cu:407-488 calcNNI (query planes OR-blended into bit masks,
 //     then per-pixel int32 atomics)        -> k_scatter_window + k_rows_final stencil
