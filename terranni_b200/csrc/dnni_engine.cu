@@ -291,7 +291,7 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
         launch(chain, k_near_far_heavy, sms * kFarCtasPerSm, 256, 0, st, bt, a.sorted, a.start, a.bmask, a.smask, a.near, far, a.pix, d_site, a.sc, a.ctr, hb.far_blocks, a.D, sites_only ? 0 : hb.n_cells, a.Dc, sites_only || packed_sure ? 0 : hb.n_cells, decide_there ? hb.win_words : 0);
     }
     if (sites_only) return;
-    if (!decide_there) launch(chain, k_decide, (int)hb.tiles.size(), 256, 0, st, bt, a.sc, far, a.ctr, hb.win_words);
+    if (!decide_there) launch(chain, k_decide, (int)hb.tiles.size(), hb.tiles.size() == 1 ? 1024 : 256, 0, st, bt, a.sc, far, a.ctr, hb.win_words);
     if (ev) cudaEventRecord(ev[1], st);
     if (nchunk == 0) {
         cudaMemsetAsync(a.D, 0, sizeof(unsigned long long) * hb.n_cells, st);

@@ -1754,7 +1754,7 @@ __device__ __forceinline__ void list_span_items(const BatchTables& bt, int t, in
 }
 
 // Per tile: the accumulator form of the span path (see decide_packing) and
-// its work items (one block of 256 threads).
+// its work items (one block).
 __device__ __forceinline__ void decide_tile(const BatchTables& bt, int t, Scalars* sc, const FarLayout& far,
                                             BatchCounters* ctr, int win_words) {
     __shared__ int direct;
@@ -1778,7 +1778,7 @@ __device__ __forceinline__ void decide_tile(const BatchTables& bt, int t, Scalar
     list_span_items(bt, t, 1, direct != 0, win_words, far, ctr);
 }
 
-__global__ void __launch_bounds__(256) k_decide(BatchTables bt, Scalars* sc, FarLayout far, BatchCounters* ctr,
+__global__ void __launch_bounds__(1024) k_decide(BatchTables bt, Scalars* sc, FarLayout far, BatchCounters* ctr,
                                                 int win_words) {
     chained();
     decide_tile(bt, blockIdx.x, sc, far, ctr, win_words);
