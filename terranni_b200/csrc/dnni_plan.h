@@ -192,9 +192,11 @@ inline void batch_add(HostBatch& hb, TileParams t, int64_t pt_off, int64_t out_o
         v.push_back((int)std::min<int64_t>(x, kMaxLaunchIndex));
     };
     add(hb.chunk_base, (t.npts + hb.chunk - 1) / hb.chunk);
-    add(hb.strip_base, t.rsh == 9 ? nbins >> 9 : 0);
-    add(hb.whole_base, t.rsh == 12 ? nbins >> 12 : 0);
-    hb.max_reg = std::max<int>(hb.max_reg, (int)(nbins >> t.rsh));
+    // (a tile without points has no region to sort: nothing counts its points,
+    // so its regions' ranges are never written, and no later kernel reads its bins)
+    add(hb.strip_base, t.npts > 0 && t.rsh == 9 ? nbins >> 9 : 0);
+    add(hb.whole_base, t.npts > 0 && t.rsh == 12 ? nbins >> 12 : 0);
+    if (t.npts > 0) hb.max_reg = std::max<int>(hb.max_reg, (int)(nbins >> t.rsh));
     add(hb.scan_base, (nbins + 1 + kScanTile - 1) / kScanTile);
     add(hb.row1_base, t.npts > 0 ? (t.bg.nby >> 3) : 0);
     add(hb.rt_base, (int64_t)((t.rw + kTileX - 1) / kTileX) * ((t.rh + kTileY - 1) / kTileY));

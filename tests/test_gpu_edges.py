@@ -1,0 +1,78 @@
+"""Calls at the edges of the engine's routes, bit for bit against the oracle:
+thin tiles without points beside tiles with points."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    from terranni_b200 import engine
+    e = engine.Engine(device=0)
+    yield e
+    e.close()
+
+
+def _same(a, b):
+    return np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+def _points(rng, n, w, h):
+    return np.stack([rng.integers(0, w, n), rng.integers(0, h, n), rng.integers(0, 3000, n)], 1).astype(np.int32)
+
+
+# tiles (ncols, nrows, points): the thin ones have several superblocks of bins
+@pytest.mark.parametrize("bin_target", [0, 1])
+@pytest.mark.parametrize("shapes", [
+    [(170, 1, 0), (64, 48, 3000)],
+    [(120, 90, 20000), (1, 300, 0), (512, 1, 0), (300, 2, 500), (2, 300, 0)],
+    [(20000, 2, 0), (512, 1, 40), (50, 1, 0), (40, 40, 9000)],
+])
+def test_batch_with_thin_empty_tiles(eng, oracle, shapes, bin_target):
+    from terranni_b200 import engine
+    rng = np.random.default_rng(len(shapes) + bin_target)
+    rows, tiles, pt, out = [], [], 0, 0
+    for nc, nr, n in shapes:
+        xyz = _points(rng, n, nc * 100, nr * 100)
+        tiles.append(engine.make_tile(engine.make_wp(nc, nr, 100), pt, n, out, out))
+        rows.append(xyz)
+        pt += n
+        out += nc * nr
+    xyz = np.concatenate(rows)
+    h, site = np.empty(out, np.float32), np.empty(out, np.uint32)
+    for order in (False, True):
+        with eng.batch(tiles, bin_target=bin_target, order_by_cost=order) as b:
+            for _ in range(2):
+                h[:], site[:] = 7.0, 7
+                b.run(xyz, h, out_site=site)
+                o = 0
+                for (nc, nr, n), p in zip(shapes, rows):
+                    g, s = h[o:o + nc * nr].reshape(nr, nc), site[o:o + nc * nr].reshape(nr, nc)
+                    o += nc * nr
+                    if n == 0:
+                        assert np.all(g == np.float32(-9999.0)) and np.all(s == 0xFFFFFFFF)
+                        continue
+                    ref = oracle.interpolate(oracle.make_wp(nc, nr, 100), p)
+                    assert _same(g, ref["h"]) and np.array_equal(s, ref["site"])
+
+
+def test_spacetime_transect_with_empty_time_values(eng, oracle):
+    from terranni_b200 import engine
+    rng = np.random.default_rng(4)
+    for nc, nr in ((512, 1), (1, 400)):
+        xyz = _points(rng, 9000, nc * 100, nr * 100)
+        t = rng.choice(np.array([-2, 0, 1]), 9000).astype(np.int32)      # of the values -2 .. 2, two have no point
+        ref = oracle.interpolate_spacetime(oracle.make_wp(nc, nr, 100), xyz, t, 0, 1, 120)
+        h, _ = eng.interpolate_spacetime(engine.make_wp(nc, nr, 100), xyz, t, 0, 1, 120)
+        assert _same(h, ref["h"])
+
+
+def test_segment_row_with_empty_tiles(eng, oracle):
+    rng = np.random.default_rng(6)
+    xyz = _points(rng, 12000, 100_000, 100)
+    xyz[6000:, 0] += 200_000                            # cells 1000 to 2000 hold no point
+    ref = oracle.interpolate(oracle.make_wp(3000, 1, 100), xyz)
+    for halo in (2, 0):
+        h, site, st = eng.segment_run(xyz, 3000, 1, 100, tile=250, halo=halo, tiles_per_batch=6, site=True)
+        assert _same(h, ref["h"]) and np.array_equal(site, ref["site"])
