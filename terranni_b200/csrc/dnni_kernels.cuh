@@ -1316,8 +1316,7 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
         const unsigned long long s = s_bound[lane];
         return s < (unsigned long long)b.d2 ? (D)s : b.d2;
     };
-    // the circles of the pixels' eighths; float rounding (a few 2^-23 of the
-    // distances involved) stays inside the factors
+    // the circles of the pixels' eighths (far_half, far_circle_r2)
     const int step2 = far_blocks ? 8 : 2;
     float cx0 = act ? (float)(b.px - X0) : 3e38f, cx1 = act ? (float)(b.px - X0) : -3e38f;
     float cy0 = act ? (float)(b.py - Y0) : 3e38f, cy1 = act ? (float)(b.py - Y0) : -3e38f;
@@ -1331,7 +1330,7 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
     }
     const bool none_active = cx0 > cx1;
     const float ccx = 0.5f * (cx0 + cx1), ccy = 0.5f * (cy0 + cy1);
-    const float half = (0.5f * (cx1 - cx0) + 0.5f * (cy1 - cy0));       // at least half the diagonal
+    const float half = far_half(cx1 - cx0, cy1 - cy0, fmaxf((float)(X1 - X0), (float)(Y1 - Y0)));
     const bool writes = !(lane & (1 | step2));
     const int eighth = far_blocks ? ((lane >> 1) & 3) + 4 * (lane >> 4) : lane >> 2;
     D maxd;
@@ -1342,8 +1341,8 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
         m = o > m ? o : m;
         o = __shfl_xor_sync(full, m, step2);
         m = o > m ? o : m;
-        const float r = (sqrt_est((float)m) + half) * 1.00001f + 1.0f;
-        if (writes) buf->circle[eighth] = make_float4(ccx, ccy, none_active ? -1.0f : r * r * 1.00001f, 0.0f);
+        const float r2 = far_circle_r2(sqrt_est((float)m), half);
+        if (writes) buf->circle[eighth] = make_float4(ccx, ccy, none_active ? -1.0f : r2, 0.0f);
         __syncwarp();
     };
     new_bounds();
@@ -1357,8 +1356,7 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const float4 c = buf->circle[k];
-            const float dx = x - c.x, dy = y - c.y;
-            hit |= fmaf(dx, dx, dy * dy) <= c.z;
+            hit |= far_in_circle(x, y, c.x, c.y, c.z);
         }
         in = in && hit;
         const unsigned got = __ballot_sync(full, in);

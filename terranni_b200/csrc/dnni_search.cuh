@@ -139,6 +139,25 @@ DNNI_HD int isqrt_i32(int v) {
     return s;
 }
 
+// The far pass's filter of candidate points: a point is left out when it lies
+// outside the circles of all eighths of a group's pixels.  An eighth's circle is
+// centred on its pixels' box (w x h) and has their largest bound plus half the
+// box's diagonal (at most w/2 + h/2) as its radius; centre and point are floats
+// relative to the group's corner.  Rounding must never leave out a point that
+// lies on a bound: the relative part (a few 2^-23 of the radius) is inside the
+// factors; what the offsets themselves lose, up to 2^-24 of each of the point's
+// x, the centre's and the two ends it is the mean of, grows with the group's
+// extent `ext` and not with the radius, and is inside the term of 2^-20.
+DNNI_HD float far_half(float w, float h, float ext) { return 0.5f * w + 0.5f * h + ext * (1.0f / (1 << 20)); }
+DNNI_HD float far_circle_r2(float root, float half) {
+    const float r = (root + half) * 1.00001f + 1.0f;
+    return r * r * 1.00001f;
+}
+DNNI_HD bool far_in_circle(float x, float y, float cx, float cy, float r2) {
+    const float dx = x - cx, dy = y - cy;
+    return fmaf(dx, dx, dy * dy) <= r2;
+}
+
 // a / b for 0 <= a < 2^32, 0 < b < 2^32 (32-bit unsigned divide; a 64-bit
 // divide costs several times more on the GPU)
 DNNI_HD int udiv32(long long a, long long b) { return (int)((uint32_t)a / (uint32_t)b); }

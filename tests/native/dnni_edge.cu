@@ -33,3 +33,27 @@ extern "C" int edge_batch_regions(int32_t n, const int32_t* ncols, const int32_t
     *max_reg = hb.max_reg;
     return 0;
 }
+
+// The far pass's filter for one eighth of a group, as far_search forms it: four
+// pixels (px, py relative to the group's corner, active where act) with their
+// bounds d2, the group's extent, and a point (relative to the corner): hit.  The
+// root is taken low by more than the device's estimate can be.
+extern "C" void edge_circle(int64_t n, const int64_t* px, const int64_t* py, const uint8_t* act, const int64_t* d2,
+                            const int64_t* ext, const int64_t* qx, const int64_t* qy, uint8_t* hit) {
+    for (int64_t k = 0; k < n; ++k) {
+        float cx0 = 3e38f, cx1 = -3e38f, cy0 = 3e38f, cy1 = -3e38f;
+        int64_t m = 0;
+        for (int64_t e = 4 * k; e < 4 * k + 4; ++e) {
+            if (!act[e]) continue;
+            cx0 = fminf(cx0, (float)px[e]);
+            cx1 = fmaxf(cx1, (float)px[e]);
+            cy0 = fminf(cy0, (float)py[e]);
+            cy1 = fmaxf(cy1, (float)py[e]);
+            m = d2[e] > m ? d2[e] : m;
+        }
+        const float half = far_half(cx1 - cx0, cy1 - cy0, (float)ext[k]);
+        const float root = sqrtf((float)m) * (1.0f - 4.0f / (1 << 23));
+        hit[k] = far_in_circle((float)qx[k], (float)qy[k], 0.5f * (cx0 + cx1), 0.5f * (cy0 + cy1),
+                               far_circle_r2(root, half));
+    }
+}

@@ -76,3 +76,31 @@ def test_segment_row_with_empty_tiles(eng, oracle):
     for halo in (2, 0):
         h, site, st = eng.segment_run(xyz, 3000, 1, 100, tile=250, halo=halo, tiles_per_batch=6, site=True)
         assert _same(h, ref["h"]) and np.array_equal(site, ref["site"])
+
+
+# rings of points around pixels that lie more than 2^24 units apart: nearest and
+# next differ by a unit or less, and the far pass's float filter works on offsets
+# that round by several.  The pixels between hold a point each and are settled
+# before, so that a ring's pixel is alone in its eighth of the group.
+@pytest.mark.parametrize("cell,count", [(3_000_000, 32), (10_000_000, 8), (15_000_000, 8), (10_000_000, 32)])
+def test_far_pass_on_wide_cells(oracle, cell, count):
+    from terranni_b200 import engine
+    rng = np.random.default_rng(cell + count)
+    n = 320_000 // count
+    rows = []
+    for k in range(0, count, 4):
+        a, rad = rng.uniform(0, 2 * np.pi, n), rng.uniform(40_000, 40_004, n)
+        rows.append(np.stack([k * cell + rad * np.cos(a), rad * np.sin(a), rng.integers(0, 3000, n)], 1))
+        rows.append(np.stack([(k + np.arange(1, 4)) * cell, np.zeros(3), rng.integers(0, 3000, 3)], 1))
+    xyz = np.rint(np.concatenate(rows)).astype(np.int32)
+    ref = oracle.interpolate(oracle.make_wp(count, 1, cell), xyz)
+    with engine.Engine(device=0, bin_target=1) as e:
+        h, site, st = e.interpolate(engine.make_wp(count, 1, cell), xyz, site=True)
+        assert st.evals_far > 0
+    assert np.array_equal(site, ref["site"]) and _same(h, ref["h"])
+    tile = engine.make_tile(engine.make_wp(count, 1, cell), 0, xyz.shape[0], 0, 0,
+                            extent=(*xyz[:, :2].min(0).tolist(), *xyz[:, :2].max(0).tolist()))
+    with engine.Engine(device=0) as e, e.batch([tile], bin_target=1, far_group=1) as b:     # groups in pixel rows
+        h, site = np.empty((1, count), np.float32), np.empty((1, count), np.uint32)
+        b.run(xyz, h.reshape(-1), out_site=site.reshape(-1))
+    assert np.array_equal(site, ref["site"]) and _same(h, ref["h"])
