@@ -468,10 +468,10 @@ static dnni_status compat_run(dnni_ctx* c, const dnni_compat_settings* s, const 
     G.ox = wp->origin_x;
     G.oy = wp->origin_y;
     const int64_t cells = (int64_t)wp->ncols * wp->nrows;
-    // scratch: the pixels in the context's late buffer, the tile counts (or
-    // cursors) and offsets in its bin-count buffer, the points' records (or the
-    // per-tile point lists) in its list buffer; points and outputs in its
-    // staging buffers
+    // scratch: the pixels in the context's late buffer; the gather's tile offsets,
+    // counts (or cursors) and records in its optional buffer, or else the tile
+    // counts, offsets and cursors in its bin-count buffer and the per-tile point
+    // lists in its list buffer; points and outputs in its staging buffers
     dnni_status rs;
     if ((rs = dnni_ensure(c, c->scr.late, sizeof(uint2) * (size_t)(xp * yp))) ||
         (!device && ((rs = dnni_ensure(c, c->in_xyz, sizeof(double) * 3 * (size_t)std::max<int64_t>(n, 1))) ||
@@ -487,14 +487,14 @@ static dnni_status compat_run(dnni_ctx* c, const dnni_compat_settings* s, const 
     // the offsets, then the counts, of nt tiles
     auto tile_bytes = [](long long nt, int per_tile) { return sizeof(long long) * (size_t)(nt + 1) + per_tile * sizeof(int) * (size_t)nt; };
     const long long gx = (xp + kCgTile - 1) / kCgTile, gy = (yp + kCgTile - 1) / kCgTile;
-    const size_t rec = sizeof(float4) + sizeof(uint2);
-    const bool gather = dnni_ensure(c, c->scr.cnt, tile_bytes(gx * gy, 1)) == DNNI_OK &&
-                        dnni_ensure(c, c->scr.list, rec * (size_t)std::max<int64_t>(n, 1)) == DNNI_OK;
+    const size_t recs = (size_t)std::max<int64_t>(n, 1), tiles = al256(tile_bytes(gx * gy, 1));
+    void* gather = ensure_optional(c, c->scr.part, tiles + (sizeof(float4) + sizeof(uint2)) * recs);
     if (gather) {
         const int nt = (int)(gx * gy);
-        long long* toff = (long long*)c->scr.cnt.p;
+        long long* toff = (long long*)gather;
         int* tcnt = (int*)(toff + nt + 1);
-        const CgRecs R{(float4*)c->scr.list.p, (uint2*)((float4*)c->scr.list.p + std::max<int64_t>(n, 1))};
+        float4* plane = (float4*)((unsigned char*)gather + tiles);
+        const CgRecs R{plane, (uint2*)(plane + recs)};
         const unsigned blocks = (unsigned)((n + 255) / 256);
         CK(cudaMemsetAsync(tcnt, 0, sizeof(int) * (size_t)nt, st));
         if (n > 0) {
@@ -505,7 +505,6 @@ static dnni_status compat_run(dnni_ctx* c, const dnni_compat_settings* s, const 
         if (n > 0) k_cg_fill<<<blocks, 256, 0, st>>>(G, dxyz, n, (int)gx, toff, tcnt, R);
         k_cg_sites<<<nt, 256, 0, st>>>(G, dxyz, (int)gx, (int)((span + kCgTile - 1) / kCgTile), toff, R, pixel);
     } else {
-        c->err.clear();
         const int ntx = (int)((xp + kCpTile - 1) / kCpTile), nty = (int)((yp + kCpTile - 1) / kCpTile);
         const int nt = ntx * nty;
         // tiles one square can reach
@@ -544,7 +543,7 @@ extern "C" dnni_status dnni_interpolate_compat(dnni_ctx* c, const dnni_compat_se
     if (!c || !s || !wp || !h_out || n < 0 || (n > 0 && !xyz)) return DNNI_E_INVAL;
     c->err.clear();
     DeviceGuard g(c->device);
-    return compat_run(c, s, wp, xyz, n, h_out, res_out, false, c->stream);
+    return with_room(c, [&] { return compat_run(c, s, wp, xyz, n, h_out, res_out, false, c->stream); });
 }
 
 extern "C" dnni_status dnni_interpolate_compat_device(dnni_ctx* c, const dnni_compat_settings* s,
@@ -553,5 +552,6 @@ extern "C" dnni_status dnni_interpolate_compat_device(dnni_ctx* c, const dnni_co
     if (!c || !s || !wp || !d_h || n < 0 || (n > 0 && !d_xyz)) return DNNI_E_INVAL;
     c->err.clear();
     DeviceGuard g(c->device);
-    return compat_run(c, s, wp, d_xyz, n, d_h, d_res, true, stream ? (cudaStream_t)stream : c->stream);
+    const cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
+    return with_room(c, [&] { return compat_run(c, s, wp, d_xyz, n, d_h, d_res, true, st); });
 }

@@ -60,7 +60,8 @@ struct ScratchSizes {
     size_t sorted, cnt, bsum, bmask, smask, rownear, near, pix, far, D, Dc, sc, ctr, tables;
     size_t part;                     // the points grouped by region
     size_t late() const { return al256(pix) + al256(far) + al256(D) + al256(Dc); }
-    size_t late_part() const { return std::max(late(), al256(part)); }
+    // of the grouped points' own buffer, 0 where they fit over `bytes` of late arrays
+    size_t own_part(size_t bytes) const { return bytes >= part ? 0 : al256(part); }
 };
 
 ScratchSizes scratch_sizes(const HostBatch& hb) {
@@ -72,7 +73,7 @@ ScratchSizes scratch_sizes(const HostBatch& hb) {
     z.bsum = sizeof(int) * std::max<int64_t>(hb.scan_base.back(), 1);
     z.bmask = sizeof(uint64_t) * std::max<int64_t>(hb.blk_base.back(), 1);
     z.smask = sizeof(uint64_t) * std::max<int64_t>(hb.sup_base.back(), 1);
-    z.rownear = sizeof(int) * std::max<int64_t>(hb.blk_base.back(), 1);
+    z.rownear = sizeof(int) * (hb.max_n2x > kNearMaskCols ? std::max<int64_t>(hb.blk_base.back(), 1) : 1);
     z.near = sizeof(int64_t) * std::max<int64_t>(hb.blk_base.back(), 1);
     z.pix = sizeof(int2) * std::max<int64_t>(hb.n_pix, 1);
     z.far = kFarSlotBytes * std::max<int64_t>(hb.n_far, 1);
@@ -84,11 +85,12 @@ ScratchSizes scratch_sizes(const HostBatch& hb) {
     return z;
 }
 
-// Lays out the arrays of the phases after the binning in `bytes` at base, and
-// over them, where they are large enough for it, the points grouped by region.
-void carve_late(void* base, size_t bytes, const ScratchSizes& z, DevArrays& a) {
+// Lays out the arrays of the phases after the binning in `bytes` at base; the
+// points grouped by region go over them where they are large enough, else to
+// `part` (null: no room for them).
+void carve_late(void* base, size_t bytes, const ScratchSizes& z, DevArrays& a, void* part) {
     unsigned char* p = (unsigned char*)base;
-    a.part = bytes >= z.part ? (int4*)p : nullptr;
+    a.part = (int4*)(z.own_part(bytes) ? part : base);
     a.pix = (int2*)p;
     p += al256(z.pix);
     a.far = (int4*)p;
@@ -98,23 +100,27 @@ void carve_late(void* base, size_t bytes, const ScratchSizes& z, DevArrays& a) {
     a.Dc = (int*)p;
 }
 
-// The late arrays with room for the grouped points, or, where that would pass
-// the context's budget or the device's memory, without.
-dnni_status ensure_late(dnni_ctx* c, DevBuf& b, size_t with_part, size_t plain) {
-    if (dnni_ensure(c, b, with_part) == DNNI_OK) return DNNI_OK;
-    c->err.clear();
-    return dnni_ensure(c, b, plain);
+// Room that a call can do without, or null: none where it would pass the
+// context's budget or the device's memory.
+void* ensure_optional(dnni_ctx* c, DevBuf& b, size_t bytes, bool slack = true) {
+    if (bytes == 0) return nullptr;
+    if (b.cap < bytes && (c->tight || dnni_ensure(c, b, bytes, slack))) {
+        c->err.clear();
+        return nullptr;
+    }
+    return b.p;
 }
 
-dnni_status ensure_scratch(dnni_ctx* c, Scratch& s, const ScratchSizes& z, DevArrays& a) {
-    dnni_status rs;
-    if ((rs = dnni_ensure(c, s.sorted, z.sorted)) || (rs = dnni_ensure(c, s.cnt, z.cnt)) || (rs = dnni_ensure(c, s.start, z.cnt)) ||
-        (rs = dnni_ensure(c, s.bsum, z.bsum)) || (rs = dnni_ensure(c, s.bmask, z.bmask)) ||
-        (rs = dnni_ensure(c, s.smask, z.smask)) || (rs = dnni_ensure(c, s.rownear, z.rownear)) ||
-        (rs = dnni_ensure(c, s.near, z.near)) ||
-        (rs = dnni_ensure(c, s.sc, z.sc)) || (rs = dnni_ensure(c, s.ctr, z.ctr)) ||
-        (rs = dnni_ensure(c, s.tables, z.tables)) || (rs = ensure_late(c, s.late, z.late_part(), z.late())))
-        return rs;
+// (with_part: also the room for the grouped points, which only a launch of the
+// binning needs; slack: see dnni_ensure)
+dnni_status ensure_scratch(dnni_ctx* c, Scratch& s, const ScratchSizes& z, DevArrays& a, bool with_part = true,
+                           bool slack = true) {
+    const std::pair<DevBuf*, size_t> needs[] = {
+        {&s.sorted, z.sorted}, {&s.cnt, z.cnt}, {&s.start, z.cnt}, {&s.bsum, z.bsum}, {&s.bmask, z.bmask},
+        {&s.smask, z.smask}, {&s.rownear, z.rownear}, {&s.near, z.near}, {&s.late, z.late()}, {&s.sc, z.sc},
+        {&s.ctr, z.ctr}, {&s.tables, z.tables}};
+    for (const auto& n : needs)
+        if (const dnni_status rs = dnni_ensure(c, *n.first, n.second, slack)) return rs;
     a.sorted = (int4*)s.sorted.p;
     a.cnt = (int*)s.cnt.p;
     a.start = (int*)s.start.p;
@@ -123,7 +129,7 @@ dnni_status ensure_scratch(dnni_ctx* c, Scratch& s, const ScratchSizes& z, DevAr
     a.smask = (uint64_t*)s.smask.p;
     a.rownear = (int*)s.rownear.p;
     a.near = (int64_t*)s.near.p;
-    carve_late(s.late.p, s.late.cap, z, a);
+    carve_late(s.late.p, s.late.cap, z, a, with_part ? ensure_optional(c, s.part, z.own_part(s.late.cap), slack) : nullptr);
     a.sc = (Scalars*)s.sc.p;
     a.ctr = (BatchCounters*)s.ctr.p;
     a.tables = (unsigned char*)s.tables.p;
@@ -132,8 +138,51 @@ dnni_status ensure_scratch(dnni_ctx* c, Scratch& s, const ScratchSizes& z, DevAr
 
 void release_scratch(dnni_ctx* c, Scratch& s) {
     DevBuf* bufs[] = {&s.sorted, &s.list, &s.cnt, &s.start, &s.bsum, &s.bmask, &s.smask, &s.rownear,
-                      &s.near, &s.late, &s.sc, &s.ctr, &s.tables};
+                      &s.near, &s.late, &s.sc, &s.ctr, &s.tables, &s.part};
     for (DevBuf* b : bufs) dnni_release(*b, c);
+}
+
+// Ends the captured graph of a batch whose scratch moves or goes.
+void drop_graph(dnni_batch* b) {
+    if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
+    if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
+}
+
+// After a refused allocation: waits for all queued work and gives back what
+// nothing depends on between calls, the context's own buffers and the batches'
+// staging and room for grouped points; from then on buffers take exactly what
+// they need, until dnni_clear.  False when that was done before.
+bool give_back(dnni_ctx* c) {
+    if (c->tight) return false;
+    c->tight = true;
+    cudaDeviceSynchronize();
+    dnni_free_all(c);
+    for (dnni_batch* b : c->batches) {
+        DevBuf* staging[] = {&b->in_xyz, &b->in_gid, &b->out_h, &b->out_site};
+        for (DevBuf* s : staging) dnni_release(*s, c);
+        if (!b->scr.part.p) continue;
+        // (grouped points that lie over the late arrays stay there)
+        const auto drop = [&](DevArrays& a) {
+            const size_t off = (size_t)((unsigned char*)a.part - (unsigned char*)b->scr.part.p);
+            if (a.part && off < b->scr.part.cap) a.part = nullptr;
+        };
+        drop(b->arr);
+        for (BatchSlice& sl : b->slices) drop(sl.arr);
+        drop_graph(b);
+        dnni_release(b->scr.part, c);
+    }
+    return true;
+}
+
+// An entry point's work; where an allocation is refused, once more with all
+// that can be given back (the first try has only queued work and filled buffers
+// that the second one fills again).
+template <typename F>
+dnni_status with_room(dnni_ctx* c, F call) {
+    const dnni_status rs = call();
+    if (rs != DNNI_E_NOMEM || !give_back(c)) return rs;
+    c->err.clear();
+    return call();
 }
 
 // A kernel launch; chain: as a link of a chain whose kernels start with chained(),
@@ -350,9 +399,9 @@ dnni_status stage_tables(dnni_ctx* c, const HostBatch& hb, unsigned char* d_tabl
 
 }  // namespace
 
-dnni_status dnni_ensure(dnni_ctx* c, DevBuf& b, size_t bytes) {
+dnni_status dnni_ensure(dnni_ctx* c, DevBuf& b, size_t bytes, bool slack) {
     if (bytes <= b.cap) return DNNI_OK;
-    size_t want = bytes + bytes / 4;
+    size_t want = c->tight || !slack ? bytes : bytes + bytes / 4;
     want = (want + 255) & ~(size_t)255;
     if (c->s.mem_budget) {
         if (c->held - b.cap + want > c->s.mem_budget) want = (bytes + 255) & ~(size_t)255;
@@ -406,7 +455,7 @@ static dnni_status run_device(dnni_ctx* c, const dnni_workpackage* wp, const int
     set_chunk(hb, n);
     batch_add(hb, t, 0, 0, d_site ? 0 : -1);
     DevArrays a;
-    if ((rs = ensure_scratch(c, c->scr, scratch_sizes(hb), a))) return rs;
+    if ((rs = ensure_scratch(c, c->scr, scratch_sizes(hb), a, false))) return rs;
     BatchTables bt = device_tables(a.tables, hb);
     if (timing) CK(cudaEventRecord(c->ev[0], st));
     launch_one_tables(hb, a, true, 0, st);
@@ -609,7 +658,7 @@ dnni_status dnni_setup_run(dnni_ctx* c, const dnni_workpackage* wp, int64_t max_
     HostBatch hb;
     batch_add(hb, t, 0, 0, 0);
     DevArrays a;
-    return ensure_scratch(c, c->scr, scratch_sizes(hb), a);
+    return with_room(c, [&] { return ensure_scratch(c, c->scr, scratch_sizes(hb), a); });
 }
 
 dnni_status dnni_interpolate_segment_device(dnni_ctx* c, const dnni_workpackage* wp, const int32_t* d_xyz,
@@ -620,13 +669,11 @@ dnni_status dnni_interpolate_segment_device(dnni_ctx* c, const dnni_workpackage*
     DeviceGuard g(c->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
     if (stats) memset(stats, 0, sizeof(*stats));
-    return run_device(c, wp, d_xyz, d_gid, n, d_h, d_site, st, stats);
+    return with_room(c, [&] { return run_device(c, wp, d_xyz, d_gid, n, d_h, d_site, st, stats); });
 }
 
-dnni_status dnni_interpolate_segment(dnni_ctx* c, const dnni_workpackage* wp, const int32_t* xyz, const uint32_t* gid,
-                                     int64_t n, float* out_h, uint32_t* out_site, dnni_stats* stats) {
-    if (!c) return DNNI_E_INVAL;
-    c->err.clear();
+static dnni_status run_host(dnni_ctx* c, const dnni_workpackage* wp, const int32_t* xyz, const uint32_t* gid, int64_t n,
+                            float* out_h, uint32_t* out_site, dnni_stats* stats) {
     if (!out_h) return set_err(c, DNNI_E_INVAL, "output grid pointer is NULL");
     if (n > 0 && !xyz) return set_err(c, DNNI_E_INVAL, "point pointer is NULL");
     DeviceGuard g(c->device);
@@ -660,11 +707,19 @@ dnni_status dnni_interpolate_segment(dnni_ctx* c, const dnni_workpackage* wp, co
     return DNNI_OK;
 }
 
+dnni_status dnni_interpolate_segment(dnni_ctx* c, const dnni_workpackage* wp, const int32_t* xyz, const uint32_t* gid,
+                                     int64_t n, float* out_h, uint32_t* out_site, dnni_stats* stats) {
+    if (!c) return DNNI_E_INVAL;
+    c->err.clear();
+    return with_room(c, [&] { return run_host(c, wp, xyz, gid, n, out_h, out_site, stats); });
+}
+
 dnni_status dnni_clear(dnni_ctx* c) {
     if (!c) return DNNI_E_INVAL;
     DeviceGuard g(c->device);
     cudaStreamSynchronize(c->stream);
     dnni_free_all(c);
+    c->tight = false;
     return DNNI_OK;
 }
 
@@ -735,7 +790,8 @@ dnni_status dnni_batch_create(dnni_ctx* c, const dnni_tile* tiles, int32_t ntile
             return rs;
         }
     }
-    dnni_status rs = ensure_scratch(c, b->scr, scratch_sizes(b->hb), b->arr);
+    // (a batch's scratch never grows)
+    dnni_status rs = with_room(c, [&] { return ensure_scratch(c, b->scr, scratch_sizes(b->hb), b->arr, true, false); });
     if (!rs) {
         b->bt = device_tables(b->arr.tables, b->hb);
         rs = stage_tables(c, b->hb, b->arr.tables, c->stream);
@@ -747,6 +803,7 @@ dnni_status dnni_batch_create(dnni_ctx* c, const dnni_tile* tiles, int32_t ntile
         return rs;
     }
     b->h_sc.resize(ntiles);
+    c->batches.push_back(b);
     *out = b;
     return DNNI_OK;
 }
@@ -764,8 +821,7 @@ dnni_status dnni_batch_run_device(dnni_batch* b, const int32_t* d_xyz, const uin
     if (b->use_graph) {
         const void* key[4] = {d_xyz, d_gid, d_h, d_site};
         if (!b->exec || memcmp(key, b->graph_key, sizeof(key)) != 0) {
-            if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
-            if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
+            drop_graph(b);
             cudaStream_t cap;
             CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
             cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
@@ -837,6 +893,7 @@ static dnni_status plan_slices(dnni_batch* b) {
     const int S = b->hb.n_rows >= (4 << 20) ? std::min(n, kSlices) : 1;
     const bool ramp = S == kSlices;
     b->sliced = S > 1;
+    for (BatchSlice& sl : b->slices) dnni_release(sl.tables, c);     // of a try that was refused
     b->slices.clear();
     if (!b->sliced) {
         b->slices_planned = true;
@@ -886,7 +943,7 @@ static dnni_status plan_slices(dnni_batch* b) {
                 sl.site1 = std::max<int64_t>(sl.site1, t.site_off + (int64_t)t.rw * t.rh);
             }
         if (sl.site0 == INT64_MAX) sl.site0 = sl.site1 = 0;
-        if ((rs = dnni_ensure(c, sl.tables, TableLayout((int)part.size()).total))) return rs;
+        if ((rs = dnni_ensure(c, sl.tables, TableLayout((int)part.size()).total, false))) return rs;
         sl.bt = device_tables((const unsigned char*)sl.tables.p, sl.hb);
         if ((rs = stage_tables(c, sl.hb, (unsigned char*)sl.tables.p, c->stream))) return rs;
         b->slices.push_back(std::move(sl));
@@ -896,33 +953,26 @@ static dnni_status plan_slices(dnni_batch* b) {
     // consecutive slices can compute on two streams at once
     const int ns = (int)b->slices.size();
     dnni_status rs;
-    if ((rs = dnni_ensure(c, b->slice_ctrs, sizeof(BatchCounters) * (size_t)ns))) return rs;
-    ScratchSizes full_z = scratch_sizes(b->hb);
-    size_t with_part = 0, plain = 0;
-    for (const BatchSlice& sl : b->slices) {
-        const ScratchSizes z = scratch_sizes(sl.hb);
-        with_part += z.late_part();
-        plain += z.late();
-    }
-    if ((rs = ensure_late(c, b->scr.late, std::max(with_part, full_z.late_part()), std::max(plain, full_z.late())))) return rs;
-    // the full batch's view of its scratch (the graph captured for it is
-    // rebuilt if the arrays moved)
-    DevArrays full;
-    if ((rs = ensure_scratch(c, b->scr, full_z, full))) return rs;
-    full.tables = b->arr.tables;
-    if (full.sorted != b->arr.sorted || full.pix != b->arr.pix) {
-        if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
-        if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
-    }
-    b->arr = full;
+    if ((rs = dnni_ensure(c, b->slice_ctrs, sizeof(BatchCounters) * (size_t)ns, false))) return rs;
+    // a slice's grouped points lie over its worklist where they fit, else in the
+    // batch's `part`, which the whole batch's share with them (a batch runs as
+    // slices or whole, one at a time)
+    const ScratchSizes z = scratch_sizes(b->hb);
+    const auto own_part = [](const HostBatch& h) { return kFarSlotBytes * h.n_far >= (int64_t)sizeof(int4) * h.n_pts ? 0 : h.n_pts; };
+    int64_t part_pts = 0;
+    for (const BatchSlice& sl : b->slices) part_pts += own_part(sl.hb);
+    const size_t whole = z.own_part(b->scr.late.cap);
+    const void* was = b->scr.part.p;
+    int4* part = (int4*)ensure_optional(c, b->scr.part, std::max(sizeof(int4) * (size_t)part_pts, whole), false);
+    // (a refused growth leaves the buffer as it was, or none)
+    if (b->scr.part.p != was) drop_graph(b);
+    carve_late(b->scr.late.p, b->scr.late.cap, z, b->arr, b->scr.part.cap >= whole ? b->scr.part.p : nullptr);
     {
-        const bool parts = b->scr.late.cap >= with_part;
-        unsigned char* late = (unsigned char*)b->scr.late.p;
-        int64_t pts = 0, bins = 0, scan = 0, blk = 0, sup = 0, tiles = 0;
+        int64_t pts = 0, bins = 0, scan = 0, blk = 0, sup = 0, pix = 0, far = 0, cells = 0, tiles = 0;
         for (int s = 0; s < ns; ++s) {
             BatchSlice& sl = b->slices[s];
             const HostBatch& h = sl.hb;
-            DevArrays v = full;
+            DevArrays v = b->arr;
             v.sorted += pts;
             v.cnt += bins;
             v.start += bins;
@@ -931,10 +981,12 @@ static dnni_status plan_slices(dnni_batch* b) {
             v.smask += sup;
             v.rownear += blk;
             v.near += blk;
-            const ScratchSizes z = scratch_sizes(h);
-            const size_t bytes = parts ? z.late_part() : z.late();
-            carve_late(late, bytes, z, v);
-            late += bytes;
+            v.pix += pix;
+            v.far += far;
+            v.D += cells;
+            v.Dc += cells;
+            v.part = own_part(h) ? part : v.far;
+            if (part) part += own_part(h);
             v.sc += tiles;
             v.ctr = (BatchCounters*)b->slice_ctrs.p + s;
             v.tables = (unsigned char*)sl.tables.p;
@@ -944,6 +996,9 @@ static dnni_status plan_slices(dnni_batch* b) {
             scan += h.scan_base.back();
             blk += h.blk_base.back();
             sup += h.sup_base.back();
+            pix += h.n_pix;
+            far += h.n_far;
+            cells += h.n_cells;
             tiles += (int64_t)h.tiles.size();
         }
     }
@@ -965,12 +1020,9 @@ static dnni_status plan_slices(dnni_batch* b) {
     return DNNI_OK;
 }
 
-dnni_status dnni_batch_run(dnni_batch* b, const int32_t* xyz, const uint32_t* gid, int64_t n_rows, float* out_h,
-                           uint32_t* out_site, dnni_stats* stats) {
-    if (!b) return DNNI_E_INVAL;
+static dnni_status batch_run_host(dnni_batch* b, const int32_t* xyz, const uint32_t* gid, int64_t n_rows, float* out_h,
+                                  uint32_t* out_site, dnni_stats* stats) {
     dnni_ctx* c = b->ctx;
-    c->err.clear();
-    DeviceGuard g(c->device);
     if (n_rows < b->hb.n_rows) return set_err(c, DNNI_E_INVAL, "fewer point rows than the tiles reference");
     if (!out_h || (n_rows > 0 && !xyz)) return set_err(c, DNNI_E_INVAL, "NULL buffer");
     cudaStream_t st = c->stream;
@@ -1060,14 +1112,23 @@ dnni_status dnni_batch_run(dnni_batch* b, const int32_t* xyz, const uint32_t* gi
     return DNNI_OK;
 }
 
+dnni_status dnni_batch_run(dnni_batch* b, const int32_t* xyz, const uint32_t* gid, int64_t n_rows, float* out_h,
+                           uint32_t* out_site, dnni_stats* stats) {
+    if (!b) return DNNI_E_INVAL;
+    dnni_ctx* c = b->ctx;
+    c->err.clear();
+    DeviceGuard g(c->device);
+    return with_room(c, [&] { return batch_run_host(b, xyz, gid, n_rows, out_h, out_site, stats); });
+}
+
 dnni_status dnni_batch_destroy(dnni_batch* b) {
     if (!b) return DNNI_E_INVAL;
     dnni_ctx* c = b->ctx;
     {
         DeviceGuard g(c->device);
         cudaDeviceSynchronize();
-        if (b->exec) cudaGraphExecDestroy(b->exec);
-        if (b->graph) cudaGraphDestroy(b->graph);
+        c->batches.erase(std::remove(c->batches.begin(), c->batches.end(), b), c->batches.end());
+        drop_graph(b);
         for (BatchSlice& sl : b->slices) dnni_release(sl.tables, c);
         for (cudaEvent_t e : b->ev_in)
             if (e) cudaEventDestroy(e);
@@ -1090,12 +1151,9 @@ dnni_status dnni_batch_destroy(dnni_batch* b) {
 
 // ---- autotuner -------------------------------------------------------------
 
-dnni_status dnni_batch_autotune(dnni_ctx* c, const dnni_tile* tiles, int32_t ntiles, const int32_t* d_xyz,
-                                const uint32_t* d_gid, int32_t sample_tiles, dnni_batch_options* options,
-                                dnni_tune_report* report) {
-    if (!c || !tiles || ntiles <= 0 || !options) return DNNI_E_INVAL;
-    c->err.clear();
-    DeviceGuard g(c->device);
+static dnni_status autotune(dnni_ctx* c, const dnni_tile* tiles, int32_t ntiles, const int32_t* d_xyz,
+                            const uint32_t* d_gid, int32_t sample_tiles, dnni_batch_options* options,
+                            dnni_tune_report* report) {
     const dnni_batch_options given = *options;
     // sample: tiles evenly spaced in cost order, so that it spans the sizes
     std::vector<int> idx(ntiles);
@@ -1215,6 +1273,15 @@ dnni_status dnni_batch_autotune(dnni_ctx* c, const dnni_tile* tiles, int32_t nti
     return DNNI_OK;
 }
 
+dnni_status dnni_batch_autotune(dnni_ctx* c, const dnni_tile* tiles, int32_t ntiles, const int32_t* d_xyz,
+                                const uint32_t* d_gid, int32_t sample_tiles, dnni_batch_options* options,
+                                dnni_tune_report* report) {
+    if (!c || !tiles || ntiles <= 0 || !options) return DNNI_E_INVAL;
+    c->err.clear();
+    DeviceGuard g(c->device);
+    return with_room(c, [&] { return autotune(c, tiles, ntiles, d_xyz, d_gid, sample_tiles, options, report); });
+}
+
 }  // extern "C"
 
 void SegBufs::release(dnni_ctx* c) {
@@ -1291,8 +1358,8 @@ bool carve_noalloc(unsigned char* base, const ScratchSizes& z, bool with_part, D
     a.tables = take(z.tables);
     a.sc = (Scalars*)take(z.sc);
     a.ctr = (BatchCounters*)take(z.ctr);
-    const size_t late = with_part ? z.late_part() : z.late();
-    carve_late(take(late), late, z, a);
+    const size_t late = with_part ? std::max(z.late(), al256(z.part)) : z.late();
+    carve_late(take(late), late, z, a, nullptr);
     a.sorted = (int4*)take(z.sorted);
     a.cnt = (int*)take(z.cnt);
     a.start = (int*)take(z.cnt);

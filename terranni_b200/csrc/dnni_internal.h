@@ -23,15 +23,17 @@ struct DevBuf {
 // `list` serves only the reference-default mode (its per-tile point lists);
 // `late` holds what the phases after the binning use (pixel records,
 // worklist, span words and counts: carve_late), and before that the points
-// grouped by region.
+// grouped by region, where it is large enough for them; else they lie in
+// `part`, which is optional: it is taken after all the others, and given back
+// when an allocation is refused (give_back).
 struct Scratch {
-    DevBuf sorted, list, cnt, start, bsum, bmask, smask, rownear, near, late, sc, ctr, tables;
+    DevBuf sorted, list, cnt, start, bsum, bmask, smask, rownear, near, late, sc, ctr, tables, part;
 };
 
 // Raw device pointers of a scratch set for one launch sequence.
 struct DevArrays {
     int4* sorted = nullptr;
-    int4* part = nullptr;            // points grouped by region, over pix .. Dc; null: no room, bin directly
+    int4* part = nullptr;            // points grouped by region; null: no room, bin directly
     int* cnt = nullptr;
     int* start = nullptr;
     int* bsum = nullptr;
@@ -49,6 +51,7 @@ struct DevArrays {
 };
 
 struct dnni_ctx;
+struct dnni_batch;
 
 // Device buffers of the segment driver and the server's resident cloud.
 struct SegBufs {
@@ -79,6 +82,10 @@ struct dnni_ctx {
     cudaEvent_t ev[6] = {};
     std::string err;
     size_t held = 0;
+    // an allocation was refused since the last dnni_clear: buffers take exactly
+    // what they need, and none of them is optional (give_back)
+    bool tight = false;
+    std::vector<dnni_batch*> batches;
     double acc_ms[4] = {};
     int64_t calls = 0;
 };
@@ -118,6 +125,7 @@ struct dnni_batch {
     std::vector<dnni::Scalars> h_sc;
 };
 
-dnni_status dnni_ensure(dnni_ctx* c, DevBuf& b, size_t bytes);
+// (slack: a quarter more, for buffers that the next call may want a little larger)
+dnni_status dnni_ensure(dnni_ctx* c, DevBuf& b, size_t bytes, bool slack = true);
 void dnni_release(DevBuf& b, dnni_ctx* c);
 void dnni_free_all(dnni_ctx* c);

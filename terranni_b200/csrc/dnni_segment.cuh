@@ -801,7 +801,7 @@ extern "C" dnni_status dnni_segment_run(dnni_ctx* c, const dnni_segment* sp, con
         return set_err(c, DNNI_E_INVAL, "part must lie in [0, parts)");
     // buffers stay with the context (grow-only) for the next call; dnni_clear
     // and dnni_destroy free them
-    const dnni_status rs = segment_run(c, s, h_xyz, n, h_out, h_site, stats, c->seg, c->seg_scr);
+    const dnni_status rs = with_room(c, [&] { return segment_run(c, s, h_xyz, n, h_out, h_site, stats, c->seg, c->seg_scr); });
     if (c->stream) cudaStreamSynchronize(c->stream);
     return rs;
 }

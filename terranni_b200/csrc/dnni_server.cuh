@@ -258,7 +258,7 @@ dnni_status srv_launch(dnni_server* s, SrvSlot& sl, std::vector<SrvItem>& items,
     a.sc = (Scalars*)take(z.sc);
     a.ctr = (BatchCounters*)take(z.ctr);
     // (no room beyond the admitted footprint: denser batches bin directly)
-    carve_late(take(z.late()), z.late(), z, a);
+    carve_late(take(z.late()), z.late(), z, a, nullptr);
     a.sorted = (int4*)take(z.sorted);
     a.cnt = (int*)take(z.cnt);
     a.start = (int*)take(z.cnt);
@@ -557,26 +557,8 @@ void srv_loop(dnni_server* s) {
 
 }  // namespace
 
-extern "C" {
-
-dnni_status dnni_server_create(dnni_ctx* c, const int32_t* h_xyz, int64_t n, const dnni_server_options* opt,
-                               dnni_server** out) {
-    if (!c || !out || n < 0 || (n > 0 && !h_xyz)) return DNNI_E_INVAL;
-    *out = nullptr;
-    c->err.clear();
-    DeviceGuard g(c->device);
-    if ((uint64_t)n >= 0xFFFFFFFFull) return set_err(c, DNNI_E_INVAL, "more points than 32-bit site ids can name");
-    dnni_server_options o{};
-    if (opt) o = *opt;
-    if (!o.bucket) o.bucket = 25600;
-    if (!o.slots) o.slots = 2;
-    if (!o.max_batch) o.max_batch = 64;
-    if (!o.slot_bytes) o.slot_bytes = 16ull << 30;
-    if (!o.small_radius) o.small_radius = c->s.small_radius;
-    if (!o.bin_target) o.bin_target = c->s.bin_target;
-    if (o.bucket < 1 || o.fine < 0 || o.slots < 1 || o.slots > 8 || o.max_batch < 1 || o.max_batch > 4096 ||
-        o.small_radius < 1 || o.small_radius > kMaxSmallRadius || o.bin_target < 0)
-        return set_err(c, DNNI_E_INVAL, "bad server options");
+static dnni_status server_create(dnni_ctx* c, const int32_t* h_xyz, int64_t n, const dnni_server_options& o,
+                                 dnni_server** out) {
     const double t0 = now_s();
     dnni_server* s = new dnni_server();
     s->ctx = c;
@@ -654,6 +636,29 @@ dnni_status dnni_server_create(dnni_ctx* c, const int32_t* h_xyz, int64_t n, con
     s->th = std::thread(srv_loop, s);
     *out = s;
     return DNNI_OK;
+}
+
+extern "C" {
+
+dnni_status dnni_server_create(dnni_ctx* c, const int32_t* h_xyz, int64_t n, const dnni_server_options* opt,
+                               dnni_server** out) {
+    if (!c || !out || n < 0 || (n > 0 && !h_xyz)) return DNNI_E_INVAL;
+    *out = nullptr;
+    c->err.clear();
+    DeviceGuard g(c->device);
+    if ((uint64_t)n >= 0xFFFFFFFFull) return set_err(c, DNNI_E_INVAL, "more points than 32-bit site ids can name");
+    dnni_server_options o{};
+    if (opt) o = *opt;
+    if (!o.bucket) o.bucket = 25600;
+    if (!o.slots) o.slots = 2;
+    if (!o.max_batch) o.max_batch = 64;
+    if (!o.slot_bytes) o.slot_bytes = 16ull << 30;
+    if (!o.small_radius) o.small_radius = c->s.small_radius;
+    if (!o.bin_target) o.bin_target = c->s.bin_target;
+    if (o.bucket < 1 || o.fine < 0 || o.slots < 1 || o.slots > 8 || o.max_batch < 1 || o.max_batch > 4096 ||
+        o.small_radius < 1 || o.small_radius > kMaxSmallRadius || o.bin_target < 0)
+        return set_err(c, DNNI_E_INVAL, "bad server options");
+    return with_room(c, [&] { return server_create(c, h_xyz, n, o, out); });
 }
 
 dnni_status dnni_server_submit(dnni_server* s, const dnni_request* r, uint64_t* ticket) {

@@ -596,7 +596,7 @@ extern "C" dnni_status dnni_interpolate_spacetime(dnni_ctx* c, const dnni_workpa
     if (!wp || !o || !h_out || n < 0 || (n > 0 && (!xyz || !tt)))
         return set_err(c, DNNI_E_INVAL, "NULL argument or negative point count");
     DeviceGuard g(c->device);
-    return spacetime_run(c, wp, o, xyz, tt, n, h_out, false, c->stream, stats);
+    return with_room(c, [&] { return spacetime_run(c, wp, o, xyz, tt, n, h_out, false, c->stream, stats); });
 }
 
 extern "C" dnni_status dnni_interpolate_spacetime_device(dnni_ctx* c, const dnni_workpackage* wp,
@@ -608,5 +608,6 @@ extern "C" dnni_status dnni_interpolate_spacetime_device(dnni_ctx* c, const dnni
     if (!wp || !o || !d_h || n < 0 || (n > 0 && (!d_xyz || !d_t)))
         return set_err(c, DNNI_E_INVAL, "NULL argument or negative point count");
     DeviceGuard g(c->device);
-    return spacetime_run(c, wp, o, d_xyz, d_t, n, d_h, true, stream ? (cudaStream_t)stream : c->stream, stats);
+    const cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
+    return with_room(c, [&] { return spacetime_run(c, wp, o, d_xyz, d_t, n, d_h, true, st, stats); });
 }

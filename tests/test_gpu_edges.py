@@ -104,3 +104,79 @@ def test_far_pass_on_wide_cells(oracle, cell, count):
         h, site = np.empty((1, count), np.float32), np.empty((1, count), np.uint32)
         b.run(xyz, h.reshape(-1), out_site=site.reshape(-1))
     assert np.array_equal(site, ref["site"]) and _same(h, ref["h"])
+
+
+def _budget_calls():
+    """Calls whose grouped points (or gathered records) need more room than the
+    rest of their scratch: name -> (call on an engine -> heights)."""
+    from terranni_b200 import engine
+    rng = np.random.default_rng(12)
+    xyz = _points(rng, 60000, 6400, 6400)
+    wp = engine.make_wp(64, 64, 100)
+    times = rng.integers(-3, 4, 60000).astype(np.int32)
+    big = np.concatenate([_points(rng, 300_000, 9600, 9600) + np.array([k * 20000, 0, 0], np.int32) for k in range(15)])
+    world = np.stack([rng.uniform(0, 80, 30000), rng.uniform(0, 60, 30000), rng.uniform(0, 30, 30000)], 1)
+    cset = engine.CompatSettings(scale=2, cell_size=2.0, site_radius=5.0, query_radius=4.99, point_min=0, multiplier=10000,
+                                 total_ncols=40, total_nrows=30)
+
+    def batch(e, tiles, rows, cells, graph):
+        out = np.empty(cells, np.float32)
+        with e.batch(tiles, use_graph=graph) as b:
+            for _ in range(2):
+                out[:] = 5.0
+                b.run(rows, out)
+        return out
+
+    def two_kinds(e):
+        # a batch keeps its scratch while other calls come and go beside it
+        out = np.empty(64 * 64, np.float32)
+        with e.batch([engine.make_tile(wp, 0, 60000, 0)], use_graph=True) as b:
+            b.run(xyz, out)
+            h = e.interpolate(wp, xyz, site=True)[0]
+            assert _same(h.reshape(-1), out)
+            out[:] = 5.0
+            b.run(xyz, out)
+        return out
+
+    return {
+        "single": lambda e: e.interpolate(wp, xyz, site=True)[0],
+        "batch": lambda e: batch(e, [engine.make_tile(wp, 0, 60000, 0)], xyz, 64 * 64, False),
+        "batch_graph": lambda e: batch(e, [engine.make_tile(wp, 0, 60000, 0)], xyz, 64 * 64, True),
+        "batch_slices": lambda e: batch(e, [engine.make_tile(engine.make_wp(96, 96, 100, k * 20000, 0), k * 300_000, 300_000,
+                                                             k * 9216) for k in range(15)], big, 15 * 9216, False),
+        "two_kinds": two_kinds,
+        "segment": lambda e: e.segment_run(xyz, 64, 64, 100, tile=32, halo=6, tiles_per_batch=1)[0],
+        "spacetime": lambda e: e.interpolate_spacetime(wp, xyz, times, 0, 1, 100)[0],
+        "compat": lambda e: e.interpolate_compat(cset, engine.CompatWP(nrows=30, ncols=40), world)[0],
+    }
+
+
+# the room that only speeds a call up never costs another allocation its place:
+# every budget above the smallest accepted one is accepted, with the same bits
+@pytest.mark.parametrize("kind", ["single", "batch", "batch_graph", "batch_slices", "two_kinds", "segment", "spacetime",
+                                  "compat"])
+def test_no_budget_is_refused_above_an_accepted_one(eng, kind):
+    from terranni_b200 import engine
+    call = _budget_calls()[kind]
+    want = call(eng).copy()
+
+    def accepted(budget):
+        with engine.Engine(device=0, mem_budget=budget) as e:
+            try:
+                got = call(e)
+            except engine.DnniError as err:
+                assert err.status == 2
+                return False
+        assert _same(got, want)
+        return True
+
+    lo, hi = 1, 1 << 30
+    assert accepted(hi) and not accepted(lo)
+    while hi - lo > 256:
+        mid = (lo + hi) // 2
+        if accepted(mid):
+            hi = mid
+        else:
+            lo = mid
+    for k in range(1, 49):
+        assert accepted(int(hi * 1.025 ** k))
