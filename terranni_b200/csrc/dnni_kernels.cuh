@@ -1191,31 +1191,47 @@ __global__ void __launch_bounds__(256, 3) k_near_dense(BatchTables bt, const int
 // far pass: the exact nearest site of the pixels that the bin rings leave
 // ---------------------------------------------------------------------------
 
-// Number types of the search: 32-bit where every distance it can meet fits
-// (see far_fits32), 64-bit otherwise.
+// Number types of the search: D holds a site's squared distance, T the squared
+// gaps and bounds that the tests compare.  32-bit where every distance it can
+// meet fits (far_fits32); otherwise 64-bit distances, and floats in the tests: a
+// gap is exact, its square rounded down, a bound rounded up.  Coordinates in the
+// tests are unsigned, relative to the bin grid's origin (below 2^32).
 template <bool k32> struct FarNum;
 template <> struct FarNum<true> {
-    using I = int;
     using D = unsigned;
-    static __device__ __forceinline__ D warp_min(D v) { return __reduce_min_sync(0xffffffffu, v); }
-    static __device__ __forceinline__ D warp_max(D v) { return __reduce_max_sync(0xffffffffu, v); }
+    using T = unsigned;
+    static __device__ __forceinline__ T none() { return ~0u; }
+    static __device__ __forceinline__ T bound(D d2) { return d2; }
+    static __device__ __forceinline__ unsigned bits(T v) { return v; }
+    static __device__ __forceinline__ T value(unsigned b) { return b; }
+    // gap of [a0, a1] and [b0, b1] (within 2^31 of each other), 0 when they meet
+    static __device__ __forceinline__ unsigned gap(unsigned a0, unsigned a1, unsigned b0, unsigned b1) {
+        return (unsigned)max(max((int)(b0 - a1), (int)(a0 - b1)), 0);
+    }
+    // (46340^2 exceeds every bound here)
+    static __device__ __forceinline__ T square(unsigned dx, unsigned dy) {
+        dx = min(dx, 46340u);
+        dy = min(dy, 46340u);
+        return dx * dx + dy * dy;
+    }
     // at least floor(sqrt(v)) + 1: below 2^31 the estimate is within 0.05
-    static __device__ __forceinline__ I reach(D v) { return (I)sqrt_est((float)v) + 2; }
+    static __device__ __forceinline__ long long reach(T v) { return (long long)sqrt_est((float)v) + 2; }
 };
 template <> struct FarNum<false> {
-    using I = long long;
     using D = unsigned long long;
-    static __device__ __forceinline__ D warp_min(D v) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) { const D w = __shfl_xor_sync(0xffffffffu, v, o); v = w < v ? w : v; }
-        return v;
+    using T = float;
+    static __device__ __forceinline__ T none() { return __uint_as_float(0x7F800000u); }
+    static __device__ __forceinline__ T bound(D d2) { return __ull2float_ru(d2); }
+    static __device__ __forceinline__ unsigned bits(T v) { return __float_as_uint(v); }   // ordered as the values, none negative
+    static __device__ __forceinline__ T value(unsigned b) { return __uint_as_float(b); }
+    static __device__ __forceinline__ unsigned gap(unsigned a0, unsigned a1, unsigned b0, unsigned b1) {
+        return (max(b0, a1) - a1) + (a0 - min(b1, a0));      // one of them is zero
     }
-    static __device__ __forceinline__ D warp_max(D v) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) { const D w = __shfl_xor_sync(0xffffffffu, v, o); v = w > v ? w : v; }
-        return v;
+    static __device__ __forceinline__ T square(unsigned dx, unsigned dy) {
+        const float x = __uint2float_rd(dx), y = __uint2float_rd(dy);
+        return __fmaf_rd(x, x, __fmul_rd(y, y));
     }
-    static __device__ __forceinline__ I reach(D v) { return reach_of((long long)v); }
+    static __device__ __forceinline__ long long reach(T v) { return reach_of((long long)v) + 1; }
 };
 
 // One lane's pixel and best site so far.
@@ -1232,8 +1248,8 @@ struct FarLane {
             const int dx = p.x - px, dy = p.y - py;
             d = (unsigned)(dx * dx) + (unsigned)(dy * dy);
         } else {
-            const long long dx = (long long)p.x - px, dy = (long long)p.y - py;
-            d = (unsigned long long)(dx * dx) + (unsigned long long)(dy * dy);
+            const int dx = p.x - px, dy = p.y - py;          // |p.x|, |px| < 2^30
+            d = (unsigned long long)((long long)dx * dx) + (unsigned long long)((long long)dy * dy);
         }
         if (__builtin_expect(d <= d2, 0)) {
             const uint32_t g = (uint32_t)p.w;
@@ -1247,18 +1263,15 @@ struct FarLane {
     }
 };
 
-// Gap between the intervals [a0, a1] and [b0, b1] (0 when they meet).
-template <typename I>
-__device__ __forceinline__ I interval_gap(I a0, I a1, I b0, I b1) {
-    const I l = b0 - a1, r = a0 - b1, m = l > r ? l : r;
-    return m > 0 ? m : 0;
-}
-
 // A warp leaves a group to the heavy pass once it has searched this many
 // blocks for it and more remain: fewer while the groups leave warps without
 // work (below four to a warp), and none at all below one group per CTA of the
-// heavy pass, which then takes every group.
-constexpr int kFarDefer = 32, kFarDeferFew = 8;
+// heavy pass, which then takes every group.  Beyond 32-bit distances, where a
+// CTA's warps share a group less well, a warp goes on as long as kFarKeep groups
+// per warp wait to be handed out (2048^2 cells, 0.5 and 8 points per cell around a
+// lake 1843 cells wide: far passes 9.6 -> 8.6 and 122 -> 84 ms; going on always
+// left long groups to the end, and two smaller lakes took 3.8 in place of 2.2 ms).
+constexpr int kFarDefer = 32, kFarDeferFew = 8, kFarKeep = 2;
 constexpr int kFarCtasPerSm = 4;
 __device__ __forceinline__ bool far_all_heavy(int groups) { return groups <= (int)gridDim.x; }
 constexpr int kFarPixels = 32;   // a group spans at most this many cells in x and y
@@ -1283,8 +1296,8 @@ __device__ __forceinline__ bool far_fits32(long long reach, int bs, int cs) {
 
 // Warp-cooperative exact search for the 32 pixels of one worklist group; every
 // lane holds a real site on entry (idle lanes repeat another lane's pixel).
-// The group's superblocks within the largest bound are walked from the
-// group's own; a superblock's blocks, two to a lane, are tested against the
+// The group's own superblock comes first, then those within the largest bound,
+// one tested per lane; a superblock's blocks, two to a lane, are tested against the
 // group's box at once and searched nearest first, so that the bounds tighten
 // early; in a block, the bins within the largest bound form one run per row
 // (tested the same way), and the runs that some lane's disc touches are ranges
@@ -1296,30 +1309,32 @@ __device__ __forceinline__ bool far_fits32(long long reach, int bs, int cs) {
 //
 // kCta: the eight warps of a CTA search one group; warp w takes the blocks of
 // one residue class, and the lanes' bounds meet in s_bound.  Otherwise the
-// search ends with false after `most` blocks if more remain.
+// search ends with false after `most` blocks if more remain (with `next`, the
+// number of groups handed out: only once that has reached `keep`).
 template <bool k32, bool kCta>
 __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restrict__ pts, const int* __restrict__ start,
                                            const uint64_t* __restrict__ bmask, const uint64_t* __restrict__ smask,
                                            FarLane<k32>& b, bool act, unsigned& nev, FarBuf* buf, int far_blocks,
-                                           volatile unsigned long long* s_bound, int most) {
+                                           volatile unsigned* s_bound, int most, const int* next, int keep) {
     using N = FarNum<k32>;
-    using I = typename N::I;
-    using D = typename N::D;
+    using T = typename N::T;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const I gx0 = g.gx0, gy0 = g.gy0, bs = g.bs, u1 = bs * kBinsPerBlockEdge, u2 = bs * kBinsPerSuperEdge;
-    const I X0 = __reduce_min_sync(full, b.px), X1 = __reduce_max_sync(full, b.px);
-    const I Y0 = __reduce_min_sync(full, b.py), Y1 = __reduce_max_sync(full, b.py);
+    const unsigned bs = g.bs, u1 = bs * kBinsPerBlockEdge, u2 = bs * kBinsPerSuperEdge;
+    const int ox = __reduce_min_sync(full, b.px), oy = __reduce_min_sync(full, b.py);      // the group's corner
+    const unsigned X0 = ox - g.gx0, X1 = __reduce_max_sync(full, b.px) - g.gx0;
+    const unsigned Y0 = oy - g.gy0, Y1 = __reduce_max_sync(full, b.py) - g.gy0;
+    const unsigned px = b.px - g.gx0, py = b.py - g.gy0;
+    auto warp_min = [&](T v) { return N::value(__reduce_min_sync(full, N::bits(v))); };
     // lane's bound: nothing farther can matter to it
-    auto bound = [&]() -> D {
-        if (!kCta) return b.d2;
-        const unsigned long long s = s_bound[lane];
-        return s < (unsigned long long)b.d2 ? (D)s : b.d2;
+    auto bound = [&]() -> T {
+        const unsigned v = N::bits(N::bound(b.d2));
+        return N::value(kCta ? min(v, s_bound[lane]) : v);
     };
     // the circles of the pixels' eighths (far_half, far_circle_r2)
     const int step2 = far_blocks ? 8 : 2;
-    float cx0 = act ? (float)(b.px - X0) : 3e38f, cx1 = act ? (float)(b.px - X0) : -3e38f;
-    float cy0 = act ? (float)(b.py - Y0) : 3e38f, cy1 = act ? (float)(b.py - Y0) : -3e38f;
+    float cx0 = act ? (float)(b.px - ox) : 3e38f, cx1 = act ? (float)(b.px - ox) : -3e38f;
+    float cy0 = act ? (float)(b.py - oy) : 3e38f, cy1 = act ? (float)(b.py - oy) : -3e38f;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const int x = k ? step2 : 1;
@@ -1333,15 +1348,13 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
     const float half = far_half(cx1 - cx0, cy1 - cy0, fmaxf((float)(X1 - X0), (float)(Y1 - Y0)));
     const bool writes = !(lane & (1 | step2));
     const int eighth = far_blocks ? ((lane >> 1) & 3) + 4 * (lane >> 4) : lane >> 2;
-    D maxd;
+    T maxd;
     auto new_bounds = [&]() {
-        D m = act ? bound() : (D)0;
-        maxd = N::warp_max(m);
-        D o = __shfl_xor_sync(full, m, 1);
-        m = o > m ? o : m;
-        o = __shfl_xor_sync(full, m, step2);
-        m = o > m ? o : m;
-        const float r2 = far_circle_r2(sqrt_est((float)m), half);
+        unsigned m = act ? N::bits(bound()) : 0u;
+        maxd = N::value(__reduce_max_sync(full, m));
+        m = max(m, __shfl_xor_sync(full, m, 1));
+        m = max(m, __shfl_xor_sync(full, m, step2));
+        const float r2 = far_circle_r2(sqrt_est((float)N::value(m)), half);
         if (writes) buf->circle[eighth] = make_float4(ccx, ccy, none_active ? -1.0f : r2, 0.0f);
         __syncwarp();
     };
@@ -1351,7 +1364,7 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
     auto round = [&](int q, bool in) {
         int4 p = make_int4(0, 0, 0, 0);
         if (in) p = __ldg(&pts[q]);
-        const float x = (float)((I)p.x - X0), y = (float)((I)p.y - Y0);
+        const float x = (float)(p.x - ox), y = (float)(p.y - oy);
         bool hit = false;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -1371,54 +1384,56 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
 #pragma unroll 4
         for (int k = 0; k < n; ++k) b.consider(buf->p[k], buf->q[k]);
         nev += n;
-        if (kCta && (unsigned long long)b.d2 < s_bound[lane])
-            atomicMin((unsigned long long*)&s_bound[lane], (unsigned long long)b.d2);
+        if (kCta) {
+            const unsigned v = N::bits(N::bound(b.d2));
+            if (v < s_bound[lane]) atomicMin((unsigned*)&s_bound[lane], v);
+        }
         new_bounds();                    // (its barrier also ends the buffer's use)
     };
-    const I reach = N::reach(maxd);
-    auto cell = [&](I v, I o, int n) {   // superblock column (row) of v, clamped to the grid
-        const long long c = (long long)v - o;
+    const long long reach = N::reach(maxd);
+    auto cell = [&](long long c, int n) {   // superblock column (row) of a place, clamped to the grid
         return c <= 0 ? 0 : (c >= (long long)n * u2 ? n - 1 : udiv32(c, u2));
     };
-    const int sx0 = cell(X0 - reach, gx0, g.n2x), sx1 = cell(X1 + reach, gx0, g.n2x);
-    const int sy0 = cell(Y0 - reach, gy0, g.n2y), sy1 = cell(Y1 + reach, gy0, g.n2y);
-    const int cx = cell(X0, gx0, g.n2x), cy = cell(Y0, gy0, g.n2y);
+    const int sx0 = cell(X0 - reach, g.n2x), sx1 = cell(X1 + reach, g.n2x);
+    const int sy0 = cell(Y0 - reach, g.n2y), sy1 = cell(Y1 + reach, g.n2y);
+    const int cx = cell(X0, g.n2x), cy = cell(Y0, g.n2y);
     const int nsx = sx1 - sx0 + 1, ns = nsx * (sy1 - sy0 + 1);
+    // whether superblock k of the box (row by row; the group's own one: k < 0)
+    // can hold points within the bounds
+    auto super_at = [&](int k, int& sx, int& sy) {
+        sy = k < 0 ? cy : sy0 + (int)((unsigned)k / (unsigned)nsx);
+        sx = k < 0 ? cx : sx0 + (int)((unsigned)k % (unsigned)nsx);
+        const unsigned SX0 = sx * u2, SY0 = sy * u2;
+        return N::square(N::gap(X0, X1, SX0, SX0 + u2 - 1), N::gap(Y0, Y1, SY0, SY0 + u2 - 1)) <= maxd;
+    };
     int searched = 0;
-    for (int k = -1, sx = cx, sy = cy; k < ns; ++k) {
-        // the group's own superblock first, then the others row by row
-        if (k >= 0) {
-            sx = k == 0 ? sx0 : (sx == sx1 ? sx0 : sx + 1);
-            sy = k == 0 ? sy0 : (sx == sx0 ? sy + 1 : sy);
-            if (sx == cx && sy == cy) continue;
-        }
+    // the group's own superblock first, then the others, one to a lane, and those
+    // that remain one by one
+    for (int s0 = -1; s0 < ns; s0 += s0 < 0 ? 1 : 32) {
+        const int mine = s0 < 0 ? -1 : s0 + lane;
+        int mx, my;
+        const bool within = mine < ns && (s0 >= 0 || lane == 0) && super_at(mine, mx, my);
+        unsigned live = __ballot_sync(full, within && (mine < 0 || mx != cx || my != cy) && __ldg(&smask[my * g.n2x + mx]));
+        while (live) {
+        int sx, sy;
+        const bool still = super_at(s0 < 0 ? -1 : s0 + __ffs(live) - 1, sx, sy);
+        live &= live - 1;
+        if (!still) continue;            // the bounds have shrunk
         const int sidx = sy * g.n2x + sx;
         const uint64_t sm = __ldg(&smask[sidx]);
-        if (!sm) continue;
-        const I SX0 = gx0 + (I)sx * u2, SY0 = gy0 + (I)sy * u2;
-        {
-            const I dx = interval_gap(X0, X1, SX0, SX0 + u2 - 1), dy = interval_gap(Y0, Y1, SY0, SY0 + u2 - 1);
-            if (dx > N::reach(maxd) || dy > N::reach(maxd) || (D)(dx * dx) + (D)(dy * dy) > maxd) continue;
-        }
+        const unsigned SX0 = sx * u2, SY0 = sy * u2;
         // this lane's two blocks: column lane & 7, rows lane >> 3 and + 4
-        D key0, key1;
-        const D none = ~(D)0;
+        T key0, key1;
         {
-            const I bx = SX0 + (I)(lane & 7) * u1, by = SY0 + (I)(lane >> 3) * u1;
-            I dx = interval_gap(X0, X1, bx, bx + u1 - 1);
-            I dy = interval_gap(Y0, Y1, by, by + u1 - 1), ey = interval_gap(Y0, Y1, by + 4 * u1, by + 5 * u1 - 1);
-            if (k32) {       // 46340^2 exceeds every bound here
-                dx = dx < 46340 ? dx : 46340;
-                dy = dy < 46340 ? dy : 46340;
-                ey = ey < 46340 ? ey : 46340;
-            }
-            key0 = (sm >> lane) & 1 ? (D)(dx * dx) + (D)(dy * dy) : none;
-            key1 = (sm >> (lane + 32)) & 1 ? (D)(dx * dx) + (D)(ey * ey) : none;
+            const unsigned bx = SX0 + (lane & 7) * u1, by = SY0 + (lane >> 3) * u1;
+            const unsigned dx = N::gap(X0, X1, bx, bx + u1 - 1);
+            key0 = (sm >> lane) & 1 ? N::square(dx, N::gap(Y0, Y1, by, by + u1 - 1)) : N::none();
+            key1 = (sm >> (lane + 32)) & 1 ? N::square(dx, N::gap(Y0, Y1, by + 4 * u1, by + 5 * u1 - 1)) : N::none();
             if (kCta) {
                 // residue classes of the blocks: neighbouring blocks go to different warps
                 const int c = (lane & 7) + 3 * (lane >> 3) + sx + sy;
-                if ((c & 7) != warp) key0 = none;
-                if (((c + 12) & 7) != warp) key1 = none;
+                if ((c & 7) != warp) key0 = N::none();
+                if (((c + 12) & 7) != warp) key1 = N::none();
             }
         }
         // their occupancy and point ranges, all in flight at once
@@ -1438,23 +1453,22 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
             }
         }
         for (;;) {
-            const D key = key0 < key1 ? key0 : key1, least = N::warp_min(key);
-            if (least > maxd || least == none) break;
+            const T key = key0 < key1 ? key0 : key1, least = warp_min(key);
+            if (least > maxd || least == N::none()) break;
             const int who = __ffs(__ballot_sync(full, key == least)) - 1;
             const int second = __shfl_sync(full, (int)(key0 != least), who);
             if (lane == who) {
-                if (second) key1 = none; else key0 = none;
+                if (second) key1 = N::none(); else key0 = N::none();
             }
             const int m = who + 32 * second;
-            const I BX0 = SX0 + (I)(m & 7) * u1, BY0 = SY0 + (I)(m >> 3) * u1;
-            // a disc must touch it (its gap to every lane is at most the bound, and fits)
-            const D bd = bound();
-            {
-                I dx = interval_gap((I)b.px, (I)b.px, BX0, BX0 + u1 - 1), dy = interval_gap((I)b.py, (I)b.py, BY0, BY0 + u1 - 1);
-                if (k32) { dx = dx < 46340 ? dx : 46340; dy = dy < 46340 ? dy : 46340; }
-                if (!__any_sync(full, (D)(dx * dx) + (D)(dy * dy) <= bd)) continue;
+            const unsigned BX0 = SX0 + (m & 7) * u1, BY0 = SY0 + (m >> 3) * u1;
+            // a disc must touch it
+            const T bd = bound();
+            if (!__any_sync(full, N::square(N::gap(px, px, BX0, BX0 + u1 - 1), N::gap(py, py, BY0, BY0 + u1 - 1)) <= bd)) continue;
+            if (!kCta && ++searched > most) {
+                if (!next || *(const volatile int*)next >= keep) return false;
+                searched = 0;
             }
-            if (!kCta && ++searched > most) return false;
             const int* st = start + (((int64_t)sidx << 6) + m << 6);
             const int bp0 = __shfl_sync(full, second ? first1 : first0, who);
             const int bp1 = __shfl_sync(full, second ? last1 : last0, who);
@@ -1463,54 +1477,45 @@ __device__ __forceinline__ bool far_search(const BinGrid& g, const int4* __restr
             // consecutive), else the rows' runs, first to last bin, that some
             // disc touches
             uint64_t run = 0;
-            int t0 = 0, t1 = 0, s0 = bp0, e0 = bp1;
+            int t0 = 0, t1 = 0, q0 = bp0, q1 = bp1;
             if (bp1 - bp0 > 32) {
-                e0 = bp0;
+                q1 = bp0;
                 t0 = __ldg(&st[lane]);
                 t1 = __ldg(&st[lane + 32]);
                 const unsigned bm0 = __shfl_sync(full, second ? (unsigned)mask1 : (unsigned)mask0, who);
                 const unsigned bm1 = __shfl_sync(full, second ? (unsigned)(mask1 >> 32) : (unsigned)(mask0 >> 32), who);
-                {
-                    const I qx = BX0 + (I)(lane & 7) * bs, qy = BY0 + (I)(lane >> 3) * bs;
-                    I dx = interval_gap(X0, X1, qx, qx + bs - 1);
-                    I dy = interval_gap(Y0, Y1, qy, qy + bs - 1), ey = interval_gap(Y0, Y1, qy + 4 * bs, qy + 5 * bs - 1);
-                    if (k32) {
-                        dx = dx < 46340 ? dx : 46340;
-                        dy = dy < 46340 ? dy : 46340;
-                        ey = ey < 46340 ? ey : 46340;
-                    }
-                    const unsigned lo = __ballot_sync(full, (D)(dx * dx) + (D)(dy * dy) <= maxd);
-                    const unsigned hi = __ballot_sync(full, (D)(dx * dx) + (D)(ey * ey) <= maxd);
-                    run = (uint64_t)(bm0 & lo) | ((uint64_t)(bm1 & hi) << 32);
-                }
+                const unsigned qx = BX0 + (lane & 7) * bs, qy = BY0 + (lane >> 3) * bs;
+                const unsigned dx = N::gap(X0, X1, qx, qx + bs - 1);
+                const unsigned lo = __ballot_sync(full, N::square(dx, N::gap(Y0, Y1, qy, qy + bs - 1)) <= maxd);
+                const unsigned hi = __ballot_sync(full, N::square(dx, N::gap(Y0, Y1, qy + 4 * bs, qy + 5 * bs - 1)) <= maxd);
+                run = (uint64_t)(bm0 & lo) | ((uint64_t)(bm1 & hi) << 32);
             }
             for (;;) {
                 int fill = 0, q = 0;
                 while (fill < 32) {
-                    if (s0 == e0) {
+                    if (q0 == q1) {
                         if (!run) break;
                         const int r = ffs64(run) >> 3;
                         const unsigned bits = (unsigned)(run >> (8 * r)) & 0xFFu;
                         run &= ~(0xFFull << (8 * r));
                         const int a = __ffs(bits) - 1, e = 31 - __clz(bits);
-                        const I qx = BX0 + (I)a * bs, qy = BY0 + (I)r * bs;
-                        I dx = interval_gap((I)b.px, (I)b.px, qx, qx + (I)(e - a + 1) * bs - 1);
-                        I dy = interval_gap((I)b.py, (I)b.py, qy, qy + bs - 1);
-                        if (k32) { dx = dx < 46340 ? dx : 46340; dy = dy < 46340 ? dy : 46340; }
-                        if (!__any_sync(full, (D)(dx * dx) + (D)(dy * dy) <= bd)) continue;
+                        const unsigned qx = BX0 + a * bs, qy = BY0 + r * bs;
+                        if (!__any_sync(full, N::square(N::gap(px, px, qx, qx + (e - a + 1) * bs - 1),
+                                                        N::gap(py, py, qy, qy + bs - 1)) <= bd)) continue;
                         const int ia = 8 * r + a, ie = 8 * r + e + 1;
-                        s0 = __shfl_sync(full, ia < 32 ? t0 : t1, ia & 31);
-                        e0 = __shfl_sync(full, ie < 32 ? t0 : t1, ie & 31);
-                        if (ie == 64) e0 = bp1;
+                        q0 = __shfl_sync(full, ia < 32 ? t0 : t1, ia & 31);
+                        q1 = __shfl_sync(full, ie < 32 ? t0 : t1, ie & 31);
+                        if (ie == 64) q1 = bp1;
                     }
-                    const int take = min(32 - fill, e0 - s0);
-                    if ((unsigned)(lane - fill) < (unsigned)take) q = s0 + lane - fill;
+                    const int take = min(32 - fill, q1 - q0);
+                    if ((unsigned)(lane - fill) < (unsigned)take) q = q0 + lane - fill;
                     fill += take;
-                    s0 += take;
+                    q0 += take;
                 }
                 if (fill) round(q, lane < fill);
                 if (fill < 32) break;
             }
+        }
         }
     }
     return true;
@@ -1593,10 +1598,10 @@ __device__ __forceinline__ void far_load(FarWork& w, const BatchTables& bt, cons
 template <bool k32, bool kCta>
 __device__ __forceinline__ bool far_run(FarWork& w, const TileParams& T, const int4* pts_all, const int* start_all,
                                         const uint64_t* bmask_all, const uint64_t* smask_all, FarBuf* buf, int far_blocks,
-                                        volatile unsigned long long* s_bound, int most) {
+                                        volatile unsigned* s_bound, int most, const int* next = nullptr, int keep = 0) {
     FarLane<k32> b{w.px, w.py, (typename FarNum<k32>::D)w.b.d2, w.b.gid, w.b.z, w.b.idx};
     const bool done = far_search<k32, kCta>(T.bg, pts_all + T.srt_off, start_all + T.bin_off, bmask_all + T.blk_off,
-                                            smask_all + T.sup_off, b, w.act, w.nev, buf, far_blocks, s_bound, most);
+                                            smask_all + T.sup_off, b, w.act, w.nev, buf, far_blocks, s_bound, most, next, keep);
     w.b.d2 = (long long)b.d2;
     w.b.gid = b.gid;
     w.b.z = b.z;
@@ -1607,6 +1612,15 @@ __device__ __forceinline__ bool far_run(FarWork& w, const TileParams& T, const i
 __device__ __forceinline__ bool far_small(const FarWork& w, const TileParams& T) {
     const long long r = w.b.d2 < (1LL << 31) ? (long long)sqrt_est((float)w.b.d2) + 2 : LLONG_MAX / 4;
     return __all_sync(0xffffffffu, far_fits32(r, T.bg.bs, T.cs));
+}
+
+// The searches beyond 32-bit distances, as functions of their own: inlined, their
+// registers cost the 32-bit ones spills.
+template <bool kCta>
+__device__ __noinline__ bool far_run_wide(FarWork* w, const TileParams* T, const int4* pts_all, const int* start_all,
+                                          const uint64_t* bmask_all, const uint64_t* smask_all, FarBuf* buf, int far_blocks,
+                                          volatile unsigned* s_bound, int most, const int* next, int keep) {
+    return far_run<false, kCta>(*w, *T, pts_all, start_all, bmask_all, smask_all, buf, far_blocks, s_bound, most, next, keep);
 }
 
 __device__ __forceinline__ void far_settle(const FarWork& w, const TileParams& T, int2* __restrict__ pix,
@@ -1626,11 +1640,14 @@ __device__ __forceinline__ void far_settle(const FarWork& w, const TileParams& T
 
 // Far pass over the worklist: one warp per group, handed out by a counter
 // (groups differ in cost by orders of magnitude: a lake's centre against its
-// shore).  Groups that need more than kFarDefer blocks, or 64-bit arithmetic
-// (this kernel then holds one search, which fits the instruction cache: with
-// both, and the candidate round in four places, a warp waited four issue slots
-// for instructions), go, with the sites found so far, to the heavy list (in the span items' place, which are listed
-// later; at most 64 groups per raster tile).
+// shore).  Groups that need more than `most` blocks go, with the sites found so
+// far, to the heavy list (in the span items' place, which are listed later; at
+// most 64 groups per raster tile).  Groups beyond 32-bit distances (nearest sites
+// more than 463 m away at 1 cm) run the wide search, a function of its own: with
+// both inlined a warp waited four issue slots for instructions and the 32-bit one
+// spilled.  (All such groups on whole CTAs, with 64-bit tests: a 4096^2 tile at
+// 0.1 points per cell in millimetres, with lakes, 30.3 ms, now 19.8; 200 mixed
+// tiles in millimetres 11.4 ms, now 7.6.)
 __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4* __restrict__ pts_all,
                                                      const int* __restrict__ start_all,
                                                      const uint64_t* __restrict__ bmask_all,
@@ -1655,8 +1672,14 @@ __global__ void __launch_bounds__(256, 4) k_near_far(BatchTables bt, const int4*
         FarWork w;
         far_load(w, bt, far, k, far_blocks, pts_all, start_all, bmask_all, near_all);
         const TileParams& T = bt.tiles[w.t];
-        const bool done = far_small(w, T) &&
-                          far_run<true, false>(w, T, pts_all, start_all, bmask_all, smask_all, buf, far_blocks, nullptr, most);
+        bool done;
+        if (far_small(w, T)) {
+            done = far_run<true, false>(w, T, pts_all, start_all, bmask_all, smask_all, buf, far_blocks, nullptr, most);
+        } else {
+            FarWork v = w;
+            done = far_run_wide<false>(&v, &T, pts_all, start_all, bmask_all, smask_all, buf, far_blocks, nullptr, most, &ctr->far_next, count - kFarKeep * 8 * (int)gridDim.x);
+            w = v;
+        }
         if (done) {
             far_settle(w, T, pix, site, sc, far, blockIdx.x * 3 + (threadIdx.x >> 5));
         } else {
@@ -1799,7 +1822,7 @@ __global__ void __launch_bounds__(256, 4) k_near_far_heavy(BatchTables bt, const
     chained();
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n64; k += (int64_t)gridDim.x * blockDim.x) D[k] = 0;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n32; k += (int64_t)gridDim.x * blockDim.x) Dc[k] = 0;
-    __shared__ unsigned long long s_bound[32];
+    __shared__ unsigned s_bound[32];         // each lane's bound, as FarNum::bits gives it
     __shared__ Best s_best[8][32];
     __shared__ FarBuf s_buf[8];
     __shared__ int s_k;
@@ -1814,10 +1837,11 @@ __global__ void __launch_bounds__(256, 4) k_near_far_heavy(BatchTables bt, const
         if (s_k >= count) break;
         FarWork w;
         far_load(w, bt, far, all ? s_k : heavy[s_k], far_blocks, pts_all, start_all, bmask_all, near_all);
-        if (warp == 0) s_bound[lane] = (unsigned long long)w.b.d2;
-        __syncthreads();
         const TileParams& T = bt.tiles[w.t];
-        if (far_small(w, T)) far_run<true, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], far_blocks, s_bound, 0);
+        const bool small = far_small(w, T);
+        if (warp == 0) s_bound[lane] = ~0u;
+        __syncthreads();
+        if (small) far_run<true, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], far_blocks, s_bound, 0);
         else far_run<false, true>(w, T, pts_all, start_all, bmask_all, smask_all, &s_buf[warp], far_blocks, s_bound, 0);
         w.b.nev = (int)w.nev;
         s_best[warp][lane] = w.b;

@@ -180,3 +180,26 @@ def test_no_budget_is_refused_above_an_accepted_one(eng, kind):
             lo = mid
     for k in range(1, 49):
         assert accepted(int(hi * 1.025 ** k))
+
+
+# groups beyond 32-bit distances against the same geometry in smaller units: few
+# groups, groups that leave their warp, and a list long enough that they stay
+@pytest.mark.parametrize("side,n,scale", [(60, 900, 500), (300, 90_000, 50), (300, 9000, 50_000), (800, 120_000, 50),
+                                          (800, 30_000, 50_000)])
+@pytest.mark.parametrize("groups", [1, 2])
+def test_far_pass_beyond_32_bits(eng, side, n, scale, groups):
+    from terranni_b200 import engine
+    rng = np.random.default_rng(side + n)
+    w = 20 * side
+    xyz = _points(rng, n, w, w)
+    d = (xyz[:, :2] - w // 2).astype(np.int64)
+    xyz = xyz[(d * d).sum(1) > (0.46 * w) ** 2]
+    out = []
+    for k in (1, scale):
+        p = xyz * np.array([k, k, 1], np.int32)
+        tile = engine.make_tile(engine.make_wp(side, side, 20 * k), 0, p.shape[0], 0, 0, extent=(0, 0, w * k - 1, w * k - 1))
+        h, site = np.empty(side * side, np.float32), np.empty(side * side, np.uint32)
+        with eng.batch([tile], far_group=groups) as b:
+            b.run(p, h, out_site=site)
+        out.append((h, site))
+    assert np.array_equal(out[0][1], out[1][1]) and _same(out[0][0], out[1][0])
