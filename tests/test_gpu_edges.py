@@ -203,3 +203,23 @@ def test_far_pass_beyond_32_bits(eng, side, n, scale, groups):
             b.run(p, h, out_site=site)
         out.append((h, site))
     assert np.array_equal(out[0][1], out[1][1]) and _same(out[0][0], out[1][0])
+
+
+def test_a_request_by_itself_does_not_wait_for_company():
+    """While a long batch runs and a slot is free, a request that comes alone is
+    launched at once."""
+    import time
+    from terranni_b200 import engine
+    rng = np.random.default_rng(3)
+    xyz = _points(rng, 400_000, 120_000, 120_000)
+    queued = []
+    with engine.Engine(device=0) as e, e.server(xyz, slots=2, slot_bytes=4 << 30) as srv:
+        srv.wait(srv.submit(0, 0, 64, 64, 100))
+        for _ in range(8):
+            long = srv.submit(0, 0, 6000, 6000, 20)
+            time.sleep(0.002)
+            h, _, r = srv.wait(srv.submit(10_000, 20_000, 64, 64, 100))
+            queued.append(r["ms_queue"])
+            srv.wait(long)
+            time.sleep(0.002)
+    assert min(queued) < 0.09
