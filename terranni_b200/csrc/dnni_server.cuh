@@ -218,13 +218,16 @@ bool srv_plan(dnni_server* s, uint64_t ticket, const SrvReq& q, std::vector<SegC
     return true;
 }
 
+// A slot's late arrays, which hold the batch's chunk list until its points are
+// gathered (before any kernel of the launch sequence).
+size_t srv_late(const ScratchSizes& z, size_t nchunks) { return std::max(z.late(), al256(sizeof(SegChunk) * nchunks)); }
+
 // Device bytes a batch needs in a slot arena: staging plus scratch.
 size_t srv_footprint(const HostBatch& hb, int64_t pts, int64_t out, int64_t site, size_t nchunks) {
     const ScratchSizes z = scratch_sizes(hb);
     size_t b = al256(12 * (size_t)pts) + al256(4 * (size_t)pts) + al256(4 * (size_t)out) + al256(4 * (size_t)site) +
-               al256(sizeof(SegChunk) * nchunks);
-    const size_t parts[] = {z.tables, z.sc, z.ctr, z.pix, z.far, z.D, z.Dc, z.sorted, z.cnt, z.cnt, z.bsum,
-                            z.bmask, z.smask, z.rownear, z.near};
+               srv_late(z, nchunks);
+    const size_t parts[] = {z.tables, z.sc, z.ctr, z.sorted, z.cnt, z.cnt, z.bsum, z.bmask, z.smask, z.rownear, z.near};
     for (size_t p : parts) b += al256(p);
     return b;
 }
@@ -256,14 +259,15 @@ dnni_status srv_launch(dnni_server* s, SrvSlot& sl, std::vector<SrvItem>& items,
     uint32_t* ggid = (uint32_t*)take(4 * (size_t)pts);
     float* gout = (float*)take(4 * (size_t)out);
     uint32_t* gsite = (uint32_t*)take(4 * (size_t)site);
-    SegChunk* dch = (SegChunk*)take(sizeof(SegChunk) * chunks.size());
     DevArrays a;
     const ScratchSizes z = scratch_sizes(hb);
     a.tables = take(z.tables);
     a.sc = (Scalars*)take(z.sc);
     a.ctr = (BatchCounters*)take(z.ctr);
     // (no room beyond the admitted footprint: denser batches bin directly)
-    carve_late(take(z.late()), z.late(), z, a, nullptr);
+    void* late = take(srv_late(z, chunks.size()));
+    SegChunk* dch = (SegChunk*)late;
+    carve_late(late, z.late(), z, a, nullptr);
     a.sorted = (int4*)take(z.sorted);
     a.cnt = (int*)take(z.cnt);
     a.start = (int*)take(z.cnt);

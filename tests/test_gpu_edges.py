@@ -223,3 +223,29 @@ def test_a_request_by_itself_does_not_wait_for_company():
             srv.wait(long)
             time.sleep(0.002)
     assert min(queued) < 0.09
+
+
+def test_a_slot_has_no_room_to_spare_for_the_gather_list():
+    """The smallest slot that takes a request over the whole cloud does not depend
+    on how many buckets, and so gather chunks, the cloud has."""
+    from terranni_b200 import engine
+    rng = np.random.default_rng(5)
+    xyz = _points(rng, 60_000, 40_000, 40_000)
+
+    def fits(bucket, bytes_):
+        with engine.Engine(device=0) as e, e.server(xyz, bucket=bucket, slots=1, slot_bytes=bytes_) as srv:
+            try:
+                srv.wait(srv.submit(0, 0, 100, 100, 400))
+            except engine.DnniError as err:
+                assert err.status == 2
+                return False
+            return True
+
+    least = []
+    for bucket in (40_000, 100):
+        lo, hi = 1 << 12, 1 << 26
+        while hi - lo > 256:                # a slot takes a quarter more than it is asked for
+            mid = (lo + hi) // 2
+            lo, hi = (lo, mid) if fits(bucket, mid) else (mid, hi)
+        least.append(hi)
+    assert least[1] <= least[0] + 256
