@@ -482,8 +482,9 @@ static dnni_status compat_run(dnni_ctx* c, const dnni_compat_settings* s, const 
     float* dh = device ? h_out : (float*)c->out_h.p;
     int32_t* dres = res_out ? (device ? res_out : (int32_t*)c->out_site.p) : nullptr;
     uint2* pixel = (uint2*)c->scr.late.p;
-    // pixels one square spans at most, one axis (with its rounding)
-    const long long span = (long long)std::ceil(2.0 * G.rs / G.pixel_size) + 3;
+    // pixels of the raster that one square spans at most, one axis (with its rounding)
+    const double across = std::ceil(2.0 * G.rs / G.pixel_size), most = (double)std::max(xp, yp);
+    const long long span = (long long)(across < most ? across : most) + 3;
     // the offsets, then the counts, of nt tiles
     auto tile_bytes = [](long long nt, int per_tile) { return sizeof(long long) * (size_t)(nt + 1) + per_tile * sizeof(int) * (size_t)nt; };
     const long long gx = (xp + kCgTile - 1) / kCgTile, gy = (yp + kCgTile - 1) / kCgTile;

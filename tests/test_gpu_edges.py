@@ -249,3 +249,18 @@ def test_a_slot_has_no_room_to_spare_for_the_gather_list():
             lo, hi = (lo, mid) if fits(bucket, mid) else (mid, hi)
         least.append(hi)
     assert least[1] <= least[0] + 256
+
+
+# site squares over the whole raster and far beyond it: the count of tiles that one
+# reaches has to stay within what the raster has
+@pytest.mark.parametrize("site_radius", [1e4, 2.5e10, 1e11, 1e12, 1e14])
+def test_compat_squares_beyond_the_raster(eng, oracle, site_radius):
+    from terranni_b200 import engine
+    rng = np.random.default_rng(2)
+    nc, nr, n = 40, 30, 60
+    pts = np.stack([rng.uniform(0, 2 * nc, n), rng.uniform(0, 2 * nr, n), rng.uniform(0, 30, n)], 1)
+    arg = dict(scale=5, cell_size=2.0, site_radius=site_radius, query_radius=4.99, point_min=0, multiplier=10000,
+               total_ncols=nc, total_nrows=nr)
+    ref_h, ref_res = oracle.compat(oracle.CompatSettings(**arg), oracle.CompatWP(nrows=nr, ncols=nc), pts)
+    h, res = eng.interpolate_compat(engine.CompatSettings(**arg), engine.CompatWP(nrows=nr, ncols=nc), pts)
+    assert np.array_equal(res, ref_res) and _same(h, ref_h)
