@@ -1890,7 +1890,8 @@ __device__ __forceinline__ void emit_span(int row, int a, int b, int ncols, int 
 // R2 < 2^20: t = R2 - dy^2 + 1/2 is exact in a float, and for k^2 <= t - 1/2 <
 // (k+1)^2, k < 1024, its root lies at least 1/(4k+4) > 2.4e-4 from both k and
 // k+1, twice the error of the hardware estimate (relative 2^-23, so 1.3e-4);
-// the estimate rounded down is therefore the half-width itself.  The floor
+// the estimate rounded down is therefore the half-width itself (the tests run
+// every value of the range on the device).  The floor
 // is taken by adding 2^23 with rounding towards minus infinity, which leaves
 // the integer in the low mantissa bits: no conversion instructions.  Larger
 // discs take the estimate and one exact integer step each way.

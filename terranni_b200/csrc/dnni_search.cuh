@@ -116,10 +116,10 @@ struct Scalars {
 
 #ifdef __CUDACC__
 // Square-root estimate of a non-negative float from the hardware
-// approximation (PTX sqrt.approx.ftz.f32; relative error a few units of
-// 2^-23), for callers that correct the result with exact integer products or
-// need it only within a fraction of one unit (below 2^31 the absolute error
-// stays under 0.05).
+// approximation (PTX sqrt.approx.ftz.f32, documented to a relative error of
+// 2^-23), for callers that correct the result with exact integer products, need
+// it only within a fraction of one unit (below 2^31 the absolute error stays
+// under 0.05), or take it over a range whose every value a test runs (SpanRows).
 __device__ __forceinline__ float sqrt_est(float x) {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

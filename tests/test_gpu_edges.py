@@ -1,7 +1,13 @@
 """Calls at the edges of the engine's routes, bit for bit against the oracle:
-thin tiles without points beside tiles with points."""
+thin tiles without points beside tiles with points, wide cells, scratch limits."""
+import ctypes
+import os
+import subprocess
+
 import numpy as np
 import pytest
+
+from conftest import NATIVE, ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -264,3 +270,28 @@ def test_compat_squares_beyond_the_raster(eng, oracle, site_radius):
     ref_h, ref_res = oracle.compat(oracle.CompatSettings(**arg), oracle.CompatWP(nrows=nr, ncols=nc), pts)
     h, res = eng.interpolate_compat(engine.CompatSettings(**arg), engine.CompatWP(nrows=nr, ncols=nc), pts)
     assert np.array_equal(res, ref_res) and _same(h, ref_h)
+
+
+@pytest.fixture(scope="module")
+def span():
+    src, so = os.path.join(NATIVE, "dnni_span.cu"), os.path.join(NATIVE, "libdnni_span.so")
+    csrc = os.path.join(ROOT, "terranni_b200", "csrc")
+    deps = [src] + [os.path.join(csrc, f) for f in ("dnni_search.cuh", "dnni_kernels.cuh", "dnni_plan.h")]
+    if not os.path.exists(so) or any(os.path.getmtime(d) > os.path.getmtime(so) for d in deps):
+        subprocess.run(["/usr/local/cuda/bin/nvcc", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-gencode",
+                        "arch=compute_100a,code=sm_100a", "-o", so, src], check=True, capture_output=True)
+    return ctypes.CDLL(so)
+
+
+# the estimate's exact range, R2 - dy^2 of every value below 2^20, and samples of
+# the corrected estimate beyond it up to the largest R2
+@pytest.mark.parametrize("n0,step,dy,n", [(0, 1, 0, 1 << 20), (0, 1, 1, (1 << 20) - 1), (0, 1, 511, (1 << 20) - 511 ** 2),
+                                          (0, 1, 1023, (1 << 20) - 1023 ** 2), (1 << 20, 1, 0, 1 << 22),
+                                          (0, 4093, 30000, 300_000), (1 << 20, 2039, 0, 1_050_000)])
+def test_half_widths_are_exact(span, n0, step, dy, n):
+    out = np.empty(n, np.int32)
+    assert span.span_half_widths(ctypes.c_int64(n0), ctypes.c_int64(step), dy, n, out.ctypes.data_as(ctypes.c_void_p)) == 0
+    v = n0 + np.arange(n, dtype=np.int64) * step
+    assert int(v[-1]) + dy * dy < 1 << 31
+    w = np.floor(np.sqrt(v.astype(np.float64))).astype(np.int64)
+    assert np.all(w * w <= v) and np.all((w + 1) ** 2 > v) and np.array_equal(out, w)
