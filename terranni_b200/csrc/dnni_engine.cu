@@ -325,8 +325,8 @@ void launch_body(const HostBatch& hb, const BatchTables& bt, const DevArrays& a,
         if (nblk > 0) launch(chain, k_block_near, (int)((nblk + 255) / 256), 256, 0, st, bt, a.smask, a.rownear, a.near, far.rtmax);
     }
     if (ev) cudaEventRecord(ev[0], st);
-    // a raster tile goes to several CTAs while the tiles alone leave the SMs
-    // (four CTAs each) without two rounds of work
+    // a raster tile goes to several CTAs while the tiles alone are fewer than
+    // eight to an SM, which holds three at once
     int split = 1;
     while (split < kTileY / 8 && (int64_t)nrt * split < 8 * (int64_t)sms) split *= 2;
     const auto dense = d_gid && !unique_gid ? k_near_dense<true> : k_near_dense<false>;

@@ -1,7 +1,9 @@
-// dnni_search.cuh -- data layout and the exact nearest-site search of the
-// discrete natural-neighbour interpolation engine, as __host__ __device__
-// code shared by the sm_100a kernels (dnni_kernels.cuh) and a host build
-// that the test suite checks against the oracle.
+// dnni_search.cuh -- data layout, the ring search and the arithmetic helpers of
+// the discrete natural-neighbour interpolation engine, as __host__ __device__
+// code shared by the sm_100a kernels (dnni_kernels.cuh) and a host build that
+// the test suite checks against the oracle; and a whole search of one pixel
+// (nearest_search and what only it calls) that serves that host build alone:
+// the far pass of the kernels is warp-cooperative and lives beside them.
 //
 // Replaces, per work package:
 //   nni.cpp:722-790 renderInputPoints / nni.cpp:171-230 drawPlane (the GL
@@ -332,7 +334,7 @@ struct BinWindow {
     const int4* lpts;
 };
 
-// search_bins on a staged window; identical results.  Every bin within
+// search_bins on a staged window (host build); identical results.  Every bin within
 // kRingsBins rings of the pixel's bin (inside the grid) must lie in the window.
 DNNI_HD bool search_bins_window(const BinGrid& g, const BinWindow& w, int px, int py, Best& b) {
     const long long gx0 = g.gx0, gy0 = g.gy0, bs = g.bs;
@@ -584,6 +586,14 @@ DNNI_HD int ffs64(uint64_t v) {
 #endif
 }
 
+// Block index (in bmask order) of block (cx, cy) of the block grid.
+DNNI_HD int64_t block_index(const BinGrid& g, int cx, int cy) {
+    return ((int64_t)((cy >> 3) * g.n2x + (cx >> 3)) << 6) + (((cy & 7) << 3) | (cx & 7));
+}
+
+// ---- the rest of a pixel's search, one pixel at a time (host build): the tests'
+// counterpart of the kernels' far pass, from other seeds and in another order ----
+
 // A first bound for a pixel whose bound is still infinite: the nearest
 // non-empty superblock ring is found, and in each of its non-empty
 // superblocks the closest non-empty block and, in it, the closest non-empty
@@ -707,11 +717,6 @@ DNNI_HD void search_disc(const BinGrid& g, const int4* __restrict__ pts, const i
             }
         }
     }
-}
-
-// Block index (in bmask order) of block (cx, cy) of the block grid.
-DNNI_HD int64_t block_index(const BinGrid& g, int cx, int cy) {
-    return ((int64_t)((cy >> 3) * g.n2x + (cx >> 3)) << 6) + (((cy & 7) << 3) | (cx & 7));
 }
 
 // 8 x 8 mask of the cells [a0,a1] x [b0,b1] of a block (x = bit & 7,
