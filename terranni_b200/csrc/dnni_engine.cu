@@ -59,10 +59,15 @@ size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 struct ScratchSizes {
     size_t sorted, cnt, bsum, bmask, smask, rownear, near, pix, far, D, Dc, sc, ctr, tables;
     size_t part;                     // the points grouped by region
-    size_t late() const { return al256(pix) + al256(far) + al256(D) + al256(Dc); }
+    size_t spare = 0;                // of the late arrays: room for the slices' rounding (kSlicePad)
+    size_t late_bytes() const { return far + D + pix + Dc; }
+    size_t late() const { return al256(late_bytes() + spare); }
     // of the grouped points' own buffer, 0 where they fit over `bytes` of late arrays
     size_t own_part(size_t bytes) const { return bytes >= part ? 0 : al256(part); }
 };
+
+constexpr int kSlices = 16;          // most slices of a pipelined batch
+constexpr size_t kSlicePad = 15;     // a slice's late arrays start on 16 bytes
 
 ScratchSizes scratch_sizes(const HostBatch& hb) {
     const int n = (int)hb.tiles.size();
@@ -85,18 +90,25 @@ ScratchSizes scratch_sizes(const HostBatch& hb) {
     return z;
 }
 
+// A batch's, whose late arrays may be laid out slice by slice.
+ScratchSizes batch_sizes(const HostBatch& hb) {
+    ScratchSizes z = scratch_sizes(hb);
+    z.spare = kSlices * kSlicePad;
+    return z;
+}
+
 // Lays out the arrays of the phases after the binning in `bytes` at base; the
 // points grouped by region go over them where they are large enough, else to
 // `part` (null: no room for them).
 void carve_late(void* base, size_t bytes, const ScratchSizes& z, DevArrays& a, void* part) {
-    unsigned char* p = (unsigned char*)base;
+    unsigned char* p = (unsigned char*)base;         // in order of their alignment
     a.part = (int4*)(z.own_part(bytes) ? part : base);
-    a.pix = (int2*)p;
-    p += al256(z.pix);
     a.far = (int4*)p;
-    p += al256(z.far);
+    p += z.far;
     a.D = (unsigned long long*)p;
-    p += al256(z.D);
+    p += z.D;
+    a.pix = (int2*)p;
+    p += z.pix;
     a.Dc = (int*)p;
 }
 
@@ -791,7 +803,7 @@ dnni_status dnni_batch_create(dnni_ctx* c, const dnni_tile* tiles, int32_t ntile
         }
     }
     // (a batch's scratch never grows)
-    dnni_status rs = with_room(c, [&] { return ensure_scratch(c, b->scr, scratch_sizes(b->hb), b->arr, true, false); });
+    dnni_status rs = with_room(c, [&] { return ensure_scratch(c, b->scr, batch_sizes(b->hb), b->arr, true, false); });
     if (!rs) {
         b->bt = device_tables(b->arr.tables, b->hb);
         rs = stage_tables(c, b->hb, b->arr.tables, c->stream);
@@ -885,7 +897,6 @@ static dnni_status plan_slices(dnni_batch* b) {
     // the next ones grow by 1.5x (each upload, at about two thirds of the
     // compute rate, then ends before the compute of its predecessor), and a
     // small last slice shortens the final download
-    constexpr int kSlices = 16;
     constexpr double kSliceWeight[kSlices] = {0.05, 0.075, 0.11, 0.17, 0.25, 0.38, 0.57, 0.85,
                                               1.0, 1.0, 1.0, 1.0, 1.0, 0.5, 0.25, 0.12};
     const int n = (int)b->tiles_in.size();
@@ -954,21 +965,24 @@ static dnni_status plan_slices(dnni_batch* b) {
     const int ns = (int)b->slices.size();
     dnni_status rs;
     if ((rs = dnni_ensure(c, b->slice_ctrs, sizeof(BatchCounters) * (size_t)ns, false))) return rs;
-    // a slice's grouped points lie over its worklist where they fit, else in the
-    // batch's `part`, which the whole batch's share with them (a batch runs as
-    // slices or whole, one at a time)
-    const ScratchSizes z = scratch_sizes(b->hb);
-    const auto own_part = [](const HostBatch& h) { return kFarSlotBytes * h.n_far >= (int64_t)sizeof(int4) * h.n_pts ? 0 : h.n_pts; };
-    int64_t part_pts = 0;
-    for (const BatchSlice& sl : b->slices) part_pts += own_part(sl.hb);
+    // a slice's late arrays lie together, its grouped points over them where they
+    // fit and else in the batch's `part`, which the whole batch's share with them
+    // (a batch runs as slices or whole, one at a time)
+    const ScratchSizes z = batch_sizes(b->hb);
+    size_t part_bytes = 0;
+    for (const BatchSlice& sl : b->slices) {
+        const ScratchSizes zs = scratch_sizes(sl.hb);
+        part_bytes += zs.own_part(zs.late_bytes());
+    }
     const size_t whole = z.own_part(b->scr.late.cap);
     const void* was = b->scr.part.p;
-    int4* part = (int4*)ensure_optional(c, b->scr.part, std::max(sizeof(int4) * (size_t)part_pts, whole), false);
+    unsigned char* part = (unsigned char*)ensure_optional(c, b->scr.part, std::max(part_bytes, whole), false);
     // (a refused growth leaves the buffer as it was, or none)
     if (b->scr.part.p != was) drop_graph(b);
     carve_late(b->scr.late.p, b->scr.late.cap, z, b->arr, b->scr.part.cap >= whole ? b->scr.part.p : nullptr);
     {
-        int64_t pts = 0, bins = 0, scan = 0, blk = 0, sup = 0, pix = 0, far = 0, cells = 0, tiles = 0;
+        unsigned char* late = (unsigned char*)b->scr.late.p;
+        int64_t pts = 0, bins = 0, scan = 0, blk = 0, sup = 0, tiles = 0;
         for (int s = 0; s < ns; ++s) {
             BatchSlice& sl = b->slices[s];
             const HostBatch& h = sl.hb;
@@ -981,12 +995,10 @@ static dnni_status plan_slices(dnni_batch* b) {
             v.smask += sup;
             v.rownear += blk;
             v.near += blk;
-            v.pix += pix;
-            v.far += far;
-            v.D += cells;
-            v.Dc += cells;
-            v.part = own_part(h) ? part : v.far;
-            if (part) part += own_part(h);
+            const ScratchSizes zs = scratch_sizes(h);
+            carve_late(late, zs.late_bytes(), zs, v, part);
+            late += (zs.late_bytes() + kSlicePad) & ~kSlicePad;
+            if (part) part += zs.own_part(zs.late_bytes());
             v.sc += tiles;
             v.ctr = (BatchCounters*)b->slice_ctrs.p + s;
             v.tables = (unsigned char*)sl.tables.p;
@@ -996,9 +1008,6 @@ static dnni_status plan_slices(dnni_batch* b) {
             scan += h.scan_base.back();
             blk += h.blk_base.back();
             sup += h.sup_base.back();
-            pix += h.n_pix;
-            far += h.n_far;
-            cells += h.n_cells;
             tiles += (int64_t)h.tiles.size();
         }
     }
