@@ -68,7 +68,11 @@ typedef struct dnni_settings {
     int32_t bin_target;     /* mean points per search bin; 0 = default (4) */
     int32_t flags;          /* DNNI_F_* */
     uint64_t mem_budget;    /* bytes of device scratch a context may hold;
-                               0 = no limit */
+                               0 = no limit.  A call that would pass it (or
+                               the device's memory) first gives back what
+                               the context keeps from earlier calls; from
+                               then until dnni_clear buffers take exactly
+                               what they need */
 } dnni_settings;
 
 #define DNNI_F_TIMING 1     /* record per-phase CUDA-event times in dnni_stats */

@@ -218,17 +218,18 @@ def test_a_request_by_itself_does_not_wait_for_company():
     from terranni_b200 import engine
     rng = np.random.default_rng(3)
     xyz = _points(rng, 400_000, 120_000, 120_000)
-    queued = []
+    idle, queued = [], []
     with engine.Engine(device=0) as e, e.server(xyz, slots=2, slot_bytes=4 << 30) as srv:
-        srv.wait(srv.submit(0, 0, 64, 64, 100))
-        for _ in range(8):
+        for _ in range(16):
+            idle.append(srv.wait(srv.submit(0, 0, 64, 64, 100))[2]["ms_queue"])
+            time.sleep(0.002)
             long = srv.submit(0, 0, 6000, 6000, 20)
             time.sleep(0.002)
             h, _, r = srv.wait(srv.submit(10_000, 20_000, 64, 64, 100))
             queued.append(r["ms_queue"])
             srv.wait(long)
             time.sleep(0.002)
-    assert min(queued) < 0.09
+    assert min(queued) < min(idle) + 0.05
 
 
 def test_a_slot_has_no_room_to_spare_for_the_gather_list():
